@@ -18,7 +18,7 @@ BUILD = os.path.join(HERE, "_build")
 REF_OUT = os.path.join(HERE, "_ref")
 # The reference checkout: $SRK_REFERENCE_DIR, else a directory named
 # "reference" beside the repository (the checkout layout this recipe is
-# used with).  Nothing is built from it when neither exists.
+# used with).  Nothing is built from it when its sources are not there.
 REF_SRC = os.environ.get("SRK_REFERENCE_DIR") or os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference")
 NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -49,10 +49,10 @@ def build_oracle(force=False):
 
 def build_reference(force=False):
     """Compile the reference's host generators and GPU training forward."""
-    if not os.path.isdir(REF_SRC):
+    inc = os.path.join(REF_SRC, "third_party", "include")
+    if not os.path.isdir(inc):  # no checkout, or an empty directory in its place
         return None
     os.makedirs(REF_OUT, exist_ok=True)
-    inc = os.path.join(REF_SRC, "third_party", "include")
     host_src = [os.path.join(HERE, "ref_wrap", "ref_host.cpp"),
                 os.path.join(REF_SRC, "third_party", "src", "patternUtil", "test_pattern.cu")]
     host_out = os.path.join(REF_OUT, "libref_host.so")
