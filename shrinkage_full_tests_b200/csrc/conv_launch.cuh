@@ -7,6 +7,12 @@
 
 namespace srk {
 
+// L2 prefetch distance of the adjoint-type P1 in launch positions per SM.
+#ifndef SRK_P1_AHEAD
+#define SRK_P1_AHEAD 1
+#endif
+constexpr int kP1Ahead = SRK_P1_AHEAD;
+
 template <typename K>
 srk_status set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024)
@@ -23,15 +29,14 @@ srk_status set_smem(K kernel, size_t bytes) {
 template <int OP, typename T>
 srk_status launch_tensor_rows(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt, cudaStream_t s) {
   constexpr int M = kHybM;
-  constexpr int LPU = lpu_of<M>();
   const size_t per = wt_elems<M, OP>(g.S);
   const size_t s1 = s1_elems<M, OP>();
   const size_t plane_wt = (size_t)2 * M * M;  // halves per work tile
   const size_t cap = std::min<size_t>(p->scratch_bytes / sizeof(float2) / per, p->hyb_s1_bytes / sizeof(__half) / plane_wt);
   const size_t smp1 = p1h_smem_bytes();
-  const size_t sm3 = phase_smem_bytes<M>() + (p3_async_window<OP, T>() ? sizeof(float) * p3_window_floats<M>() : 0);
+  constexpr size_t sm3 = p3_smem_bytes<M, OP>();
   SRK_TRY(set_smem(k_p1h<OP, T>, smp1));
-  SRK_TRY(set_smem(k_p3<M, OP, T, kHybS2Layout>, sm3));
+  SRK_TRY(set_smem(k_p3<M, OP, T, kS2Rotated>, sm3));
   SRK_TRY(set_smem(k_p1h_refit<OP, T>, smp1));
   static_assert(OpTraits<OP>::PAIRS, "the tensor-row schedule serves the pair ops");
   // k_p1g (column DFT on the tensor cores): a uniform batch, N % 8 == 0
@@ -68,15 +73,15 @@ srk_status launch_tensor_rows(srk_plan_s* p, const OpArgs& a, const Geom& g, int
       p1g::k_p1g<T><<<std::min(items, std::max(p->nsm, 1)), p1g::kThreadsG, p1g::smem_bytes(), st>>>(
           tmapg, smapg, pmapg, ga);
     } else {
-      k_p1h<OP, T><<<dim3(M / kP1hCols, c), kThreads, smp1, st>>>(pmap, a, g, p->tw, w0, p->nsm, max_of(k),
-                                                                   p->direct_err);
+      k_p1h<OP, T><<<dim3(M / kP1hCols, c), kP1hThreads, smp1, st>>>(pmap, a, g, p->tw, w0, max_of(k),
+                                                                      p->direct_err);
     }
-    k_p1h_refit<OP, T><<<std::max(p->nsm, 1) * 2, kThreads, smp1, st>>>(pmap, a, g, p->tw, w0, c, max_of(k),
-                                                                        p->direct_err);
+    k_p1h_refit<OP, T><<<std::max(p->nsm, 1) * 2, kP1hThreads, smp1, st>>>(pmap, a, g, p->tw, w0, c, max_of(k),
+                                                                           p->direct_err);
     return SRK_OK;
   };
   auto p3 = [&](int w0, int c, float2* base, cudaStream_t st) {
-    k_p3<M, OP, T, kHybS2Layout><<<dim3((g.S + LPU - 1) / LPU, c), kThreads, sm3, st>>>(base, a, g, p->tw, w0, p->nsm);
+    k_p3<M, OP, T, kS2Rotated><<<dim3(s2_blocks(g.S, 0), c), kThreads, sm3, st>>>(base, a, g, p->tw, w0);
   };
   const int whole = (int)std::min<size_t>(std::max<size_t>(cap, 1), 65535);
   int launches = 0;
@@ -132,19 +137,21 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
   if constexpr (M == kHybM && OpTraits<OP>::K == 1 && OpTraits<OP>::PAIRS && !std::is_same<T, float>::value) {
     if (p->schedule == SRK_SCHEDULE_TENSOR_ROWS && p->hyb_ready) return launch_tensor_rows<OP, T>(p, a, g, nwt, s);
   }
-  const size_t sm1 = phase_smem_bytes<M>();
-  const size_t sm2 = sm1 + p2_tile_bytes<M>(g.S);
-  const size_t sm3 = sm1 + (p3_async_window<OP, T>() ? sizeof(float) * p3_window_floats<M>() : 0);
+  constexpr size_t sm1 = p1_smem_bytes<M>(), sm2 = p2_smem_bytes<M>();
+  constexpr size_t sm3 = p3_smem_bytes<M, OP>();
+  constexpr int NG = groups_of<M>();
+  const int n3 = (s2_blocks(g.S, g.e - s2_first(g.e)) + NG - 1) / NG;  // P3 CTAs per work tile
   const size_t per = wt_elems<M, OP>(g.S);
   const size_t cap = p->scratch_bytes / sizeof(float2) / per;  // WTs that fit the scratch
   if (p->schedule == SRK_SCHEDULE_PERSISTENT && cap >= 3) {
-    SRK_TRY(set_smem(k_persist<M, OP, T>, sm2));
+    constexpr size_t smp = sm2;
+    SRK_TRY(set_smem(k_persist<M, OP, T>, smp));
     int dev = 0, nsm = 0, per_sm = 0;
     SRK_CUDA(cudaGetDevice(&dev));
     SRK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    SRK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<M, OP, T>, kThreads, sm2));
-    if (per_sm < 1) return fail(SRK_ERR_UNSUPPORTED, "persistent kernel does not fit an SM (smem %zu)", sm2);
-    const int round = M / lpu_of<M>() * 2 + (g.S + lpu_of<M>() - 1) / lpu_of<M>();
+    SRK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<M, OP, T>, kThreads, smp));
+    if (per_sm < 1) return fail(SRK_ERR_UNSUPPORTED, "persistent kernel does not fit an SM (smem %zu)", smp);
+    const int round = M / unit_lines<M>() * 2 + n3;
     int grid = nsm * per_sm;
     if (p->persist_grid > 0) grid = std::min(grid, p->persist_grid);
     // Tickets in flight ~ grid (x2 with prefetch): the lag between the phases
@@ -164,7 +171,7 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
     const long long tickets = (long long)(nwt + 2 * pp.lag) * round;
     grid = (int)std::min<long long>(grid, tickets);
     SRK_CUDA(cudaMemsetAsync(p->ctl, 0, sizeof(Ctl), s));
-    k_persist<M, OP, T><<<grid, kThreads, sm2, s>>>(a, g, p->G[0], p->G[1], conjG ? 1 : 0, p->tw, p->scratch, nwt,
+    k_persist<M, OP, T><<<grid, kThreads, smp, s>>>(a, g, p->G[0], p->G[1], conjG ? 1 : 0, p->tw, p->scratch, nwt,
                                                    p->ctl, pp);
     SRK_CUDA(cudaGetLastError());
     SRK_CUDA(cudaMemcpyAsync(p->mailbox, &p->ctl->abort, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
@@ -182,30 +189,28 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
     p->last_nslot = pp.nslot;
     return SRK_OK;
   }
-  const size_t smp1 = p1_smem_bytes<M, OP>();
-  SRK_TRY(set_smem(k_p1<M, OP, T>, smp1));
   const bool tan = OP == OP_ADJ && a.dI != nullptr;  // the tangent-adjoint's adjoint-type pass
-  if (tan) SRK_TRY(set_smem(k_p1<M, OP, T, true>, smp1));
-  SRK_TRY(set_smem(k_p2<M, OP>, sm2));
-  SRK_TRY(set_smem(k_p3<M, OP, T>, sm3));
-  constexpr int LPU = lpu_of<M>();
+  constexpr bool kAdj = OP == OP_ADJ;
+  static_assert(sm1 <= 48 * 1024 && sm2 <= 48 * 1024 && sm3 <= 48 * 1024, "no shared-memory opt-in needed");
   auto launch3 = [&](int w0, int c, float2* base, cudaStream_t s1, cudaStream_t s2, cudaStream_t s3,
                      cudaEvent_t e1, cudaEvent_t e2) -> srk_status {
-    const dim3 g1(M / LPU / p1_units<M, OP>(), c);
-    if (tan)
-      k_p1<M, OP, T, true><<<g1, kThreads, smp1, s1>>>(a, g, p->tw, w0, base, g.S, p->nsm);
+    const dim3 g1(M / unit_lines<M>(), c);
+    if (kAdj && a.e < 1)
+      k_p1<M, OP, T, false, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, 0);
+    else if (tan)
+      k_p1<M, OP, T, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, p->nsm * kP1Ahead);
     else
-      k_p1<M, OP, T><<<g1, kThreads, smp1, s1>>>(a, g, p->tw, w0, base, g.S, p->nsm);
+      k_p1<M, OP, T><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, p->nsm * kP1Ahead);
     if (e1) {
       SRK_CUDA(cudaEventRecord(e1, s1));
       SRK_CUDA(cudaStreamWaitEvent(s2, e1, 0));
     }
-    k_p2<M, OP><<<dim3(M / LPU, c), kThreads, sm2, s2>>>(base, p->G[0], p->G[1], conjG ? 1 : 0, g, p->tw);
+    k_p2<M, OP><<<dim3(M / unit_lines<M>(), c), kThreads, sm2, s2>>>(base, p->G[0], p->G[1], conjG ? 1 : 0, g, p->tw);
     if (e2) {
       SRK_CUDA(cudaEventRecord(e2, s2));
       SRK_CUDA(cudaStreamWaitEvent(s3, e2, 0));
     }
-    k_p3<M, OP, T><<<dim3((g.S + LPU - 1) / LPU, c), kThreads, sm3, s3>>>(base, a, g, p->tw, w0, p->nsm);
+    k_p3<M, OP, T><<<dim3(n3, c), kThreads, sm3, s3>>>(base, a, g, p->tw, w0);
     return SRK_OK;
   };
   const int whole = (int)std::min<size_t>(std::max<size_t>(cap, 1), 65535);

@@ -11,16 +11,28 @@
 //              packed tiles with two fields each (adjoint-type ops).
 //
 // One WT goes through three passes whose intermediates live in a scratch
-// buffer (column-contiguous, 8-byte complex):
+// buffer (8-byte complex, blocked by four lines so that both the pass that
+// writes and the pass that reads touch whole 128-byte pieces straight from
+// registers, see fft_quad.cuh for the lane order):
 //   P1  per column x: load the field(s) (the op's loader computes them on
 //       the fly: image values, or v*df/dx products for the adjoint), FFT
-//       along y                                    -> S1[wt][k][x][ky]
-//   P2  per block of 8 rows ky: FFT along x, spectral map with the kernel
-//       spectra (Gx, Gy; conjugated for a true adjoint), inverse FFT along
-//       kx, keep valid columns                    -> S2[wt][l][x'][ky]
+//       along y                          -> S1[wt][k][ky/4][x][ky%4]
+//   P2  per row ky: FFT along x, spectral map with the kernel spectra (Gx,
+//       Gy; conjugated for a true adjoint), inverse FFT along kx, keep the
+//       valid columns                    -> S2[wt][l][(x-xa)/4][ky][x%4]
 //   P3  per valid column: inverse FFT along ky, then the op's epilogue
 //       (central differences of f, combine, store) — conv(g,Gx), conv(g,Gy)
 //       never leave registers.
+// xa = e rounded down to a multiple of four (s2_first).
+//
+// A group of one (M = 128, 256) or two (M = 512) warps transforms four lines
+// with 32 (M = 128: 16) complex values per thread, straight from global
+// memory into registers and back; shared memory holds one exchange per
+// transform and the gradient windows of P3.  A second field (P2's Z*Gy, P3's
+// and the adjoint's second field) stays in registers: at 168 registers and
+// 12 warps per SM that costs less than its round trip through shared memory
+// at a higher occupancy, since the packed transforms have 16 independent
+// chains per thread.
 //
 // The reference performs the same linear "valid" convolution with cufftDX
 // tiles (srk_forward.cuh:354-423) or whole-image cuFFT
@@ -34,27 +46,30 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 #include <type_traits>
-#include "fft_warp.cuh"
+#include "fft_quad.cuh"
+#include "tc.cuh"
 
-// CTAs per SM the kernels are compiled for (register cap 65536/(256*n)).
-#ifndef SRK_MIN_BLOCKS
-#define SRK_MIN_BLOCKS 4
-#endif
+// CTAs of kThreads threads per SM the kernels are compiled for (register cap
+// 65536 / (kThreads n), in steps of 8): 8 -> 128 registers, 6 -> 168.
 #ifndef SRK_P1_MIN_BLOCKS
-#define SRK_P1_MIN_BLOCKS SRK_MIN_BLOCKS
+#define SRK_P1_MIN_BLOCKS 8
+#endif
+#ifndef SRK_P1_ADJ_MIN_BLOCKS
+#define SRK_P1_ADJ_MIN_BLOCKS 6
 #endif
 #ifndef SRK_P2_MIN_BLOCKS
-#define SRK_P2_MIN_BLOCKS SRK_MIN_BLOCKS
+#define SRK_P2_MIN_BLOCKS 6
 #endif
 #ifndef SRK_P3_MIN_BLOCKS
-#define SRK_P3_MIN_BLOCKS SRK_MIN_BLOCKS
+#define SRK_P3_MIN_BLOCKS 6
+#endif
+#ifndef SRK_P3_ADJ_MIN_BLOCKS
+#define SRK_P3_ADJ_MIN_BLOCKS 8
 #endif
 
 namespace srk {
 
-constexpr int kWarps = 8;
-constexpr int kThreads = 32 * kWarps;
-constexpr int kThreadsStage = kThreads;
+constexpr int kThreads = 64;
 
 enum Op : int {
   OP_FWD = 0,       // R = ux*df/dx + uy*df/dy (pairs of tiles); optional ux/uy
@@ -100,6 +115,7 @@ struct Geom {
   int wout_n; // outputs are N x N (adjoint-type) rather than W x W
   const int4* __restrict__ rtile;      // ragged: tile -> (image, x0, y0, 0); else nullptr
   const RagImage* __restrict__ rimg;   // ragged: per-image sizes and offsets
+  unsigned int* err;                   // error word of the bounded waits (may be nullptr)
 };
 
 // Operand pointers.  All images are column-major; batch strides are
@@ -214,529 +230,23 @@ __device__ __forceinline__ float h_at(const OpArgs& a, const TileRef& t, int k, 
   return dot2(dv, g, v, dg);
 }
 
-// Column x of one real tile of image `img` (forward-type ops): values at
-// rows y = lane + 32 i, zero outside the image.  Pointers are hoisted so the
-// loads are (base + immediate); bounds are tested per element only for a
-// tile that crosses the bottom edge.
-template <int M, typename T>
-__device__ __forceinline__ void load_tile_column(const T* __restrict__ img, const TileRef& t, int x, int lane,
-                                                 float (&v)[M / tpf_of<M>()]) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  const int N = t.N;
-  const int gx = t.x0 + x;
-  if (!t.live || gx >= N) {
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) v[i] = 0.f;
-    return;
-  }
-  const T* col = img + t.on + (long long)gx * N + t.y0 + lane;
-  const int rows = N - t.y0 - lane;  // rows available below this lane's first element
-  if (N - t.y0 >= M) {
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) v[i] = ldf(col, TPF * i);
-  } else {
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) v[i] = (TPF * i < rows) ? ldf(col, TPF * i) : 0.f;
-  }
-}
-
-template <int M, int OP, typename T>
-__device__ __forceinline__ void load_column(const OpArgs& a, const Geom& g, int w, int k, int x, int lane,
-                                            float2 (&z)[M / tpf_of<M>()]) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  if constexpr (OP == OP_ADJ) {
-    const TileRef t0 = tile_of(g, 2 * w), t1 = tile_of(g, 2 * w + 1);
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      const int y = lane + TPF * i;
-      const float re = h_at<T>(a, t0, k, t0.x0 + x, t0.y0 + y);
-      const float im = t1.live ? h_at<T>(a, t1, k, t1.x0 + x, t1.y0 + y) : 0.f;
-      z[i] = make_float2(re, im);
-    }
-  } else if constexpr (OpTraits<OP>::PAIRS) {
-    float re[EPT], im[EPT];
-    const T* E = static_cast<const T*>(a.E);
-    load_tile_column<M, T>(E, tile_of(g, 2 * w), x, lane, re);
-    load_tile_column<M, T>(E, tile_of(g, 2 * w + 1), x, lane, im);
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) z[i] = make_float2(re[i], im[i]);
-  } else {
-    float re[EPT], im[EPT];
-    const TileRef t = tile_of(g, w);
-    load_tile_column<M, T>(static_cast<const T*>(a.E), t, x, lane, re);
-    load_tile_column<M, T>(static_cast<const T*>(a.dE), t, x, lane, im);
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) z[i] = make_float2(re[i], im[i]);
-  }
-}
-
-// Both adjoint-type fields of one P1 column at once (erosion >= 1, so every
-// gradient neighbour of the valid window lies inside the image): zx = h_x of
-// the two tiles of WT w (re / im) at virtual column x, rows lane + TPF i,
-// and h_y of the same element straight into this thread's stash slot
-// st[kThreads i].  Per element one load of v (and dv) and the four
-// neighbours of f (and df), shared by h_x and h_y; the arithmetic is h_at's.
-// TAN: the tangent-adjoint's fields (dv, df given), a compile-time choice so
-// that the plain adjoint carries none of their registers.
-template <int M, typename T, bool TAN>
-__device__ __forceinline__ void load_adj_column(const OpArgs& a, const Geom& g, int w, int x, int lane,
-                                                float2 (&zx)[M / tpf_of<M>()], float2* __restrict__ st) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  const T* vc[2];
-  const T* fc[2];
-  const T* dvc[2];
-  const T* dfc[2];
-  int N[2], W[2], oy0[2];
-  bool on[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const TileRef tr = tile_of(g, 2 * w + h);
-    const int qx = tr.x0 + x - a.e, ox = qx - a.e;  // image / valid-window column
-    on[h] = tr.live && ox >= 0 && ox < tr.W;
-    const int qy0 = tr.y0 + lane - a.e;
-    oy0[h] = qy0 - a.e;
-    N[h] = tr.N;
-    W[h] = tr.W;
-    const long long vo = tr.ow + (long long)ox * tr.W + oy0[h];
-    const long long fo = tr.on + (long long)qx * tr.N + qy0;
-    vc[h] = static_cast<const T*>(a.v) + vo;
-    fc[h] = static_cast<const T*>(a.I) + fo;
-    dvc[h] = TAN ? static_cast<const T*>(a.dv) + vo : vc[h];
-    dfc[h] = TAN ? static_cast<const T*>(a.dI) + fo : fc[h];
-  }
-#pragma unroll
-  for (int i = 0; i < EPT; ++i) {
-    const int o = TPF * i;
-    float hx[2], hy[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool in = on[h] && (unsigned)(oy0[h] + o) < (unsigned)W[h];
-      const int n = N[h];
-      const float v = in ? ldf(vc[h], o) : 0.f;
-      const float gx = ((in ? ldf(fc[h] + n, o) : 0.f) - (in ? ldf(fc[h] - n, o) : 0.f)) * 0.5f;
-      const float gy = ((in ? ldf(fc[h] + 1, o) : 0.f) - (in ? ldf(fc[h] - 1, o) : 0.f)) * 0.5f;
-      hx[h] = v * gx;
-      hy[h] = v * gy;
-      if constexpr (TAN) {
-        const float dv = in ? ldf(dvc[h], o) : 0.f;
-        const float dgx = ((in ? ldf(dfc[h] + n, o) : 0.f) - (in ? ldf(dfc[h] - n, o) : 0.f)) * 0.5f;
-        const float dgy = ((in ? ldf(dfc[h] + 1, o) : 0.f) - (in ? ldf(dfc[h] - 1, o) : 0.f)) * 0.5f;
-        hx[h] = dot2(dv, gx, v, dgx);
-        hy[h] = dot2(dv, gy, v, dgy);
-      }
-      if (!in) hx[h] = hy[h] = 0.f;
-    }
-    zx[i] = make_float2(hx[0], hx[1]);
-    st[kThreads * i] = make_float2(hy[0], hy[1]);
-  }
-}
-
-// Central differences of f at image column gx for this lane's rows
-// gy = gy0 + 32 i: fx = (f[gx+1] - f[gx-1])/2, fy = (f[gy+1] - f[gy-1])/2.
-// With erosion >= 1 every valid output has its 4 neighbours inside the
-// image, so the zero-padding rule of srk_grad_x/_y never applies and the
-// loads need no test; erosion 0 takes the tested path.
-template <typename T>
-struct GradCol {
-  const T* __restrict__ c;   // f + gx*N + gy0
-  int N;
-  bool tested;
-  int gx, gy0;
-  int st;  // row step between a thread's elements (threads per transform)
-  __device__ __forceinline__ void at(int i, float& fx, float& fy) const {
-    if (!tested) {
-      fx = (ldf(c + N, st * i) - ldf(c - N, st * i)) * 0.5f;
-      fy = (ldf(c + 1, st * i) - ldf(c - 1, st * i)) * 0.5f;
-    } else {
-      const int gy = gy0 + st * i;
-      const float r = (gx + 1 < N) ? ldf(c + N, st * i) : 0.f;
-      const float l = (gx > 0) ? ldf(c - N, st * i) : 0.f;
-      const float d = (gy + 1 < N) ? ldf(c + 1, st * i) : 0.f;
-      const float u = (gy > 0) ? ldf(c - 1, st * i) : 0.f;
-      fx = (r - l) * 0.5f;
-      fy = (d - u) * 0.5f;
-    }
-  }
-};
-template <typename T>
-__device__ __forceinline__ GradCol<T> grad_col(const T* f_img, int N, int e, int gx, int gy0, int st) {
-  GradCol<T> gc;
-  gc.st = st;
-  gc.c = f_img + (long long)gx * N + gy0;
-  gc.N = N;
-  gc.tested = e < 1;
-  gc.gx = gx;
-  gc.gy0 = gy0;
-  return gc;
-}
-
-// Rows of this lane that carry valid outputs, as a bit mask over i.
+// ---- blocks, groups and scratch layout -----------------------------------------
+// A CTA of kThreads threads holds groups_of<M>() groups of four lines.
 template <int M>
-__device__ __forceinline__ unsigned valid_rows(const Geom& g, const TileRef& t, int lane) {
-  // rows y = lane + TPF*i are valid for e <= y < yhi: a contiguous run of i
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  const int yhi = min(g.e + g.S, t.Wout - t.y0 + g.e);
-  const int ilo = max(0, (g.e - lane + TPF - 1) / TPF);        // first i with y >= e (g.e - lane > -TPF)
-  const int ihi = yhi - lane > 0 ? (yhi - lane + TPF - 1) / TPF : 0;  // first i with y >= yhi
-  const int hi = min(ihi, EPT);
-  return hi > ilo ? (((1u << hi) - 1u) & ~((1u << ilo) - 1u)) : 0u;
-}
-
-template <int M, int OP, typename T>
-__device__ __forceinline__ void epilogue_column(const OpArgs& a, const Geom& g, int w, int x, int lane,
-                                                float2 (&z0)[M / tpf_of<M>()], float2 (&z1)[M / tpf_of<M>()]) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  const int e = a.e;
-  if constexpr (OP == OP_FWD || OP == OP_VJP_F) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const TileRef t = tile_of(g, 2 * w + h);
-      const int ox = t.x0 + x - g.e;
-      if (!t.live || ox >= t.Wout) continue;
-      const unsigned vm = valid_rows<M>(g, t, lane);
-      // output row oy = y0 + y - e  ->  offset of row (y0 - e + lane)
-      const long long ob = t.ow + (long long)ox * t.W + t.y0 - g.e + lane;
-      if constexpr (OP == OP_FWD) {
-        T* __restrict__ R = static_cast<T*>(a.out0);
-        T* __restrict__ UX = static_cast<T*>(a.out_ux);
-        T* __restrict__ UY = static_cast<T*>(a.out_uy);
-        if (UX) {
-#pragma unroll
-          for (int i = 0; i < EPT; ++i)
-            if (vm >> i & 1u) stf(UX, ob + TPF * i, h ? z0[i].y : z0[i].x);
-        }
-        if (UY) {
-#pragma unroll
-          for (int i = 0; i < EPT; ++i)
-            if (vm >> i & 1u) stf(UY, ob + TPF * i, h ? z1[i].y : z1[i].x);
-        }
-        if (R) {
-          const GradCol<T> gc = grad_col(static_cast<const T*>(a.I) + t.on, t.N, e, ox + e, t.y0 + lane, TPF);
-          // gradients for all rows first (every load in flight before the
-          // first store); the result overwrites this image's half of z0
-#pragma unroll
-          for (int i = 0; i < EPT; ++i) {
-            float fx = 0.f, fy = 0.f;
-            if (vm >> i & 1u) gc.at(i, fx, fy);
-            float& o = h ? z0[i].y : z0[i].x;
-            o = dot2(o, fx, h ? z1[i].y : z1[i].x, fy);
-          }
-#pragma unroll
-          for (int i = 0; i < EPT; ++i)
-            if (vm >> i & 1u) stf(R, ob + TPF * i, h ? z0[i].y : z0[i].x);
-        }
-      } else {  // OP_VJP_F: w = u * v
-        const T* __restrict__ V = static_cast<const T*>(a.v);
-        float* __restrict__ WX = static_cast<float*>(a.out0);
-        float* __restrict__ WY = static_cast<float*>(a.out1);
-        float v[EPT];
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) v[i] = (vm >> i & 1u) ? ldf(V, ob + TPF * i) : 0.f;
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) {
-          if (!(vm >> i & 1u)) continue;
-          WX[ob + TPF * i] = (h ? z0[i].y : z0[i].x) * v[i];
-          WY[ob + TPF * i] = (h ? z1[i].y : z1[i].x) * v[i];
-        }
-      }
-    }
-  } else if constexpr (OP == OP_JVP || OP == OP_TANADJ_F) {
-    const TileRef t = tile_of(g, w);
-    const int ox = t.x0 + x - g.e;
-    if (ox >= t.Wout) return;
-    const unsigned vm = valid_rows<M>(g, t, lane);
-    const long long ob = t.ow + (long long)ox * t.W + t.y0 - g.e + lane;
-    if constexpr (OP == OP_JVP) {
-      // srk_tangent_combine (tan_tanadj/srk_tangent.cuh:28-52); re: conv of g, im: conv of dg
-      const GradCol<T> gf = grad_col(static_cast<const T*>(a.I) + t.on, t.N, e, ox + e, t.y0 + lane, TPF);
-      const GradCol<T> gd = grad_col(static_cast<const T*>(a.dI) + t.on, t.N, e, ox + e, t.y0 + lane, TPF);
-      T* __restrict__ DH = static_cast<T*>(a.out0);
-#pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        float fx = 0.f, fy = 0.f, dfx = 0.f, dfy = 0.f;
-        if (vm >> i & 1u) {
-          gf.at(i, fx, fy);
-          gd.at(i, dfx, dfy);
-        }
-        z0[i].x = __fmaf_rn(z1[i].x, dfy, __fmaf_rn(z0[i].x, dfx, dot2(z0[i].y, fx, z1[i].y, fy)));
-      }
-#pragma unroll
-      for (int i = 0; i < EPT; ++i)
-        if (vm >> i & 1u) stf(DH, ob + TPF * i, z0[i].x);
-    } else {
-      const T* __restrict__ LAM = static_cast<const T*>(a.v);
-      const T* __restrict__ DLAM = static_cast<const T*>(a.dv);
-      float* __restrict__ WX = static_cast<float*>(a.out0);
-      float* __restrict__ WY = static_cast<float*>(a.out1);
-#pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        if (!(vm >> i & 1u)) continue;
-        const float lam = ldf(LAM, ob + TPF * i), dlam = ldf(DLAM, ob + TPF * i);
-        WX[ob + TPF * i] = dot2(dlam, z0[i].x, lam, z0[i].y);
-        WY[ob + TPF * i] = dot2(dlam, z1[i].x, lam, z1[i].y);
-      }
-    }
-  } else {  // OP_ADJ: output is the full N x N image
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const TileRef t = tile_of(g, 2 * w + h);
-      const int ox = t.x0 + x - g.e;
-      if (!t.live || ox >= t.Wout) continue;
-      const unsigned vm = valid_rows<M>(g, t, lane);
-      const long long ob = t.on + (long long)ox * t.N + t.y0 - g.e + lane;
-      T* __restrict__ O = static_cast<T*>(a.out0);
-#pragma unroll
-      for (int i = 0; i < EPT; ++i)
-        if (vm >> i & 1u) stf(O, ob + TPF * i, h ? z0[i].y : z0[i].x);
-    }
-  }
-}
-
-// ---- unit geometry ----------------------------------------------------------------
-// A CTA of kWarps warps processes one unit of LPU lines (columns in P1/P3,
-// rows in P2); each line is one transform over TPF threads (line = thread /
-// TPF, t = thread % TPF, named barrier 1 + line when TPF > 32).
+__host__ __device__ constexpr int groups_of() { return kThreads / Quad<M>::GT; }
 template <int M>
-__host__ __device__ constexpr int lpu_of() { return kThreads / tpf_of<M>(); }
-
-// ---- staged gradients -------------------------------------------------------------
-// The LPU output columns of a P3 unit need the image columns gx-1 ..
-// gx+LPU and rows gy-1 .. gy+S.  They are staged into shared memory, one
-// warp per window column: window column c <-> image column x0 + e - 1 + c;
-// window row r <-> image row gy0 + r, gy0 = y0 + e - 1, stored at column
-// offset off + r.  Out-of-image elements are zero (the central-difference
-// rule).  With 16-byte copies the column starts at the aligned row
-// gy0 - off (off = gy0 mod 4); otherwise off = 0.  The pitch is a multiple
-// of 4 floats (16-byte aligned columns).
-__host__ __device__ inline int gwin_pitch(int S) { return (S + 8) & ~3; }
-// The same for a window of raw storage values (16-byte chunks of EPC
-// elements): a multiple of EPC that holds off + S + 2 for any off < EPC.
-template <typename T>
-__host__ __device__ inline int gwin_pitch_t(int S) {
-  constexpr int EPC = 16 / (int)sizeof(T);
-  return (S + 2 + 2 * (EPC - 1)) / EPC * EPC;
-}
-// Shared-memory window value as float.
-template <typename T> __device__ __forceinline__ float swin(const T* p);
-template <> __device__ __forceinline__ float swin<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float swin<__half>(const __half* p) { return __half2float(*p); }
-template <> __device__ __forceinline__ float swin<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-// (LPU + 2) * gwin_pitch(S) floats <= (LPU + 2) * (M + 4) <= 2 * LPU * (M + M/16 + 2)
-// for S <= M - 2: one image's window always fits the LPU staging rows of the
-// second field.
-struct GradWin {
-  int gx0, gy0;  // image coordinates of window column 0, row 0
-  int ncol, S;   // columns, and S + 2 rows
-  int HP, off;   // column pitch (floats), offset of row 0 in a column
-};
-
-// Synchronous staging (any storage type; values converted to float).
-template <typename T>
-__device__ __forceinline__ void stage_grad_window(const T* __restrict__ img, int N, const GradWin& gw,
-                                                  float* __restrict__ dst) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int H = gw.S + 2;
-  for (int c = warp; c < gw.ncol; c += kWarps) {
-    const int gx = gw.gx0 + c;
-    const bool colin = gx >= 0 && gx < N;
-    const T* col = img + (long long)(colin ? gx : 0) * N;
-    float* d = dst + c * gw.HP;
-    for (int r = lane; r < H; r += 32) {
-      const int gy = gw.gy0 + r;
-      d[r] = (colin && gy >= 0 && gy < N) ? ldf(col, gy) : 0.f;
-    }
-  }
-}
-
-// Asynchronous staging with cp.async (FP32 images): the caller commits the
-// group and waits for it later, so the loads overlap other work.
-__device__ __forceinline__ void cp_async4_zfill(float* dst, const float* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async16_zfill(float* dst, const float* src, bool valid) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Raw storage values of the window.  vec16: 16-byte chunks of EPC values
-// (needs N % EPC == 0 and a 16-byte aligned image, so every chunk lies
-// wholly inside or wholly outside the image); else 4-byte copies (FP32 only).
-template <typename T>
-__device__ __forceinline__ void stage_grad_window_async(const T* __restrict__ img, int N, const GradWin& gw,
-                                                        bool vec16, T* __restrict__ dst) {
-  constexpr int EPC = 16 / (int)sizeof(T);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int c = warp; c < gw.ncol; c += kWarps) {
-    const int gx = gw.gx0 + c;
-    const bool colin = gx >= 0 && gx < N;
-    const T* col = img + (long long)(colin ? gx : 0) * N;
-    T* d = dst + c * gw.HP;
-    if (vec16) {
-      // chunk q of the column: rows gya + EPC*q ..; gya = gy0 - off >= 0, so
-      // a chunk is outside the image only past its last row (or off its columns)
-      const int gya = gw.gy0 - gw.off;
-      const int nch = (gw.off + gw.S + 2 + EPC - 1) / EPC;
-      const int glim = colin ? N : -1;
-      const char* src = reinterpret_cast<const char*>(col + gya) + 16 * lane;
-      unsigned dsm = static_cast<unsigned>(__cvta_generic_to_shared(d)) + 16u * lane;
-      int gy = gya + EPC * lane;
-      for (int q = lane; q < nch; q += 32, src += 512, dsm += 512u, gy += 32 * EPC) {
-        const bool in = gy < glim;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dsm), "l"(in ? src : (const char*)img),
-                     "r"(in ? 16 : 0)
-                     : "memory");
-      }
-    } else if constexpr (std::is_same<T, float>::value) {
-      for (int r = lane; r < gw.S + 2; r += 32) {
-        const int gy = gw.gy0 + r;
-        const bool in = colin && gy >= 0 && gy < N;
-        cp_async4_zfill(d + r, in ? col + gy : img, in);
-      }
-    }
-  }
-}
-// Floats of one staged window at tile size M (S <= M - 2 when erosion >= 1);
-// a window of 2-byte values needs at most (LPU + 2) * (M + 8) of them.
-template <int M>
-__host__ __device__ constexpr int p3_window_floats() { return (lpu_of<M>() + 2) * (M + 4); }
-// P3 of the three-launch schedule prefetches the first window asynchronously
-// into a buffer of its own (forward / tangent epilogues).
-template <int OP, typename T>
-__host__ __device__ constexpr bool p3_async_window() {
-  return OP == OP_FWD || OP == OP_JVP;
-}
-
-// Forward / tangent epilogue, round h, with the central differences read
-// from the staged window (window column line+1 is this line's image
-// column).  FWD: round h finishes image h of the pair.  JVP: round 0
-// (window = f) leaves the f terms in z0.y, round 1 (window = df) adds the df
-// terms.  z0 stays stashed in the line's padded row (z0s = row + t +
-// (t >> 4), element i at z0s[(TPF + TPF/16) i]) to keep registers free.
-template <int M, int OP, typename T, typename WT>
-__device__ __forceinline__ void epilogue_staged(const OpArgs& a, const Geom& g, const TileRef& tr, int x, int line,
-                                                int t, int h, float2* __restrict__ z0s,
-                                                const float2 (&z1)[M / tpf_of<M>()], const WT* __restrict__ win,
-                                                const GradWin& gw) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  constexpr int RSP = TPF + TPF / 16;
-  const int W = tr.W;
-  const int rb = gw.off + t - g.e + 1;     // window row of element 0: y - e + 1, y = t
-  const WT* cm = win + line * gw.HP + rb;  // image column gx - 1
-  const WT* cc = cm + gw.HP;               // gx
-  const WT* cp = cc + gw.HP;               // gx + 1
-  const int ox = tr.x0 + x - g.e;
-  if (!tr.live || ox >= tr.Wout) return;
-  const unsigned vm = valid_rows<M>(g, tr, t);
-  const long long ob = tr.ow + (long long)ox * W + tr.y0 - g.e + t;
-  if constexpr (OP == OP_FWD) {
-    T* __restrict__ R = static_cast<T*>(a.out0);
-    T* __restrict__ UX = static_cast<T*>(a.out_ux);
-    T* __restrict__ UY = static_cast<T*>(a.out_uy);
-    if (!UX && !UY) {
-      // R only (R is never NULL here): the common case; of the stashed z0
-      // only this round's half is read
-      T* __restrict__ Rp = R + ob;
-      const float* z0h = reinterpret_cast<const float*>(z0s) + h;
-#pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        if (!(vm >> i & 1u)) continue;
-        const float ux = z0h[2 * RSP * i];
-        const float uy = h ? z1[i].y : z1[i].x;
-        // the central differences' factor 1/2 applied once: halving is
-        // exact, so dot2(ux, dx/2, uy, dy/2) == dot2(ux, dx, uy, dy)/2
-        const float dx = swin(cp + TPF * i) - swin(cm + TPF * i);
-        const float dy = swin(cc + TPF * i + 1) - swin(cc + TPF * i - 1);
-        stf(Rp, TPF * i, dot2(ux, dx, uy, dy) * 0.5f);
-      }
-      return;
-    }
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      if (!(vm >> i & 1u)) continue;
-      const float2 z0i = z0s[RSP * i];
-      const float ux = h ? z0i.y : z0i.x;
-      const float uy = h ? z1[i].y : z1[i].x;
-      if (UX) stf(UX, ob + TPF * i, ux);
-      if (UY) stf(UY, ob + TPF * i, uy);
-      if (R) {
-        const float dx = swin(cp + TPF * i) - swin(cm + TPF * i);
-        const float dy = swin(cc + TPF * i + 1) - swin(cc + TPF * i - 1);
-        stf(R, ob + TPF * i, dot2(ux, dx, uy, dy) * 0.5f);
-      }
-    }
-  } else {
-    // srk_tangent_combine (tan_tanadj/srk_tangent.cuh:28-52):
-    // dh = Im(zx) fx + Im(zy) fy + Re(zx) dfx + Re(zy) dfy
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      if (!(vm >> i & 1u)) continue;
-      const float dx_ = (swin(cp + TPF * i) - swin(cm + TPF * i)) * 0.5f;
-      const float dy_ = (swin(cc + TPF * i + 1) - swin(cc + TPF * i - 1)) * 0.5f;
-      float2 z0i = z0s[RSP * i];
-      if (h == 0) {
-        z0i.y = dot2(z0i.y, dx_, z1[i].y, dy_);
-        z0s[RSP * i] = z0i;
-      } else {
-        stf(static_cast<T*>(a.out0), ob + TPF * i, __fmaf_rn(z1[i].x, dy_, __fmaf_rn(z0i.x, dx_, z0i.y)));
-      }
-    }
-  }
-}
-
-// ---- phases ------------------------------------------------------------------
-__device__ __forceinline__ void load_twiddles(float2* tw, const float2* __restrict__ twg, int M) {
-  for (int i = threadIdx.x; i < tw_entries(M); i += blockDim.x) tw[i] = twg[i];
-}
-
-// Staging rows: fft_row_words(M) or a little more, so that the rows of a
-// transposing copy fall into different banks.
-template <int M>
-__host__ __device__ constexpr int row_stride() {
-  // stage_rows writes 2 (LPU = 4) or 4 (LPU = 8) rows per half-warp: their
-  // strides must land on disjoint banks (RS = 4 or 2 mod 8 complex values)
-  int w = fft_row_words(M) + 1;
-  while (w % 8 != (lpu_of<M>() == 4 ? 4 : 2)) ++w;
-  return w;
-}
-// Valid columns x' of S2 rounded up to a multiple of 8 (>= LPU).
+__host__ __device__ constexpr int unit_lines() { return kLines * groups_of<M>(); }
+// First column of S2: the valid columns start at x = e; the blocks of four
+// start at a multiple of four so that P2's stores cover whole blocks.
+__host__ __device__ inline int s2_first(int e) { return e & ~3; }
+// Columns of S2, a multiple of 8.  With S = M - 2e (M a multiple of 8),
+// S mod 8 = -2e mod 8, so (S + 7) & ~7 >= S + e % 4: xa .. e + S - 1 fits.
 __host__ __device__ inline int s2_pitch(int S) { return (S + 7) & ~7; }
-// S2 layout.  Blocked (M = 512, LPU = 4): S2[l][x'/LPU][ky][x' % LPU], so
-// the LPU columns a P3 unit needs are one contiguous run of M*LPU values
-// (instead of 32-byte pieces of every row), and the LPU x LPU block a P2
-// unit produces per column block is contiguous too; P2 assembles the blocks
-// in a shared tile of pitch s2_block_pitch per block (LPU^2 values + padding
-// that keeps its writes free of bank conflicts).  Row layout (LPU = 8):
-// S2[l][ky][x'], pitch s2_pitch(S) — with 64-byte pieces per row the extra
-// tile pass in P2 costs more than it saves in P3.
-template <int M>
-__host__ __device__ constexpr bool s2_blocked() { return lpu_of<M>() == 4; }
-// S1 likewise (M = 512): S1[k][ky/LPU][x][ky % LPU], assembled by P1 in its
-// staging rows (free after the transforms), staged by P2 from one
-// contiguous run of M*LPU values.  At LPU = 8 the rows are read in 64-byte
-// pieces already and the blocked form measured no faster.
-template <int M>
-__host__ __device__ constexpr bool s1_blocked() { return lpu_of<M>() == 4; }
-template <int M>
-__host__ __device__ constexpr int s2_block_pitch() { return lpu_of<M>() == 4 ? 20 : 72; }
-template <int M>
-__host__ __device__ inline size_t p2_tile_bytes(int S) {
-  return s2_blocked<M>() ? sizeof(float2) * (size_t)(s2_pitch(S) / lpu_of<M>()) * s2_block_pitch<M>() : 0;
-}
-// Twiddle slots at the start of every kernel's shared memory.
-template <int M>
-__host__ __device__ constexpr int tw_slots() { return (tw_entries(M) + 7) & ~7; }
+// Blocks of four columns that hold a valid one, first valid column xa + off.
+__host__ __device__ inline int s2_blocks(int S, int off) { return (S + off + kLines - 1) / kLines; }
 
-// Scratch of one work tile: S1 [K][x < M][ky < M] then S2 (L fields of M x pitch(S), see above) (float2).
+// Scratch of one work tile: S1 [K fields] of M x M, then S2 [L fields] of
+// s2_pitch(S) x M (float2).
 template <int M, int OP>
 __host__ __device__ constexpr size_t s1_elems() { return (size_t)OpTraits<OP>::K * M * M; }
 template <int M, int OP>
@@ -744,550 +254,830 @@ __host__ __device__ inline size_t wt_elems(int S) {
   return s1_elems<M, OP>() + (size_t)OpTraits<OP>::L * M * s2_pitch(S);
 }
 
-// Shared memory of every phase: the twiddle table and 2 x LPU staging rows
-// (P2 adds its block tile, P3 its first gradient window).
-template <int M>
-constexpr size_t phase_smem_bytes() { return sizeof(float2) * (tw_slots<M>() + 2 * lpu_of<M>() * row_stride<M>()); }
-// P1 of the adjoint-type op adds the stash of the second field.
-template <int M, int OP>
-constexpr size_t p1_smem_bytes() {
-  return phase_smem_bytes<M>() + (OP == OP_ADJ ? sizeof(float2) * kThreads * (M / tpf_of<M>()) : 0);
+// Engine layout of a kernel spectrum: quads of two neighbouring kx (re, re,
+// im, im), blocked by four rows ky like S1, so P2 multiplies packed pairs
+// read as contiguous 16-byte quads.  Index of Re G(ky, kx) in floats; Im is
+// two floats further.
+__host__ __device__ inline size_t spec_index(int M, int ky, int kx) {
+  return 4 * (((size_t)(ky >> 2) * (M / 2) + (kx >> 1)) * 4 + (ky & 3)) + (kx & 1);
 }
 
-// Copies between a thread's registers (strided order) and a padded row.
+// ---- a group's shared memory and bulk copies ----------------------------------------
+// Inputs that are contiguous runs (image columns, S1 and S2 blocks, spectra)
+// arrive by bulk copies (cp.async.bulk, the TMA engine) into shared memory:
+// the copies need no registers and no L1 lines while in flight.  Loads
+// straight to registers did: at two to three exchanges of 17 KB per SM's
+// free L1 the lines in flight, not HBM, bounded the passes (P1 at M = 512
+// moved 5.5 TB/s against 6.2 with bulk copies).
+//   exchange  Quad<M>::XQ quads; also the landing zone of the first input
+//   buffer    one block of four lines (4 M complex values): the second input,
+//             the spectra, or a gradient window
+//   barriers  two mbarriers
 template <int M>
-__device__ __forceinline__ void row_to_regs(const float2* __restrict__ row, float2 (&z)[M / tpf_of<M>()], int t) {
-  constexpr int TPF = tpf_of<M>();
-  const float2* rd = row + t + (t >> 4);
-#pragma unroll
-  for (int i = 0; i < M / TPF; ++i) z[i] = rd[(TPF + TPF / 16) * i];
-}
+__host__ __device__ constexpr size_t exch_bytes() { return sizeof(float4) * (size_t)Quad<M>::XQ; }
 template <int M>
-__device__ __forceinline__ void regs_to_row(float2* __restrict__ row, const float2 (&z)[M / tpf_of<M>()], int t) {
-  constexpr int TPF = tpf_of<M>();
-  float2* wr = row + t + (t >> 4);
-#pragma unroll
-  for (int i = 0; i < M / TPF; ++i) wr[(TPF + TPF / 16) * i] = z[i];
-}
+__host__ __device__ constexpr size_t block_bytes() { return sizeof(float2) * (size_t)kLines * M; }
+template <int M, bool BUF>
+__host__ __device__ constexpr size_t group_bytes() { return exch_bytes<M>() + (BUF ? block_bytes<M>() : 0) + 16; }
+constexpr unsigned long long kBulkWaitLimit = 1ull << 22;
 
-// P1: line `line` transforms column x = xb*LPU + line of every field along y.
-// P1 output of one field: the line's transform z (ky = t + TPF*i) of
-// column xb*LPU + line -> S1.
 template <int M>
-__device__ __forceinline__ void p1_store(const float2 (&z)[M / tpf_of<M>()], float2* __restrict__ S1k, int xb,
-                                         float2* __restrict__ rows, int line, int t) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  constexpr int LPU = lpu_of<M>();
-  if constexpr (s1_blocked<M>()) {
-    // the unit's LPU columns -> shared tile of (ky/LPU) blocks -> whole
-    // LPU x LPU blocks of S1 (the staging rows are free after the transforms)
-    constexpr int PB = s2_block_pitch<M>();
-    constexpr int F4B = LPU * LPU / 2;
-    __syncthreads();
-    // ky = t + TPF*i: block t/LPU + i*TPF/LPU, position t % LPU in it
-    float2* rl = rows + (t / LPU) * PB + line * LPU + (t % LPU);
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) rl[(TPF / LPU) * PB * i] = z[i];
-    __syncthreads();
-    float2* dst = S1k + (size_t)xb * LPU * LPU;
-    for (int j = threadIdx.x; j < (M / LPU) * F4B; j += kThreads) {
-      const int q = j / F4B, v = j - (j / F4B) * F4B;
-      __stcg(reinterpret_cast<float4*>(dst + (size_t)q * M * LPU + 2 * v),
-             *reinterpret_cast<const float4*>(rows + q * PB + 2 * v));
+struct GroupMem {
+  QuadThread t;
+  float4* ex;
+  unsigned char* buf;
+  uint64_t* bar;       // two barriers
+  unsigned parity;     // bit i: the phase barrier i waits for next
+  unsigned int* err;
+  __device__ __forceinline__ bool leader() const { return threadIdx.x % Quad<M>::GT == 0; }
+  // Copies may be issued into memory that the group has used before.
+  __device__ __forceinline__ void open() const {
+    tc::fence_async_smem();
+    group_sync<M>();
+  }
+  // One contiguous run by the leader.
+  __device__ __forceinline__ void fetch(int i, void* dst, const void* src, unsigned bytes) const {
+    if (leader()) {
+      tc::mbar_expect_tx(bar + i, bytes);
+      tc::bulk_g2s(dst, src, bytes, bar + i);
     }
-    __syncthreads();  // the rows are the next transform's exchange rows
+  }
+  __device__ __forceinline__ void wait(int i) {
+    if (!tc::mbar_wait(bar + i, parity >> i & 1u, kBulkWaitLimit) && err) atomicCAS(err, 0u, 16u);
+    parity ^= 1u << i;
+  }
+};
+// Carves the group's part out of the block's shared memory and initialises
+// its barriers (once per kernel).
+template <int M, bool BUF>
+__device__ __forceinline__ GroupMem<M> group_mem(unsigned char* sm, unsigned int* err) {
+  GroupMem<M> g;
+  unsigned char* p = sm + threadIdx.x / Quad<M>::GT * group_bytes<M, BUF>();
+  g.t = quad_thread<M>();
+  g.ex = reinterpret_cast<float4*>(p);
+  g.buf = BUF ? p + exch_bytes<M>() : nullptr;
+  g.bar = reinterpret_cast<uint64_t*>(p + group_bytes<M, BUF>() - 16);
+  g.parity = 0;
+  g.err = err;
+  if (g.leader()) {
+    tc::mbar_init(g.bar, 1);
+    tc::mbar_init(g.bar + 1, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  return g;
+}
+
+// ---- loaders ------------------------------------------------------------------------
+// Shared-memory image values: one, and an aligned pair.
+template <typename T> __device__ __forceinline__ float swin(const T* p);
+template <> __device__ __forceinline__ float swin<float>(const float* p) { return *p; }
+template <> __device__ __forceinline__ float swin<__half>(const __half* p) { return __half2float(*p); }
+template <> __device__ __forceinline__ float swin<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+template <typename T> __device__ __forceinline__ pk swin2(const T* p);
+template <> __device__ __forceinline__ pk swin2<float>(const float* p) {
+  return *reinterpret_cast<const unsigned long long*>(p);
+}
+template <> __device__ __forceinline__ pk swin2<__half>(const __half* p) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(p));
+  return pk_make(f.x, f.y);
+}
+template <> __device__ __forceinline__ pk swin2<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+  return pk_make(f.x, f.y);
+}
+
+// Two consecutive values as a packed pair; VEC: one aligned access.
+template <bool VEC, typename T>
+__device__ __forceinline__ pk ld2(const T* __restrict__ p, long long i, bool lo, bool hi) {
+  if constexpr (VEC) {
+    if (!lo) return 0ull;
+    if constexpr (sizeof(T) == 4) {
+      return __ldg(reinterpret_cast<const unsigned long long*>(p + i));
+    } else if constexpr (std::is_same<T, __half>::value) {
+      const float2 f = __half22float2(__ldg(reinterpret_cast<const __half2*>(p + i)));
+      return pk_make(f.x, f.y);
+    } else {
+      const float2 f = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162*>(p + i)));
+      return pk_make(f.x, f.y);
+    }
   } else {
-    float2* dst = S1k + (size_t)(xb * LPU + line) * M + t;
+    const float a = lo ? ldf(p, i) : 0.f, b = hi ? ldf(p, i + 1) : 0.f;
+    return pk_make(a, b);
+  }
+}
+template <bool VEC, typename T>
+__device__ __forceinline__ void st2(T* __restrict__ p, long long i, pk v, bool lo, bool hi) {
+  if constexpr (VEC) {
+    if (!lo) return;
+    if constexpr (sizeof(T) == 4)
+      *reinterpret_cast<unsigned long long*>(p + i) = v;
+    else if constexpr (std::is_same<T, __half>::value)
+      *reinterpret_cast<__half2*>(p + i) = __floats2half2_rn(pk_lo(v), pk_hi(v));
+    else
+      *reinterpret_cast<__nv_bfloat162*>(p + i) = __floats2bfloat162_rn(pk_lo(v), pk_hi(v));
+  } else {
+    if (lo) stf(p, i, pk_lo(v));
+    if (hi) stf(p, i + 1, pk_hi(v));
+  }
+}
+template <typename T>
+__device__ __forceinline__ bool pair_aligned(const T* p) {
+  return (reinterpret_cast<uintptr_t>(p) & (2 * sizeof(T) - 1)) == 0;
+}
+
+// Column x of one real tile of image `img` (forward-type ops) in the pairs
+// distribution: out[r] = rows 2q, 2q + 1 (+ J r), zero outside the image.
+// Tile origins are even (multiples of the even tile stride), so with even N
+// and an aligned image every pair is one aligned access, wholly inside or
+// wholly outside.
+template <int M, typename T>
+__device__ __forceinline__ void load_tile_column(const T* __restrict__ img, const TileRef& t, int x, int q,
+                                                 pk (&out)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  const int N = t.N;
+  const int gx = t.x0 + x;
+  if (!t.live || gx >= N) {
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) __stcg(dst + TPF * i, z[i]);
+    for (int r = 0; r < R; ++r) out[r] = 0ull;
+    return;
+  }
+  const T* base = img + t.on;
+  const T* col = base + (long long)gx * N + t.y0 + 2 * q;
+  const int rows = N - t.y0 - 2 * q;  // rows available from this thread's first element on
+  if (!(N & 1) && pair_aligned(base)) {
+    if (N - t.y0 >= M) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) out[r] = ld2<true>(col, J * r, true, true);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) out[r] = ld2<true>(col, J * r, J * r < rows, true);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) out[r] = ld2<false>(col, J * r, J * r < rows, J * r + 1 < rows);
   }
 }
 
-// L2 prefetch of the image columns that P1 units xb2 .. xb2+NU-1 of WT w2
-// load (single-field ops: the two tiles of a pair, or E and dE of one
-// tile).  One 128-byte line per thread; only addresses inside the images.
-template <int M, int OP, typename T, int NU>
-__device__ __forceinline__ void p1_prefetch(const OpArgs& a, const Geom& g, int w2, int xb2) {
-  constexpr int C = lpu_of<M>() * NU;                     // columns per field
-  constexpr int RPL = 128 / (int)sizeof(T);              // rows per line
-  constexpr int LC = (M + RPL - 1) / RPL;                 // lines per column
-  static_assert(C * LC <= kThreads / 2, "one line per thread and field");
-  const int h = threadIdx.x / (kThreads / 2), r = threadIdx.x % (kThreads / 2);
-  if (r >= C * LC) return;
-  const TileRef tr = OpTraits<OP>::PAIRS ? tile_of(g, 2 * w2 + h) : tile_of(g, w2);
-  const int gx = tr.x0 + xb2 * lpu_of<M>() + r / LC;
-  const int gy = tr.y0 + (r % LC) * RPL;
-  if (!tr.live || gx >= tr.N || gy >= tr.N) return;
-  const T* img = static_cast<const T*>(OpTraits<OP>::PAIRS || h == 0 ? a.E : a.dE);
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(img + tr.on + (long long)gx * tr.N + gy));
+// The four columns 4 blk .. of the two real tiles of a single-field op, by
+// bulk copies: column c of tile h lands at element (4 h + c) column pitches,
+// a pitch of 8 (mod 32) words so that the pair reads are free of bank
+// conflicts.  Needs 16-byte pieces: N and the tile origin multiples of 16
+// bytes and an aligned image (else false, and nothing is issued).
+template <int M, typename T>
+__host__ __device__ constexpr int bulk_pitch() { return M + 32 / (int)sizeof(T); }
+template <int M, typename T>
+__device__ __forceinline__ bool load_columns_bulk(const T* const (&img)[2], const TileRef (&tr)[2], int blk,
+                                                  GroupMem<M>& gm, cpk (&z)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  constexpr int CP = bulk_pitch<M, T>();
+  constexpr int EPC = 16 / (int)sizeof(T);
+  static_assert(8 * CP * sizeof(T) <= exch_bytes<M>(), "the columns land in the exchange");
+  T* st = reinterpret_cast<T*>(gm.ex);
+  int rows[2], cols[2];
+  bool ok = true;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int N = tr[h].N;
+    rows[h] = max(0, min(M, N - tr[h].y0));
+    cols[h] = tr[h].live ? max(0, min(kLines, N - tr[h].x0 - blk * kLines)) : 0;
+    ok = ok && N % EPC == 0 && tr[h].y0 % EPC == 0 && (reinterpret_cast<uintptr_t>(img[h] + tr[h].on) & 15) == 0;
+  }
+  if (!ok) return false;
+  gm.open();
+  if (gm.leader()) {
+    tc::mbar_expect_tx(gm.bar, (unsigned)((cols[0] * rows[0] + cols[1] * rows[1]) * sizeof(T)));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const T* src = img[h] + tr[h].on + (long long)(tr[h].x0 + blk * kLines) * tr[h].N + tr[h].y0;
+      for (int c = 0; c < (rows[h] ? cols[h] : 0); ++c, src += tr[h].N)
+        tc::bulk_g2s(st + (kLines * h + c) * CP, src, (unsigned)(rows[h] * sizeof(T)), gm.bar);
+    }
+  }
+  gm.wait(0);
+  const T* c0 = st + gm.t.line * CP + 2 * gm.t.q;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int y = 2 * gm.t.q + J * r;
+    z[r].re = gm.t.line < cols[0] && y < rows[0] ? swin2(c0 + J * r) : 0ull;
+    z[r].im = gm.t.line < cols[1] && y < rows[1] ? swin2(c0 + kLines * CP + J * r) : 0ull;
+  }
+  return true;
 }
 
-// The same for the adjoint-type P1 unit xb of WT w2: the v (and dv) columns
-// and the f (and df) columns around them that load_adj_column reads, for
-// both tiles of the pair; one 128-byte line per thread and iteration.
+// The field(s) of a single-field op at tile column x: the two tiles of a
+// pair, or g and dg of one tile, as re / im.
+template <int M, int OP, typename T>
+__device__ __forceinline__ void load_column(const OpArgs& a, const Geom& g, int w, int blk, GroupMem<M>& gm,
+                                            cpk (&z)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R;
+  constexpr bool PAIRS = OpTraits<OP>::PAIRS;
+  static_assert(OpTraits<OP>::K == 1, "single-field ops");
+  const TileRef tr[2] = {tile_of(g, PAIRS ? 2 * w : w), tile_of(g, PAIRS ? 2 * w + 1 : w)};
+  const T* const img[2] = {static_cast<const T*>(a.E), static_cast<const T*>(PAIRS ? a.E : a.dE)};
+  if (load_columns_bulk<M, T>(img, tr, blk, gm, z)) return;
+  const int x = blk * kLines + gm.t.line;
+  pk re[R], im[R];
+  load_tile_column<M, T>(img[0], tr[0], x, gm.t.q, re);
+  load_tile_column<M, T>(img[1], tr[1], x, gm.t.q, im);
+#pragma unroll
+  for (int r = 0; r < R; ++r) z[r] = cpk{re[r], im[r]};
+}
+
+// Central differences (times 2) of f at a pair of rows of the column at fc:
+// gx = f[+n] - f[-n], gy = f[+1] - f[-1].  MODE 1: fc at an even offset of an
+// aligned array of even column length (one access per pair of a side
+// column); 2: at an odd offset (the row pairs around it are aligned); 0:
+// neither.  Predicates as in ld2 (equal in modes 1 and 2).
+template <int MODE, typename T>
+__device__ __forceinline__ void diff2(const T* __restrict__ fc, int n, int o, bool lo, bool hi, pk& gx, pk& gy) {
+  gx = pk_sub(ld2<MODE == 1>(fc + n, o, lo, hi), ld2<MODE == 1>(fc - n, o, lo, hi));
+  if constexpr (MODE == 2) {
+    gy = pk_sub(ld2<true>(fc, o + 1, lo, hi), ld2<true>(fc, o - 1, lo, hi));
+  } else {
+    const float m = lo ? ldf(fc, o - 1) : 0.f, p = hi ? ldf(fc, o + 2) : 0.f;
+    // the pair (f[o], f[o + 1]): f[o] serves the high lane, f[o + 1] the low one
+    const pk c = ld2<MODE == 1>(fc, o, hi, lo);
+    gy = pk_make(__fsub_rn(pk_hi(c), m), __fsub_rn(p, pk_lo(c)));
+  }
+}
+
+// One tile's adjoint-type fields at tile column x (erosion >= 1: every
+// gradient neighbour of the valid window lies inside the image), written to
+// the re (LANE 0) or im (LANE 1) parts of hx and hy: h = v * df / dx,
+// or dv * df / dx + v * d(df) / dx for the tangent-adjoint (TAN).
+template <int M, typename T, bool TAN, int LANE, int MODE>
+__device__ __forceinline__ void load_adj_tile(const OpArgs& a, const TileRef& tr, int x, int q,
+                                              cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  const int qx = tr.x0 + x - a.e, ox = qx - a.e;  // image / valid-window column
+  const bool on = tr.live && ox >= 0 && ox < tr.W;
+  const int qy0 = tr.y0 + 2 * q - a.e, oy0 = qy0 - a.e;
+  const long long vo = tr.ow + (long long)ox * tr.W + oy0;
+  const long long fo = tr.on + (long long)qx * tr.N + qy0;
+  const T* v = static_cast<const T*>(a.v) + vo;
+  const T* f = static_cast<const T*>(a.I) + fo;
+  const T* dv = TAN ? static_cast<const T*>(a.dv) + vo : v;
+  const T* df = TAN ? static_cast<const T*>(a.dI) + fo : f;
+  const pk half = pk_dup(0.5f);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int o = J * r;
+    const bool lo = on && (unsigned)(oy0 + o) < (unsigned)tr.W;
+    const bool hi = MODE ? lo : on && (unsigned)(oy0 + o + 1) < (unsigned)tr.W;
+    pk gx, gy;
+    diff2<MODE>(f, tr.N, o, lo, hi, gx, gy);
+    gx = pk_mul(gx, half);
+    gy = pk_mul(gy, half);
+    const pk vv = ld2<MODE != 0>(v, o, lo, hi);
+    pk rx, ry;
+    if constexpr (TAN) {
+      pk dgx, dgy;
+      diff2<MODE>(df, tr.N, o, lo, hi, dgx, dgy);
+      const pk dvv = ld2<MODE != 0>(dv, o, lo, hi);
+      rx = pk_dot2(dvv, gx, vv, pk_mul(dgx, half));
+      ry = pk_dot2(dvv, gy, vv, pk_mul(dgy, half));
+    } else {
+      rx = pk_mul(vv, gx);
+      ry = pk_mul(vv, gy);
+    }
+    (LANE ? hx[r].im : hx[r].re) = rx;
+    (LANE ? hy[r].im : hy[r].re) = ry;
+  }
+}
+// The fields of one tile in the tested form: any erosion (0 included, where
+// gradient neighbours may lie outside the image), one value at a time.
+template <int M, typename T, int LANE>
+__device__ __forceinline__ void load_adj_tested(const OpArgs& a, const TileRef& tr, int x, int q,
+                                                cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int px = tr.x0 + x, py = tr.y0 + 2 * q + J * r;
+    const pk vx = tr.live ? pk_make(h_at<T>(a, tr, 0, px, py), h_at<T>(a, tr, 0, px, py + 1)) : 0ull;
+    const pk vy = tr.live ? pk_make(h_at<T>(a, tr, 1, px, py), h_at<T>(a, tr, 1, px, py + 1)) : 0ull;
+    (LANE ? hx[r].im : hx[r].re) = vx;
+    (LANE ? hy[r].im : hy[r].re) = vy;
+  }
+}
+template <int M, typename T, bool TAN, bool TESTED, int LANE>
+__device__ __forceinline__ void load_adj_lane(const OpArgs& a, const Geom& g, int w, int x, int q,
+                                              cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  const TileRef tr = tile_of(g, 2 * w + LANE);
+  if constexpr (TESTED) {
+    load_adj_tested<M, T, LANE>(a, tr, x, q, hx, hy);
+    return;
+  }
+  const bool al = !(tr.N & 1) && pair_aligned(static_cast<const T*>(a.v) + tr.ow) &&
+                  pair_aligned(static_cast<const T*>(a.I) + tr.on) &&
+                  (!TAN || (pair_aligned(static_cast<const T*>(a.dv) + tr.ow) &&
+                            pair_aligned(static_cast<const T*>(a.dI) + tr.on)));
+  if (!al)
+    load_adj_tile<M, T, TAN, LANE, 0>(a, tr, x, q, hx, hy);
+  else if (a.e & 1)
+    load_adj_tile<M, T, TAN, LANE, 2>(a, tr, x, q, hx, hy);
+  else
+    load_adj_tile<M, T, TAN, LANE, 1>(a, tr, x, q, hx, hy);
+}
+
+// ---- P1 ------------------------------------------------------------------------------------
+// L2 prefetch of the inputs of the adjoint-type unit xb2 of WT w2: the v
+// (and dv) columns and the f (and df) columns around them, for both tiles of
+// the pair, one 128-byte line per thread and step; only addresses inside.
 template <int M, typename T>
 __device__ __forceinline__ void p1_prefetch_adj(const OpArgs& a, const Geom& g, int w2, int xb2) {
-  constexpr int LPU = lpu_of<M>();
+  constexpr int C = unit_lines<M>();
   constexpr int RPL = 128 / (int)sizeof(T);
   constexpr int LV = (M + RPL - 1) / RPL + 1;      // lines of a v column (start not line-aligned)
   constexpr int LF = (M + 2 + RPL - 1) / RPL + 1;  // lines of an f column
-  constexpr int PER = LPU * LV + (LPU + 2) * LF;   // per tile and array pair
+  constexpr int PER = C * LV + (C + 2) * LF;       // per tile and array pair
   const int npair = a.dI != nullptr ? 2 : 1;
   const int e = a.e;
-  for (int idx = threadIdx.x; idx < 2 * PER * npair; idx += kThreads) {
-    const int d = idx / (2 * PER), h = (idx / PER) & 1, r = idx % PER;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
     const TileRef tr = tile_of(g, 2 * w2 + h);
     if (!tr.live) continue;
-    const int x = tr.x0 + xb2 * LPU;
-    if (r < LPU * LV) {
-      const int col = x + r / LV - 2 * e, row0 = tr.y0 - 2 * e;
-      const int row = max(row0, 0) + (r % LV) * RPL;
-      if (col < 0 || col >= tr.W || row >= tr.W || row >= row0 + M) continue;
-      const T* v = static_cast<const T*>(d ? a.dv : a.v);
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(v + tr.ow + (long long)col * tr.W + row));
-    } else {
-      const int rf = r - LPU * LV;
-      const int col = x + rf / LF - e - 1, row0 = tr.y0 - e - 1;
-      const int row = max(row0, 0) + (rf % LF) * RPL;
-      if (col < 0 || col >= tr.N || row >= tr.N || row >= row0 + M + 2) continue;
-      const T* f = static_cast<const T*>(d ? a.dI : a.I);
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(f + tr.on + (long long)col * tr.N + row));
-    }
-  }
-}
-
-// P1: line `line` transforms column x = xb*LPU + line of every field along
-// y.  NU consecutive units (xb, xb+1, ...) per call, single-field ops only:
-// the next unit's columns are loaded before the current transform, so their
-// latency overlaps it, and the columns of the CTA `ahead` launch positions
-// later (about one per SM: it starts when this one is nearly done) are
-// prefetched into L2.
-template <int M, int OP, typename T, int NU = 1, bool TAN = false>
-__device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, int xb, float2* __restrict__ S1,
-                                       float2* __restrict__ rows, const float2* __restrict__ tw, int line, int t,
-                                       int ahead = 0, float2* __restrict__ stash = nullptr) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  constexpr int K = OpTraits<OP>::K;
-  constexpr int LPU = lpu_of<M>();
-  constexpr int RS = row_stride<M>();
-  static_assert(NU == 1 || (NU == 2 && K == 1), "two units per call for single-field ops only");
-  float2* row = rows + line * RS;
-  if constexpr (NU == 2) {
-    if (ahead > 0) {
-      const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
-      p1_prefetch<M, OP, T, NU>(a, g, w - (int)blockIdx.y + lin / (int)gridDim.x, (lin % (int)gridDim.x) * NU);
-    }
-    float2 za[EPT], zb[EPT];
-    load_column<M, OP, T>(a, g, w, 0, xb * LPU + line, t, za);
-    load_column<M, OP, T>(a, g, w, 0, (xb + 1) * LPU + line, t, zb);
-    fft<M, false>(za, row, tw, t, 1 + line);
-    p1_store<M>(za, S1, xb, rows, line, t);
-    fft<M, false>(zb, row, tw, t, 1 + line);
-    p1_store<M>(zb, S1, xb + 1, rows, line, t);
-  } else {
-    if constexpr (OP == OP_ADJ) {
-      // both fields from one pass over the inputs; h_y waits in the
-      // stash (kThreads x EPT values after the rows, each thread its own)
-      if (stash && a.e >= 1) {
-        if (ahead > 0) {
-          const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
-          p1_prefetch_adj<M, T>(a, g, w - (int)blockIdx.y + lin / (int)gridDim.x, lin % (int)gridDim.x);
-        }
-        float2 zx[EPT];
-        float2* st = stash + threadIdx.x;
-        load_adj_column<M, T, TAN>(a, g, w, xb * LPU + line, t, zx, st);
-        fft<M, false>(zx, row, tw, t, 1 + line);
-        p1_store<M>(zx, S1, xb, rows, line, t);
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) zx[i] = st[kThreads * i];
-        fft<M, false>(zx, row, tw, t, 1 + line);
-        p1_store<M>(zx, S1 + (size_t)M * M, xb, rows, line, t);
-        return;
+    const int x = tr.x0 + xb2 * C;
+    for (int idx = threadIdx.x; idx < PER * npair; idx += kThreads) {
+      const int d = idx / PER, r = idx % PER;
+      if (r < C * LV) {
+        const int col = x + r / LV - 2 * e, row0 = tr.y0 - 2 * e;
+        const int row = max(row0, 0) + (r % LV) * RPL;
+        if (col < 0 || col >= tr.W || row >= tr.W || row >= row0 + M) continue;
+        const T* v = static_cast<const T*>(d ? a.dv : a.v);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v + tr.ow + (long long)col * tr.W + row));
+      } else {
+        const int rf = r - C * LV;
+        const int col = x + rf / LF - e - 1, row0 = tr.y0 - e - 1;
+        const int row = max(row0, 0) + (rf % LF) * RPL;
+        if (col < 0 || col >= tr.N || row >= tr.N || row >= row0 + M + 2) continue;
+        const T* f = static_cast<const T*>(d ? a.dI : a.I);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(f + tr.on + (long long)col * tr.N + row));
       }
     }
-#pragma unroll 1
-    for (int k = 0; k < K; ++k) {
-      float2 z[EPT];
-      load_column<M, OP, T>(a, g, w, k, xb * LPU + line, t, z);
-      fft<M, false>(z, row, tw, t, 1 + line);
-      p1_store<M>(z, S1 + (size_t)k * M * M, xb, rows, line, t);
-    }
   }
 }
 
-// Transposing copy of an M x LPU block (M lines of LPU consecutive complex
-// values, line pitch `pitch`) into LPU staging rows of M values each.  All
-// threads of the CTA take part; every load is in flight before the
-// scattered shared stores.
+// The transform of column x (ky = k_i + R m) -> S1[ky/4][x][ky%4].
 template <int M>
-__device__ __forceinline__ void stage_rows(const float2* __restrict__ src, int pitch, float2* __restrict__ rows) {
-  constexpr int RS = row_stride<M>();
-  constexpr int LPU = lpu_of<M>();
-  constexpr int Q = LPU / 2;                 // float4 per line
-  constexpr int NIT = M * Q / kThreads;      // float4 loads per thread
-  static_assert(M * Q % kThreads == 0, "staging loop must divide evenly");
-  // element j of this thread: line y0 + j*YS, value pair cp (YS is a multiple
-  // of 16, so fft_pad(y0 + j*YS) = fft_pad(y0) + fft_pad(j*YS))
-  constexpr int YS = kThreads / Q;
-  static_assert(YS % 16 == 0, "line step must keep the padding separable");
-  const int y0 = threadIdx.x / Q, cp = threadIdx.x % Q;
-  const float4* sp = reinterpret_cast<const float4*>(src + (size_t)y0 * pitch + 2 * cp);
-  const size_t sstep = (size_t)YS * pitch / 2;  // float4 per j (pitch is even)
-  float4 q[NIT];
+__device__ __forceinline__ void p1_store(const float2 (&X)[Quad<M>::VPT], float2* __restrict__ S1k, int x, int q) {
+  using Q = Quad<M>;
 #pragma unroll
-  for (int j = 0; j < NIT; ++j) q[j] = __ldcg(sp + j * sstep);
-  float2* r0 = rows + (2 * cp) * RS + fft_pad(y0);
-  float2* r1 = r0 + RS;
+  for (int i = 0; i < Q::KPT; ++i) {
+    const int k = q + Q::TPL * i;
+    float2* dst = S1k + (size_t)(k >> 2) * (4 * M) + x * 4 + (k & 3);
 #pragma unroll
-  for (int j = 0; j < NIT; ++j) {
-    r0[fft_pad(j * YS)] = make_float2(q[j].x, q[j].y);
-    r1[fft_pad(j * YS)] = make_float2(q[j].z, q[j].w);
+    for (int m = 0; m < Q::J; ++m) __stcg(dst + (size_t)m * (Q::R / 4) * (4 * M), X[i * Q::J + m]);
   }
 }
 
-// stage_rows for a rotated S2 block (the tensor-core row pass's layout):
-// block line y holds frequency row (y - rot) mod M, which lands in the rows
-// at that index.  Rotating the lines by the column block spreads the row
-// pass's 32-byte pieces of one ky over the L2 instead of stacking them at one
-// offset of blocks 16 KB apart.
-template <int M>
-__device__ __forceinline__ void stage_rows_rot(const float2* __restrict__ src, int rot, float2* __restrict__ rows) {
-  constexpr int RS = row_stride<M>();
-  constexpr int LPU = lpu_of<M>();
-  constexpr int Q = LPU / 2;
-  constexpr int NIT = M * Q / kThreads;
-  constexpr int YS = kThreads / Q;
-  const int y0 = threadIdx.x / Q, cp = threadIdx.x % Q;
-  const float4* sp = reinterpret_cast<const float4*>(src + (size_t)y0 * LPU + 2 * cp);
-  constexpr size_t sstep = (size_t)YS * LPU / 2;
-  float4 q[NIT];
-#pragma unroll
-  for (int j = 0; j < NIT; ++j) q[j] = __ldcg(sp + j * sstep);
-  float2* r0 = rows + (2 * cp) * RS;
-  float2* r1 = r0 + RS;
-#pragma unroll
-  for (int j = 0; j < NIT; ++j) {
-    const int ky = (y0 + j * YS - rot) & (M - 1);
-    r0[fft_pad(ky)] = make_float2(q[j].x, q[j].y);
-    r1[fft_pad(ky)] = make_float2(q[j].z, q[j].w);
+// P1: the group transforms columns 4 blk .. 4 blk + 3 of every field along y.
+// OP_ADJ: TAN when dv and df are given; TESTED for erosion 0 (any TAN).
+template <int M, int OP, typename T, bool TAN = false, bool TESTED = false>
+__device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, int blk, float2* __restrict__ S1,
+                                       GroupMem<M>& gm, const float4* __restrict__ tw) {
+  using Q = Quad<M>;
+  const QuadThread t = gm.t;
+  const int x = blk * kLines + t.line;
+  float2 X[Q::VPT];
+  if constexpr (OP == OP_ADJ) {
+    // both fields from one pass over the inputs; h_y waits in registers
+    cpk hx[Q::R], hy[Q::R];
+    load_adj_lane<M, T, TAN, TESTED, 0>(a, g, w, x, t.q, hx, hy);
+    load_adj_lane<M, T, TAN, TESTED, 1>(a, g, w, x, t.q, hx, hy);
+    fft_dit<M, false>(hx, X, gm.ex, tw, t);
+    p1_store<M>(X, S1, x, t.q);
+    fft_dit<M, false>(hy, X, gm.ex, tw, t);
+    p1_store<M>(X, S1 + (size_t)M * M, x, t.q);
+  } else {
+    cpk z[Q::R];
+    load_column<M, OP, T>(a, g, w, blk, gm, z);
+    fft_dit<M, false>(z, X, gm.ex, tw, t);
+    p1_store<M>(X, S1, x, t.q);
   }
 }
 
-// P2: rows ky0 .. ky0+LPU-1: FFT along x, spectral map, inverse, keep the
-// valid columns, write S2 rows.  All threads of the CTA take part.
+// ---- P2 ------------------------------------------------------------------------------------
+// P2: rows ky = 4 blk .. 4 blk + 3: FFT along x, spectral map, inverse, keep
+// the valid columns.
 template <int M, int OP>
 __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __restrict__ S2,
-                                       const float2* __restrict__ Gx, const float2* __restrict__ Gy, int conjG,
-                                       const Geom& g, int ky0, float2* __restrict__ rows,
-                                       const float2* __restrict__ tw, int line, int t, float2* __restrict__ tile) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  constexpr int RSP = TPF + TPF / 16;
+                                       const float4* __restrict__ Gx, const float4* __restrict__ Gy, int conjG,
+                                       const Geom& g, int blk, GroupMem<M>& gm, const float4* __restrict__ tw) {
+  using Q = Quad<M>;
   constexpr int K = OpTraits<OP>::K;
-  constexpr int RS = row_stride<M>();
-  constexpr int LPU = lpu_of<M>();
-  const int S = g.S, e = g.e, P = s2_pitch(S);
-  const int bar = 1 + line;
-  // S1[k][x][ky0 + c]: a transposing copy of LPU consecutive ky of every column x
+  constexpr unsigned BB = (unsigned)block_bytes<M>();
+  const QuadThread t = gm.t;
+  const int S = g.S, e = g.e, P = s2_pitch(S), xa = s2_first(e);
+  const size_t row = (size_t)blk * (kLines * M);  // complex values before this block of rows
+  const float4* gb = reinterpret_cast<const float4*>(gm.buf);
+  // row ky of a staged S1 block: x = k_i + R m
+  auto load = [&](const void* blkmem, float2 (&X)[Q::VPT]) {
+    const float2* src = static_cast<const float2*>(blkmem) + t.line + 4 * t.q;
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if constexpr (s1_blocked<M>())
-      stage_rows<M>(S1 + (size_t)k * M * M + (size_t)ky0 * M, LPU, rows + k * LPU * RS);
-    else
-      stage_rows<M>(S1 + (size_t)k * M * M + ky0, M, rows + k * LPU * RS);
-  }
-  __syncthreads();
-  const int ky = ky0 + line;
-  float2* row0 = rows + line * RS;           // field 0 / exchange
-  float2* row1 = rows + (LPU + line) * RS;   // field 1 or the stash
-  const float2* gxr = Gx + (size_t)ky * M + t;
-  const float2* gyr = Gy + (size_t)ky * M + t;
-  auto spec = [&](float2 z, float2 G) { return conjG ? cmulc(z, G) : cmul(z, G); };
-  // valid columns of field l -> the shared block tile -> whole LPU x LPU
-  // blocks of S2 (16-byte stores, each block one contiguous run)
-  constexpr int PB = s2_block_pitch<M>();
-  constexpr int F4B = LPU * LPU / 2;  // float4 per block
-  const int nblk = P / LPU;
-  auto emit = [&](const float2 (&o)[EPT], int l) {
-    if constexpr (!s2_blocked<M>()) {
-      float2* dst = S2 + ((size_t)l * M + ky) * P - e + t;
+    for (int i = 0; i < Q::KPT; ++i)
 #pragma unroll
-      for (int i = 0; i < EPT; ++i) {
-        const int xv = t + TPF * i - e;
-        if (xv >= 0 && xv < S) __stcg(dst + TPF * i, o[i]);
-      }
-      return;
-    }
-    {
-      // xv = xb0 + TPF*i lies in block floor(xb0 / LPU) + i*TPF/LPU at
-      // position xb0 mod LPU (an arithmetic shift and a mask also for the
-      // negative xb0 of the columns left of the valid range, never stored)
-      const int xb0 = t - e;
-      constexpr int LS = LPU == 4 ? 2 : 3;
-      float2* tl = tile + (xb0 >> LS) * PB + line * LPU + (xb0 & (LPU - 1));
-#pragma unroll
-      for (int i = 0; i < EPT; ++i)
-        if ((unsigned)(xb0 + TPF * i) < (unsigned)S) tl[(TPF / LPU) * PB * i] = o[i];
-    }
-    __syncthreads();
-    // thread: value pair w of blocks q = q0, q0 + QS, ... (QS blocks per sweep)
-    constexpr int QS = kThreads / F4B;
-    const int q0 = threadIdx.x / F4B, w = threadIdx.x % F4B;
-    float4* dst = reinterpret_cast<float4*>(S2 + ((size_t)l * nblk * M + ky0) * LPU + (size_t)q0 * M * LPU + 2 * w);
-    const float4* src = reinterpret_cast<const float4*>(tile + q0 * PB + 2 * w);
-    for (int q = q0; q < nblk; q += QS, dst += (size_t)QS * M * LPU / 2, src += QS * PB / 2) __stcg(dst, *src);
-    __syncthreads();  // the tile is reused by the next field
+      for (int m = 0; m < Q::J; ++m) X[i * Q::J + m] = src[4 * (Q::TPL * i + Q::R * m)];
   };
-  float2 z[EPT];
-  row_to_regs<M>(row0, z, t);
-  fft<M, false>(z, row0, tw, t, bar);
-  if constexpr (K == 1) {
-    // both spectral products at once; Z*Gy waits in the line's second row
-    // (each thread rereads only its own elements)
-    float2* st = row1 + t + (t >> 4);
+  // spectrum quad of kx = 2q, 2q + 1 (+ J r): quad index 4 (q + J r / 2) + line of the block
+  const int go = 4 * t.q + t.line;
+  auto spec = [&](const float4* __restrict__ G, int r) {
+    cpk v = cpk_load(__ldg(G + row / 2 + go + r * (2 * Q::J)));
+    if (conjG) v.im = pk_neg(v.im);
+    return v;
+  };
+  auto emit = [&](const float2 (&X)[Q::VPT], int l) {
+    float2* dst0 = S2 + (size_t)l * M * P + (size_t)(blk * kLines + t.line) * 4;
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      const float2 zi = z[i];
-      st[RSP * i] = spec(zi, __ldg(gyr + TPF * i));
-      z[i] = spec(zi, __ldg(gxr + TPF * i));
+    for (int i = 0; i < Q::KPT; ++i) {
+      const int k = t.q + Q::TPL * i;
+      float2* dst = dst0 + ((k >> 2) - (xa >> 2)) * (4 * M) + (k & 3);
+#pragma unroll
+      for (int m = 0; m < Q::J; ++m)
+        if ((unsigned)(k + Q::R * m - e) < (unsigned)S) __stcg(dst + m * (Q::R / 4) * (4 * M), X[i * Q::J + m]);
     }
-    fft<M, true>(z, row0, tw, t, bar);
-    emit(z, 0);
+  };
+  float2 X[Q::VPT];
+  cpk z[Q::R], b[Q::R];
+  gm.open();
+  gm.fetch(0, gm.ex, S1 + row, BB);
+  if constexpr (K == 1) {
+    gm.fetch(1, gm.buf, Gx + row / 2, BB);
+    gm.wait(0);
+    load(gm.ex, X);
+    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
+    fft_dif_finish<M, false>(z);
+    gm.wait(1);
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) z[i] = st[RSP * i];
-    fft<M, true>(z, row0, tw, t, bar);
-    emit(z, 1);
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], cpk_load(gb[go + r * (2 * Q::J)]));
+    gm.open();
+    gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the first inverse
+    fft_dit<M, true>(b, X, gm.ex, tw, t);
+    emit(X, 0);
+    gm.wait(1);
+#pragma unroll
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], cpk_load(gb[go + r * (2 * Q::J)]));
+    fft_dit<M, true>(b, X, gm.ex, tw, t);
+    emit(X, 1);
   } else {
-    group_sync<TPF>(bar);
-    regs_to_row<M>(row0, z, t);  // stash Z0(ky, .) in its own row
-    row_to_regs<M>(row1, z, t);
-    fft<M, false>(z, row1, tw, t, bar);
-    const float2* st = row0 + t + (t >> 4);
+    gm.fetch(1, gm.buf, S1 + (size_t)M * M + row, BB);
+    gm.wait(0);
+    load(gm.ex, X);
+    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
+    fft_dif_finish<M, false>(z);
 #pragma unroll
-    for (int i = 0; i < EPT; ++i)
-      z[i] = cadd(spec(st[RSP * i], __ldg(gxr + TPF * i)), spec(z[i], __ldg(gyr + TPF * i)));
-    fft<M, true>(z, row1, tw, t, bar);
-    emit(z, 0);
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(Gx, r));
+    gm.wait(1);
+    load(gm.buf, X);
+    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
+    fft_dif_finish<M, false>(z);
+#pragma unroll
+    for (int r = 0; r < Q::R; ++r) {
+      const cpk c = cpk_mul<false>(z[r], spec(Gy, r));
+      b[r] = cpk{pk_add(b[r].re, c.re), pk_add(b[r].im, c.im)};
+    }
+    fft_dit<M, true>(b, X, gm.ex, tw, t);
+    emit(X, 0);
   }
 }
 
-// P3: columns x' = xb*LPU .. +LPU-1: stage them, inverse FFT along ky,
-// epilogue.  All threads of the CTA take part (lines without a valid column
-// still join the barriers).  For the forward and tangent epilogues with
-// erosion >= 1 the image columns the central differences need are staged in
-// shared memory after the transforms, in the rows they no longer use.
-// S2 layouts P3 reads: the engine's (blocked for M = 512), the blocked one
-// with rotated lines, or the plain one [field][ky][P] (the latter two written
-// by the tensor-core row pass).
-enum S2Layout : int { kS2Engine = 0, kS2Rotated = 1, kS2Plain = 2 };
-template <int M, int OP, typename T, bool ASYNC = false, int S2L = kS2Engine>
-__device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpArgs& a, const Geom& g, int w, int xb,
-                                       float2* __restrict__ rows, const float2* __restrict__ tw, int line, int t,
-                                       T* __restrict__ win0 = nullptr) {
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
+// ---- P3 ------------------------------------------------------------------------------------
+// Gradient windows (forward and tangent).  The four output columns of a
+// group need the image columns gx - 1 .. gx + 4 and rows y0 + e - 1 ..
+// y0 + e + S: kWinCols columns of raw storage values in shared memory,
+// window column c <-> image column gx0 + c, element i <-> image row gya + i,
+// gya <= y0 + e - 1 even, so that the pair of rows (y, y + 1), y even, is one
+// aligned access.  Out-of-image elements are zero (the central-difference
+// rule).  Column pitch: 8 (mod 32) 4-byte words, so the pair reads of a
+// half-warp (four indices of four lines) fall on distinct banks.
+constexpr int kWinCols = kLines + 2;
+// Bytes before a window that reads of the rows above the first output reach:
+// less than e <= M / 2 elements.
+template <int M>
+__host__ __device__ constexpr size_t win_lead() { return 2 * (size_t)M; }
+template <typename T>
+__host__ __device__ constexpr int win_pitch(int S) {
+  // holds off + S + 2 elements, off = y0 + e - 1 - gya < 16 / sizeof(T)
+  return sizeof(T) == 4 ? (S + 5 + 23) / 32 * 32 + 8 : (S + 9 + 47) / 64 * 64 + 16;
+}
+template <int M, typename T>
+__host__ __device__ constexpr size_t win_bytes() { return (size_t)kWinCols * win_pitch<T>(M) * sizeof(T); }
+
+template <int OP>
+__host__ __device__ constexpr bool grad_op() { return OP == OP_FWD || OP == OP_JVP; }
+// Shared memory of a block in each pass (P1 has one landing zone, P3 of the
+// adjoint one field).
+template <int M>
+__host__ __device__ constexpr size_t p1_smem_bytes() { return groups_of<M>() * group_bytes<M, false>(); }
+template <int M>
+__host__ __device__ constexpr size_t p2_smem_bytes() { return groups_of<M>() * group_bytes<M, true>(); }
+template <int OP>
+__host__ __device__ constexpr bool p3_buf() { return OpTraits<OP>::L == 2; }
+template <int M, int OP>
+__host__ __device__ constexpr size_t p3_smem_bytes() { return groups_of<M>() * group_bytes<M, p3_buf<OP>()>(); }
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Starts the copy of one window (16-byte asynchronous chunks where every
+// chunk lies wholly inside or outside the image: N a multiple of the chunk,
+// an aligned image, first row inside; else 4-byte asynchronous copies, or
+// plain ones for 2-byte values) and returns gya.  One commit group.
+template <int M, typename T>
+__device__ __forceinline__ int issue_window(const T* __restrict__ img, const TileRef& tr, int gx0, int e, int S,
+                                            T* __restrict__ win) {
+  constexpr int EPC = 16 / (int)sizeof(T);
+  constexpr int GT = Quad<M>::GT;
+  const int N = tr.N, HP = win_pitch<T>(S);
+  const int gy0 = tr.y0 + e - 1;
+  const int t = threadIdx.x % GT;
+  const bool vec = N % EPC == 0 && gy0 >= 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
+  const int gya = vec ? gy0 - gy0 % EPC : gy0 - (gy0 & 1);
+  const int nel = gy0 - gya + S + 2;
+  if (tr.live) {
+#pragma unroll 1
+    for (int c = 0; c < kWinCols; ++c) {
+      const int gx = gx0 + c;
+      const bool colin = gx >= 0 && gx < N;
+      const T* col = img + (long long)(colin ? gx : 0) * N + gya;
+      T* d = win + c * HP;
+      if (vec) {
+        const int lim = colin ? N - gya : 0;  // elements of this column inside the image
+        for (int i = EPC * t; i < nel; i += EPC * GT) {
+          const bool in = i < lim;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                           static_cast<unsigned>(__cvta_generic_to_shared(d + i))),
+                       "l"(in ? col + i : img), "r"(in ? 16 : 0)
+                       : "memory");
+        }
+      } else {
+        for (int i = t; i < nel; i += GT) {
+          const int gy = gya + i;
+          const bool in = colin && gy >= 0 && gy < N;
+          if constexpr (sizeof(T) == 4)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                             static_cast<unsigned>(__cvta_generic_to_shared(d + i))),
+                         "l"(in ? col + i : img), "r"(in ? 4 : 0)
+                         : "memory");
+          else
+            d[i] = in ? col[i] : T(0.f);
+        }
+      }
+    }
+  }
+  cp_async_commit();
+  return gya;
+}
+
+// This thread's output column of one tile: rows y = 2q + l + J r of tile
+// column x are outputs for e <= y < e + cnt.
+struct OutCol {
+  bool on;        // the column has outputs
+  unsigned cnt;   // valid rows
+  int rel;        // 2q - e: row 2q relative to the first valid one
+  long long off;  // element offset of row 2q in the output batch array
+};
+template <int M>
+__device__ __forceinline__ OutCol out_col(const Geom& g, const TileRef& tr, int x, int q, bool nsized) {
+  OutCol o;
+  const int ox = tr.x0 + x - g.e;
+  o.on = tr.live && x >= g.e && x < g.e + g.S && ox < tr.Wout;
+  o.cnt = (unsigned)max(0, min(g.S, tr.Wout - tr.y0));
+  o.rel = 2 * q - g.e;
+  o.off = (nsized ? tr.on + (long long)ox * tr.N : tr.ow + (long long)ox * tr.W) + tr.y0 + o.rel;
+  return o;
+}
+// Every pair of rows is one aligned access, wholly valid or wholly not.
+__device__ __forceinline__ bool out_even(const Geom& g, const TileRef& tr) { return !((g.e | tr.Wout) & 1); }
+
+// Forward / tangent epilogue, round h, with the central differences read
+// from the staged window.  FWD: round h finishes image h of the pair.  JVP:
+// round 0 (window = f) leaves the f terms in u0.im, round 1 (window = df)
+// adds the df terms.
+template <int M, int OP, typename T, bool VEC>
+__device__ __forceinline__ void grad_round(const OpArgs& a, const OutCol& o, int line, int q, int h, int row0,
+                                           const T* __restrict__ win, int HP, cpk (&u0)[Quad<M>::R],
+                                           const cpk (&u1)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  // row0: window element of tile row 2q
+  const T* cm = win + line * HP + row0;  // image column gx - 1
+  const T* cc = cm + HP;                 // gx
+  const T* cp = cc + HP;                 // gx + 1
+  T* __restrict__ out = static_cast<T*>(a.out0) + o.off;
+  T* __restrict__ UX = a.out_ux ? static_cast<T*>(a.out_ux) + o.off : nullptr;
+  T* __restrict__ UY = a.out_uy ? static_cast<T*>(a.out_uy) + o.off : nullptr;
+  const pk half = pk_dup(0.5f);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = J * r;
+    const bool lo = (unsigned)(o.rel + i) < o.cnt;
+    const bool hi = VEC ? lo : (unsigned)(o.rel + i + 1) < o.cnt;
+    // every row is computed (no branch between the shared-memory reads of
+    // the rows); rows outside the outputs read neighbouring shared memory
+    // (win_lead) and are not stored
+    const pk dx = pk_sub(swin2(cp + i), swin2(cm + i));
+    const pk c = swin2(cc + i);
+    const pk dy = pk_make(__fsub_rn(pk_hi(c), swin(cc + i - 1)), __fsub_rn(swin(cc + i + 2), pk_lo(c)));
+    // the differences' factor 1/2 is applied once, at the end: halving is exact
+    if constexpr (OP == OP_FWD) {
+      const pk ux = h ? u0[r].im : u0[r].re, uy = h ? u1[r].im : u1[r].re;
+      if (UX) st2<VEC>(UX, i, ux, lo, hi);
+      if (UY) st2<VEC>(UY, i, uy, lo, hi);
+      st2<VEC>(out, i, pk_mul(pk_dot2(ux, dx, uy, dy), half), lo, hi);
+    } else {
+      // srk_tangent_combine (tan_tanadj/srk_tangent.cuh:28-52):
+      // dh = Im(zx) fx + Im(zy) fy + Re(zx) dfx + Re(zy) dfy
+      if (h == 0)
+        u0[r].im = pk_dot2(u0[r].im, dx, u1[r].im, dy);
+      else
+        st2<VEC>(out, i, pk_mul(pk_fma(u1[r].re, dy, pk_fma(u0[r].re, dx, u0[r].im)), half), lo, hi);
+    }
+  }
+}
+
+// The other epilogues.  VJP (f): w = u * v of image h; tangent-adjoint (f):
+// w = dlam * Re + lam * Im; adjoint: the full N x N output of image h.
+template <int M, int OP, typename T, bool VEC>
+__device__ __forceinline__ void plain_epilogue(const OpArgs& a, const OutCol& o, int h, const cpk (&u0)[Quad<M>::R],
+                                               const cpk (&u1)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = J * r;
+    const bool lo = (unsigned)(o.rel + i) < o.cnt;
+    const bool hi = VEC ? lo : (unsigned)(o.rel + i + 1) < o.cnt;
+    if constexpr (OP == OP_ADJ) {
+      st2<VEC>(static_cast<T*>(a.out0) + o.off, i, h ? u0[r].im : u0[r].re, lo, hi);
+    } else {
+      const pk v = ld2<VEC>(static_cast<const T*>(a.v) + o.off, i, lo, hi);
+      pk wx, wy;
+      if constexpr (OP == OP_VJP_F) {
+        wx = pk_mul(h ? u0[r].im : u0[r].re, v);
+        wy = pk_mul(h ? u1[r].im : u1[r].re, v);
+      } else {
+        const pk dv = ld2<VEC>(static_cast<const T*>(a.dv) + o.off, i, lo, hi);
+        wx = pk_dot2(dv, u0[r].re, v, u0[r].im);
+        wy = pk_dot2(dv, u1[r].re, v, u1[r].im);
+      }
+      st2<VEC>(static_cast<float*>(a.out0) + o.off, i, wx, lo, hi);
+      st2<VEC>(static_cast<float*>(a.out1) + o.off, i, wy, lo, hi);
+    }
+  }
+}
+
+// S2 layouts P3 reads: the engine's, first column xa = s2_first(e), or the
+// tensor-core row pass's (hybrid.cu): first column e, the lines of column
+// block b rotated by b.
+enum S2Layout : int { kS2Engine = 0, kS2Rotated = 1 };
+
+// P3: columns 4 blk .. of S2: inverse FFT along ky, epilogue.
+template <int M, int OP, typename T, int S2L = kS2Engine>
+__device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpArgs& a, const Geom& g, int w, int blk,
+                                       GroupMem<M>& gm, const float4* __restrict__ tw) {
+  using Q = Quad<M>;
   constexpr int L = OpTraits<OP>::L;
-  constexpr int RS = row_stride<M>();
-  constexpr int LPU = lpu_of<M>();
-  constexpr bool GRAD = (OP == OP_FWD || OP == OP_JVP);
-  static_assert(!ASYNC || p3_async_window<OP, T>(), "asynchronous window only for the forward / tangent");
-  constexpr int EPC = 16 / (int)sizeof(T);  // storage values per 16-byte copy
+  constexpr bool GRAD = grad_op<OP>();
+  constexpr unsigned BB = (unsigned)block_bytes<M>();
+  // rows below the last output reach less than e elements past a window
+  static_assert(!GRAD || (win_bytes<M, T>() + 2 * win_lead<M>() <= exch_bytes<M>() &&
+                          win_bytes<M, T>() + win_lead<M>() <= block_bytes<M>()),
+                "the windows reuse the buffer (behind the exchange) and the exchange");
+  const QuadThread t = gm.t;
   const int P = s2_pitch(g.S);
-  const int x0 = xb * LPU;
-  const int bar = 1 + line;
-  // window of round h: image (pair member h, or f / df) columns
-  // x0+e-1 .. x0+e+LPU, rows y0+e-1 .. y0+e+S
-  // raw: the asynchronous copy of storage values (else floats staged by the threads)
-  auto window_of = [&](int h, const TileRef& tr, bool vec16, bool raw) {
-    GradWin gw;
-    gw.gx0 = tr.x0 + x0 + a.e - 1;
-    gw.gy0 = tr.y0 + a.e - 1;
-    gw.ncol = LPU + 2;
-    gw.S = g.S;
-    gw.HP = raw ? gwin_pitch_t<T>(g.S) : gwin_pitch(g.S);
-    gw.off = vec16 ? (gw.gy0 % EPC) : 0;
-    return gw;
+  const int xg = (S2L == kS2Rotated ? g.e : s2_first(g.e)) + blk * kLines;  // the group's first tile column
+  const int x = xg + t.line;
+  auto tile_h = [&](int h) { return tile_of(g, OpTraits<OP>::PAIRS ? 2 * w + h : w); };
+  auto image_h = [&](int h, const TileRef& tr) {
+    return static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
   };
-  auto tile_h = [&](int h) { return tile_of(g, OP == OP_FWD ? 2 * w + h : w); };
-  auto image_h = [&](int h) { return static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI); };
-  // 16-byte window copies: N % EPC == 0, a 16-byte aligned image start
-  auto vec16_of = [&](int h, const TileRef& tr) {
-    return ASYNC && tr.N % EPC == 0 &&
-           ((reinterpret_cast<uintptr_t>(image_h(h)) + sizeof(T) * (uintptr_t)tr.on) & 15) == 0;
+  // the windows take the place of the second field (once every thread has
+  // read it) and of the last exchange
+  T* win[2] = {reinterpret_cast<T*>(gm.buf), reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(gm.ex) + win_lead<M>())};
+  int gya[2] = {0, 0};
+  auto window = [&](int h) {
+    const TileRef tr = tile_h(h);
+    gya[h] = issue_window<M, T>(image_h(h, tr), tr, tr.x0 + xg - 1, g.e, g.S, win[h]);
   };
-  auto issue_window = [&](int h, T* dst) {
-    if constexpr (ASYNC) {
-      const TileRef tr = tile_h(h);
-      const bool vec16 = vec16_of(h, tr);
-      if (tr.live) stage_grad_window_async<T>(image_h(h) + tr.on, tr.N, window_of(h, tr, vec16, true), vec16, dst);
-      cp_async_commit();
-    }
-  };
-  // 2-byte storage needs the 16-byte form for both windows; else the
-  // threads stage converted floats (below)
-  bool async_win = false;
-  if constexpr (ASYNC) {
-    async_win = a.e >= 1;
-    if constexpr (!std::is_same<T, float>::value)
-      async_win = async_win && vec16_of(0, tile_h(0)) && vec16_of(1, tile_h(1));
-    if (async_win) issue_window(0, win0);  // in flight during the staging and the transforms
-  }
+  // column x of a staged S2 block: ky = k_i + R m
+  auto load = [&](const void* blkmem, float2 (&X)[Q::VPT]) {
+    const float2* src = static_cast<const float2*>(blkmem) + t.line;
 #pragma unroll
-  for (int l = 0; l < L; ++l) {
-    if constexpr (S2L == kS2Rotated) {
-      static_assert(s2_blocked<M>(), "rotated blocks of the blocked layout");
-      stage_rows_rot<M>(S2 + ((size_t)l * (P / LPU) + xb) * M * LPU, xb & (M - 1), rows + l * LPU * RS);
-    } else if constexpr (s2_blocked<M>() && S2L == kS2Engine)
-      stage_rows<M>(S2 + ((size_t)l * (P / LPU) + xb) * M * LPU, LPU, rows + l * LPU * RS);
-    else
-      stage_rows<M>(S2 + (size_t)l * M * P + x0, P, rows + l * LPU * RS);
-  }
-  __syncthreads();
-  const int xv = x0 + line;
-  const bool active = xv < g.S;
-  float2* row0 = rows + line * RS;
-  float2* row1 = rows + (LPU + line) * RS;
-  float2 z0[EPT], z1[EPT];
-  if (active) {
-    row_to_regs<M>(row0, z0, t);
-    fft<M, true>(z0, row0, tw, t, bar);
-    if constexpr (L == 2) {
-      group_sync<TPF>(bar);
-      regs_to_row<M>(row0, z0, t);   // stash, reread after the second transform
-      row_to_regs<M>(row1, z1, t);
-      fft<M, true>(z1, row1, tw, t, bar);
-    }
-  }
-  if constexpr (L == 1) {
+    for (int i = 0; i < Q::KPT; ++i)
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) z1[i] = make_float2(0.f, 0.f);
-  }
-  if constexpr (ASYNC) {
-    if (async_win) {
-      // window 0 has been arriving in its own buffer; window 1 goes to the
-      // second field's rows once every line is done with them
-      T* win1 = reinterpret_cast<T*>(rows + LPU * RS);
-      float2* z0s = row0 + t + (t >> 4);
-      __syncthreads();
-      issue_window(1, win1);
-      cp_async_wait<1>();
-      __syncthreads();
-      const TileRef tr0 = tile_h(0);
-      if (active)
-        epilogue_staged<M, OP, T, T>(a, g, tr0, xv + g.e, line, t, 0, z0s, z1, win0,
-                                     window_of(0, tr0, vec16_of(0, tr0), true));
-      cp_async_wait<0>();
-      __syncthreads();
-      const TileRef tr1 = tile_h(1);
-      if (active)
-        epilogue_staged<M, OP, T, T>(a, g, tr1, xv + g.e, line, t, 1, z0s, z1, win1,
-                                     window_of(1, tr1, vec16_of(1, tr1), true));
-      return;
-    }
+      for (int m = 0; m < Q::J; ++m) {
+        const int ky = t.q + Q::TPL * i + Q::R * m;
+        X[i * Q::J + m] = src[4 * (S2L == kS2Rotated ? (ky + blk) & (M - 1) : ky)];
+      }
+  };
+  float2 X[Q::VPT];
+  cpk u0[Q::R], u1[Q::R];
+  gm.open();
+  gm.fetch(0, gm.ex, S2 + (size_t)blk * (kLines * M), BB);
+  if constexpr (L == 2) gm.fetch(1, gm.buf, S2 + (size_t)M * P + (size_t)blk * (kLines * M), BB);
+  gm.wait(0);
+  load(gm.ex, X);
+  fft_dif_begin<M, true>(X, u0, gm.ex, tw, t);
+  if constexpr (L == 2) {
+    fft_dif_finish<M, true>(u0);
+    gm.wait(1);
+    load(gm.buf, X);
+    fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
+      if constexpr (GRAD) window(0);
+    });
   }
   if constexpr (GRAD) {
-    if (a.e >= 1) {
-      // two rounds, one image window each, in the second field's rows
-      float* win = reinterpret_cast<float*>(rows + LPU * RS);
-      float2* z0s = row0 + t + (t >> 4);
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        __syncthreads();  // rows of field 1 no longer used (round 0) / window consumed (round 1)
-        const TileRef tr = tile_h(h);
-        const GradWin gw = window_of(h, tr, false, false);
-        if (tr.live) stage_grad_window<T>(image_h(h) + tr.on, tr.N, gw, win);
-        __syncthreads();
-        if (active) epilogue_staged<M, OP, T, float>(a, g, tr, xv + g.e, line, t, h, z0s, z1, win, gw);
+    group_sync<M>();  // the exchange is read: window 1 takes its place
+    window(1);
+    fft_dif_finish<M, true>(u1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 0)
+        cp_async_wait<1>();
+      else
+        cp_async_wait<0>();
+      group_sync<M>();
+      const TileRef tr = tile_h(h);
+      const OutCol o = out_col<M>(g, tr, x, t.q, false);
+      const int row0 = tr.y0 + 2 * t.q - gya[h], HP = win_pitch<T>(g.S);
+      if (!o.on) continue;
+      auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
+      const bool vec = out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy);
+      if (vec)
+        grad_round<M, OP, T, true>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
+      else
+        grad_round<M, OP, T, false>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
+    }
+  } else {
+    fft_dif_finish<M, true>(L == 2 ? u1 : u0);
+    constexpr int NH = OpTraits<OP>::PAIRS ? 2 : 1;
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const TileRef tr = tile_h(h);
+      constexpr bool NS = OP == OP_ADJ;
+      const OutCol o = out_col<M>(g, tr, x, t.q, NS);
+      if (!o.on) continue;
+      bool vec = out_even(g, tr);
+      if constexpr (NS) {
+        vec = vec && pair_aligned(static_cast<const T*>(a.out0) + tr.on);
+      } else {
+        vec = vec && pair_aligned(static_cast<const T*>(a.v) + tr.ow) &&
+              pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
+              pair_aligned(static_cast<const float*>(a.out1) + tr.ow);
+        if (OP == OP_TANADJ_F) vec = vec && pair_aligned(static_cast<const T*>(a.dv) + tr.ow);
       }
-      return;
+      if (vec)
+        plain_epilogue<M, OP, T, true>(a, o, h, u0, u1);
+      else
+        plain_epilogue<M, OP, T, false>(a, o, h, u0, u1);
     }
   }
-  if (!active) return;
-  if constexpr (L == 2) {
-    group_sync<TPF>(bar);
-    row_to_regs<M>(row0, z0, t);
-  }
-  epilogue_column<M, OP, T>(a, g, w, xv + g.e, t, z0, z1);
 }
 
 // ---- three-launch schedule (one kernel per phase over a chunk of WTs) ------
-// Units per P1 CTA (see phase1): two for single-field ops (the second
-// unit's loads overlap the first transform; -4% at N=512), else one.
-#ifndef SRK_P1_UNITS
-#define SRK_P1_UNITS 2
-#endif
-template <int M, int OP>
-__host__ __device__ constexpr int p1_units() { return OpTraits<OP>::K == 1 ? SRK_P1_UNITS : 1; }
-template <int M, int OP, typename T, bool TAN = false>
-__global__ void __launch_bounds__(kThreads, SRK_P1_MIN_BLOCKS)
-k_p1(OpArgs a, Geom g, const float2* __restrict__ twg, int w0, float2* __restrict__ scratch, int S, int ahead) {
-  // TAN (adjoint-type op of the tangent-adjoint, dv and df given) is chosen
-  // by the launch: a.dI != nullptr exactly when TAN
-  extern __shared__ float2 sm[];
-  constexpr int TPF = tpf_of<M>();
-  const int line = threadIdx.x / TPF, t = threadIdx.x % TPF;
-  load_twiddles(sm, twg, M);
-  __syncthreads();
+// Index of this thread's group in its block.
+template <int M>
+__device__ __forceinline__ int group_index() { return threadIdx.x / Quad<M>::GT; }
+
+// ahead (OP_ADJ): launch positions between this CTA and the one whose inputs
+// it prefetches into L2 (0: none).
+template <int M, int OP, typename T, bool TAN = false, bool TESTED = false>
+__global__ void __launch_bounds__(kThreads, OP == OP_ADJ ? SRK_P1_ADJ_MIN_BLOCKS : SRK_P1_MIN_BLOCKS)
+k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict__ scratch, int ahead) {
+  // TAN and TESTED (adjoint-type op) are chosen by the launch: TESTED for
+  // erosion 0, else TAN exactly when dv and df are given
+  extern __shared__ __align__(16) unsigned char sm[];
+  GroupMem<M> gm = group_mem<M, false>(sm, g.err);
   const int wl = blockIdx.y;
-  constexpr int NU = p1_units<M, OP>();
-  float2* stash = OP == OP_ADJ ? sm + tw_slots<M>() + 2 * lpu_of<M>() * row_stride<M>() : nullptr;
-  phase1<M, OP, T, NU, TAN>(a, g, w0 + wl, blockIdx.x * NU, scratch + wl * wt_elems<M, OP>(S), sm + tw_slots<M>(),
-                            sm, line, t, ahead, stash);
+  if constexpr (OP == OP_ADJ && !TESTED) {
+    const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
+    const int by2 = lin / (int)gridDim.x, bx2 = lin % (int)gridDim.x;
+    if (ahead > 0 && by2 < (int)gridDim.y) p1_prefetch_adj<M, T>(a, g, w0 + by2, bx2);
+  }
+  phase1<M, OP, T, TAN, TESTED>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
+                                scratch + wl * wt_elems<M, OP>(g.S), gm, tw);
 }
 
 template <int M, int OP>
 __global__ void __launch_bounds__(kThreads, SRK_P2_MIN_BLOCKS)
-k_p2(float2* __restrict__ scratch, const float2* __restrict__ Gx, const float2* __restrict__ Gy, int conjG, Geom g,
-     const float2* __restrict__ twg) {
-  extern __shared__ float2 sm[];
-  constexpr int TPF = tpf_of<M>();
-  const int line = threadIdx.x / TPF, t = threadIdx.x % TPF;
-  load_twiddles(sm, twg, M);
+k_p2(float2* __restrict__ scratch, const float4* __restrict__ Gx, const float4* __restrict__ Gy, int conjG, Geom g,
+     const float4* __restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  GroupMem<M> gm = group_mem<M, true>(sm, g.err);
   float2* base = scratch + blockIdx.y * wt_elems<M, OP>(g.S);
-  float2* rows = sm + tw_slots<M>();
-  phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blockIdx.x * lpu_of<M>(), rows, sm, line, t,
-                rows + 2 * lpu_of<M>() * row_stride<M>());
+  phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blockIdx.x * groups_of<M>() + group_index<M>(), gm,
+                tw);
 }
 
-// S2L: the S2 layout (S2Layout).
 template <int M, int OP, typename T, int S2L = kS2Engine>
-__global__ void __launch_bounds__(kThreads, SRK_P3_MIN_BLOCKS)
-k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float2* __restrict__ twg, int w0, int ahead) {
-  extern __shared__ float2 sm[];
-  constexpr int TPF = tpf_of<M>();
-  const int line = threadIdx.x / TPF, t = threadIdx.x % TPF;
-  load_twiddles(sm, twg, M);
+__global__ void __launch_bounds__(kThreads, OpTraits<OP>::L == 1 ? SRK_P3_ADJ_MIN_BLOCKS : SRK_P3_MIN_BLOCKS)
+k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ tw, int w0) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  GroupMem<M> gm = group_mem<M, p3_buf<OP>()>(sm, g.err);
   const int wl = blockIdx.y;
-  constexpr bool ASYNC = p3_async_window<OP, T>();
-  T* win0 = ASYNC ? reinterpret_cast<T*>(sm + tw_slots<M>() + 2 * lpu_of<M>() * row_stride<M>()) : nullptr;
-  {
-    // L2 prefetch of the S2 columns of the CTA one SM-count of launch
-    // positions later: one contiguous run per field in the blocked layout,
-    // one 8-value row piece per ky in the plain one
-    constexpr int L = OpTraits<OP>::L;
-    const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
-    const int by2 = lin / (int)gridDim.x, bx2 = lin % (int)gridDim.x;
-    if (ahead > 0 && by2 < (int)gridDim.y) {
-      const float2* s2 = scratch + by2 * wt_elems<M, OP>(g.S) + s1_elems<M, OP>();
-      if constexpr (s2_blocked<M>() && S2L != kS2Plain) {
-        constexpr int LINES = M * lpu_of<M>() * (int)sizeof(float2) / 128;  // per field
-        static_assert(L * LINES <= kThreads, "one line per thread");
-        if (threadIdx.x < L * LINES) {
-          const int l = threadIdx.x / LINES, r = threadIdx.x % LINES;
-          const float2* blk = s2 + ((size_t)l * (s2_pitch(g.S) / lpu_of<M>()) + bx2) * M * lpu_of<M>();
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(blk + r * (128 / sizeof(float2))));
-        }
-      } else {
-        const float2* col = s2 + bx2 * lpu_of<M>();
-        for (int idx = threadIdx.x; idx < L * M; idx += kThreads)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(col + (size_t)idx * s2_pitch(g.S)));
-      }
-    }
-  }
-  phase3<M, OP, T, ASYNC, S2L>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blockIdx.x,
-                          sm + tw_slots<M>(), sm, line, t, win0);
+  const int nblk = s2_blocks(g.S, S2L == kS2Rotated ? 0 : g.e - s2_first(g.e));
+  const int blk = blockIdx.x * groups_of<M>() + group_index<M>();
+  if (blk < nblk)
+    phase3<M, OP, T, S2L>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blk, gm, tw);
 }
 
 // ---- persistent schedule ---------------------------------------------------------
@@ -1350,23 +1140,20 @@ __device__ __forceinline__ bool wait_geq(const unsigned int* p, unsigned int tar
 }
 
 template <int M, int OP, typename T>
-__global__ void __launch_bounds__(kThreads, SRK_MIN_BLOCKS)
-k_persist(OpArgs a, Geom g, const float2* __restrict__ Gx, const float2* __restrict__ Gy, int conjG,
-          const float2* __restrict__ twg, float2* __restrict__ scratch, int nwt, Ctl* ctl, PersistParams pp) {
-  extern __shared__ float2 sm[];
+__global__ void __launch_bounds__(kThreads, SRK_P2_MIN_BLOCKS)
+k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restrict__ Gy, int conjG,
+          const float4* __restrict__ tw, float2* __restrict__ scratch, int nwt, Ctl* ctl, PersistParams pp) {
+  extern __shared__ __align__(16) unsigned char sm[];
   __shared__ int s_t[2];
-  constexpr int TPF = tpf_of<M>();
-  constexpr int LPU = lpu_of<M>();
-  const int line = threadIdx.x / TPF, t = threadIdx.x % TPF;
-  const int n1 = M / LPU, n2 = M / LPU, n3 = (g.S + LPU - 1) / LPU;
+  constexpr int NG = groups_of<M>();
+  GroupMem<M> gm = group_mem<M, true>(sm, g.err);
+  const int nblk = s2_blocks(g.S, g.e - s2_first(g.e));
+  const int n1 = M / unit_lines<M>(), n2 = n1, n3 = (nblk + NG - 1) / NG;
   const int round = n1 + n2 + n3;
   const int lag = pp.lag, nslot = pp.nslot;
   const long long total = (long long)(nwt + 2 * lag) * round;
   const size_t slot_elems = wt_elems<M, OP>(g.S);
   unsigned long long spins = 0;
-  float2* tw = sm;
-  float2* buf = sm + tw_slots<M>();
-  load_twiddles(tw, twg, M);
   if (threadIdx.x == 0) s_t[0] = (int)atomicAdd(&ctl->ticket, 1u);
   __syncthreads();
   int cur = s_t[0];
@@ -1395,13 +1182,13 @@ k_persist(OpArgs a, Geom g, const float2* __restrict__ Gx, const float2* __restr
     if (!s_t[1]) break;
     if (live) {
       float2* base = scratch + (size_t)slot * slot_elems;
+      const int blk = unit * NG + group_index<M>();
       if (phase == 1) {
-        phase1<M, OP, T>(a, g, w, unit, base, buf, tw, line, t);
+        phase1<M, OP, T, false, OP == OP_ADJ>(a, g, w, blk, base, gm, tw);
       } else if (phase == 2) {
-        phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, unit * LPU, buf, tw, line, t,
-                      buf + 2 * LPU * row_stride<M>());
-      } else {
-        phase3<M, OP, T>(base + s1_elems<M, OP>(), a, g, w, unit, buf, tw, line, t);
+        phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blk, gm, tw);
+      } else if (blk < nblk) {
+        phase3<M, OP, T>(base + s1_elems<M, OP>(), a, g, w, blk, gm, tw);
       }
     }
     __syncthreads();  // every thread's scratch stores of this unit are issued

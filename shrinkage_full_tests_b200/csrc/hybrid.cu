@@ -10,7 +10,7 @@
 // (engine.cuh phase2) for the valid outputs, without the transforms.  The
 // inverse column FFT and the epilogue (P3) are unchanged: U is written to S2
 // in P3's blocked FP32 layout with the lines of column block b rotated by b
-// (k_p3<.., ROT = true> undoes it while staging): one item has one ky, so
+// (k_p3<.., kS2Rotated> undoes it while loading): one item has one ky, so
 // its stores are 32-byte pieces, and unrotated those sat at one offset of
 // blocks 16 KB apart (measured 159 -> 150 us per 128 work tiles).
 //
@@ -247,11 +247,8 @@ __global__ void __launch_bounds__(kThreadsH, 1) k_p2h(const __grid_constant__ CU
 #pragma unroll
       for (int h = 0; h < 4; ++h) zw[h] = __ldg(a.mx + min(wl0 + 32 * h + lane, a.c - 1));
       const int xv = MT * j + MT - 1 - mrow;      // valid-column index x' - e
-      // rotated blocked layout: S2 block xv >> 2 holds ky at line (ky + xv >> 2) mod M;
-      // plain layout: row ky, column xv
-      const size_t xo = kHybS2Layout == 2
-                            ? (size_t)ky * a.P + xv
-                            : (size_t)(xv >> 2) * M * 4 + (size_t)((ky + (xv >> 2)) & (M - 1)) * 4 + (xv & 3);
+      // rotated blocked layout: S2 block xv >> 2 holds ky at line (ky + xv >> 2) mod M
+      const size_t xo = (size_t)(xv >> 2) * M * 4 + (size_t)((ky + (xv >> 2)) & (M - 1)) * 4 + (xv & 3);
       float sp[4];
       for (int f = 0; f < 2; ++f) {
         bool w = true;
@@ -306,17 +303,18 @@ __global__ void __launch_bounds__(kThreadsH, 1) k_p2h(const __grid_constant__ CU
 
 // g_{G,ky}[d] for d = -e .. e from the engine-layout spectra (FP32 values,
 // FP64 sums): gbuf[(f * M + ky) * (2e+1) + d + e].
-__global__ void k_hyb_g(const float2* __restrict__ Gx, const float2* __restrict__ Gy, int e,
+__global__ void k_hyb_g(const float4* __restrict__ Gx, const float4* __restrict__ Gy, int e,
                         const double2* __restrict__ tab, double2* __restrict__ gbuf) {
   const int KW = 2 * e + 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= 2 * M * KW) return;
   const int f = idx / (M * KW), rem = idx - f * M * KW;
   const int ky = rem / KW, d = rem - (rem / KW) * KW - e;
-  const float2* G = (f == 0 ? Gx : Gy) + (size_t)ky * M;
+  const float* G = reinterpret_cast<const float*>(f == 0 ? Gx : Gy);
   double re = 0.0, im = 0.0;
   for (int kx = 0; kx < M; ++kx) {
-    const float2 v = G[kx];
+    const float* gv = G + spec_index(M, ky, kx);
+    const float2 v = make_float2(gv[0], gv[2]);
     int m = (d * kx) % M;
     if (m < 0) m += M;
     const double2 w = tab[m];  // (cos, sin)(2 pi m / M): exp(+i ...)

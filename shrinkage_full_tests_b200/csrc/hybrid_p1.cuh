@@ -4,7 +4,7 @@
 // in the layout the tensor-core row pass (hybrid.cu) reads with TMA:
 //   planes[((ky * 2 + part) * c + wl) * M + x]      (part 0 = re, 1 = im),
 // c = work tiles in the chunk, wl = work tile within the chunk.  Each CTA
-// transforms 8 consecutive columns (two units of four), stages their values
+// transforms 8 consecutive columns (two groups of four), stages their values
 // [ky][part][8] in shared memory and writes them with TMA stores (one
 // 16-byte piece per (ky, part) plane row).  Used for the pair ops (OP_FWD,
 // OP_VJP_F: two images per work tile) where the column DFT of
@@ -28,11 +28,12 @@ constexpr int kHybM = 512;
 // tiles against 0.81 ms with 16 columns (whole 32-byte sectors, but 3 CTAs
 // per SM and twice the transforms per line).
 constexpr int kP1hCols = 8;
+constexpr int kP1hThreads = kP1hCols / kLines * Quad<kHybM>::GT;
 // Byte offset of the staging block (128-byte aligned: the source of TMA stores).
-__host__ __device__ constexpr size_t p1h_stage_offset() { return (phase_smem_bytes<kHybM>() + 127) / 128 * 128; }
+__host__ __device__ constexpr size_t p1h_stage_offset() { return (kP1hCols / kLines * group_bytes<kHybM, false>() + 127) / 128 * 128; }
 struct P1hAux {
-  int cnt[kWarps];     // refit: flagged work tiles per warp
-  int list[kThreads];  // refit: the flagged work tiles of one group
+  int cnt[kP1hThreads / 32];  // refit: flagged work tiles per warp
+  int list[kP1hThreads];      // refit: the flagged work tiles of one group
 };
 __host__ __device__ constexpr size_t p1h_aux_offset() {
   return p1h_stage_offset() + (size_t)kHybM * 2 * kP1hCols * sizeof(__half);
@@ -46,47 +47,33 @@ constexpr int kP1hBox = 256;
 // [plane = 2 ky + part][8 columns], written by TMA stores (box {8 columns, 1
 // work tile, kP1hBox planes}: the TMA engine writes the 1024 16-byte row
 // pieces the threads would otherwise scatter).  Block-uniform arguments; the
-// twiddles are in sm.  With zmax given, each warp folds the max |Z| of its
+// twiddle quads are tw.  With zmax given, each warp folds the max |Z| of its
 // unscaled values into zmax[wl] (one atomic per warp, float bits).  Ends with
 // the stores complete and the block synchronised (the staging block may be
 // reused).
 template <int OP, typename T>
-__device__ __forceinline__ void p1h_cols(const CUtensorMap* pmap, const OpArgs& a, const Geom& g, float2* sm,
-                                         int w0, int wl, int xb, float sp, int ahead, unsigned int* zmax,
-                                         unsigned int* err) {
+__device__ __forceinline__ void p1h_cols(const CUtensorMap* pmap, const OpArgs& a, const Geom& g, unsigned char* sm,
+                                         GroupMem<kHybM>& gm, const float4* __restrict__ tw, int w0, int wl, int xb,
+                                         float sp, unsigned int* zmax, unsigned int* err) {
   constexpr int M = kHybM;
-  constexpr int TPF = tpf_of<M>();
-  constexpr int EPT = M / TPF;
-  constexpr int LPU = lpu_of<M>();
-  constexpr int NU = kP1hCols / LPU;  // units of LPU columns per CTA
-  const int line = threadIdx.x / TPF, t = threadIdx.x % TPF;
-  float2* rows = sm + tw_slots<M>();
-  __half* st = reinterpret_cast<__half*>(reinterpret_cast<unsigned char*>(sm) + p1h_stage_offset());
+  using Q = Quad<M>;
+  constexpr int NU = kP1hCols / kLines;  // groups of four columns per CTA
+  static_assert(kP1hThreads == NU * Q::GT && Q::KPT == 1, "one group of four columns per group of threads");
+  const QuadThread t = gm.t;
+  const int u = group_index<M>();
+  __half* st = reinterpret_cast<__half*>(sm + p1h_stage_offset());
   const int w = w0 + wl;
-  if (ahead > 0) {
-    // L2 prefetch of the image columns of the CTA one SM-count of launch positions later
-    const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
-    const int w2 = w - (int)blockIdx.y + lin / (int)gridDim.x, xb2 = (lin % (int)gridDim.x) * NU;
-    for (int u = 0; u < NU; u += 2) p1_prefetch<M, OP, T, 2>(a, g, w2, xb2 + u);
-  }
-  float2* row = rows + line * row_stride<M>();
-  float2 za[EPT], zb[EPT];
+  cpk z[Q::R];
+  float2 X[Q::VPT];
+  load_column<M, OP, T>(a, g, w, xb * NU + u, gm, z);
+  fft_dit<M, false>(z, X, gm.ex, tw, t);
   float m = 0.f;
-  load_column<M, OP, T>(a, g, w, 0, (NU * xb) * LPU + line, t, za);
-#pragma unroll 1
-  for (int u = 0; u < NU; ++u) {
-    // the next unit's column loads are in flight during this transform
-    if (u + 1 < NU) load_column<M, OP, T>(a, g, w, 0, (NU * xb + u + 1) * LPU + line, t, zb);
-    fft<M, false>(za, row, sm, t, 1 + line);
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      const int ky = t + TPF * i;
-      m = fmaxf(m, fmaxf(fabsf(za[i].x), fabsf(za[i].y)));
-      st[(ky * 2 + 0) * kP1hCols + u * LPU + line] = __float2half_rn(za[i].x * sp);
-      st[(ky * 2 + 1) * kP1hCols + u * LPU + line] = __float2half_rn(za[i].y * sp);
-    }
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) za[i] = zb[i];
+  for (int i = 0; i < Q::J; ++i) {
+    const int ky = t.q + Q::R * i;
+    m = fmaxf(m, fmaxf(fabsf(X[i].x), fabsf(X[i].y)));
+    st[(ky * 2 + 0) * kP1hCols + u * kLines + t.line] = __float2half_rn(X[i].x * sp);
+    st[(ky * 2 + 1) * kP1hCols + u * kLines + t.line] = __float2half_rn(X[i].y * sp);
   }
   if (zmax) {
 #pragma unroll
@@ -111,14 +98,13 @@ __device__ __forceinline__ void p1h_cols(const CUtensorMap* pmap, const OpArgs& 
 // zmax[wl] = max |Z| of work tile wl (float bits; zeroed before the launch).
 // Grid (M / kP1hCols, c).
 template <int OP, typename T>
-__global__ void __launch_bounds__(kThreads, SRK_P1_MIN_BLOCKS)
-k_p1h(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float2* __restrict__ twg, int w0, int ahead,
+__global__ void __launch_bounds__(kP1hThreads, 4)
+k_p1h(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float4* __restrict__ tw, int w0,
       unsigned int* __restrict__ zmax, unsigned int* err) {
   static_assert(OpTraits<OP>::K == 1, "single-field ops only");
-  extern __shared__ __align__(128) float2 sm[];
-  load_twiddles(sm, twg, kHybM);
-  __syncthreads();
-  p1h_cols<OP, T>(&pmap, a, g, sm, w0, blockIdx.y, blockIdx.x, 1.f, ahead, zmax, err);
+  extern __shared__ __align__(128) unsigned char smh[];
+  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, err);
+  p1h_cols<OP, T>(&pmap, a, g, smh, gm, tw, w0, blockIdx.y, blockIdx.x, 1.f, zmax, err);
 }
 
 // Refit: the work tiles whose zmax lies outside the range kept at scale 1
@@ -127,25 +113,25 @@ k_p1h(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float2* 
 // flagged work tiles, in order; every block scans zmax (c words) for them, so
 // a chunk without such work tiles costs one short launch.
 template <int OP, typename T>
-__global__ void __launch_bounds__(kThreads, SRK_P1_MIN_BLOCKS)
-k_p1h_refit(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float2* __restrict__ twg, int w0, int c,
+__global__ void __launch_bounds__(kP1hThreads, 4)
+k_p1h_refit(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float4* __restrict__ tw, int w0, int c,
             const unsigned int* __restrict__ zmax, unsigned int* err) {
   constexpr int NX = kHybM / kP1hCols;  // column blocks per work tile
-  extern __shared__ __align__(128) float2 sm[];
-  P1hAux* aux = reinterpret_cast<P1hAux*>(reinterpret_cast<unsigned char*>(sm) + p1h_aux_offset());
+  extern __shared__ __align__(128) unsigned char smh[];
+  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, err);
+  P1hAux* aux = reinterpret_cast<P1hAux*>(smh + p1h_aux_offset());
   int* cnt = aux->cnt;
   int* list = aux->list;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  bool loaded = false;
-  long long rank0 = 0;  // flagged work tiles before this group of kThreads
-  for (int b0 = 0; b0 < c; b0 += kThreads) {
+  long long rank0 = 0;  // flagged work tiles before this group of kP1hThreads
+  for (int b0 = 0; b0 < c; b0 += kP1hThreads) {
     const int wl = b0 + threadIdx.x;
     const bool f = wl < c && plane_exp(__ldg(zmax + wl)) != 0;
     const unsigned bal = __ballot_sync(0xffffffffu, f);
     if (lane == 0) cnt[warp] = __popc(bal);
     __syncthreads();
     int before = 0, total = 0;
-    for (int i = 0; i < kWarps; ++i) {
+    for (int i = 0; i < kP1hThreads / 32; ++i) {
       before += i < warp ? cnt[i] : 0;
       total += cnt[i];
     }
@@ -156,12 +142,7 @@ k_p1h_refit(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const fl
       const float sp = ldexpf(1.f, plane_exp(__ldg(zmax + wk)));
       for (int xb = 0; xb < NX; ++xb) {
         if ((int)(((rank0 + k) * NX + xb) % gridDim.x) != (int)blockIdx.x) continue;
-        if (!loaded) {
-          load_twiddles(sm, twg, kHybM);
-          __syncthreads();
-          loaded = true;
-        }
-        p1h_cols<OP, T>(&pmap, a, g, sm, w0, wk, xb, sp, 0, nullptr, err);
+        p1h_cols<OP, T>(&pmap, a, g, smh, gm, tw, w0, wk, xb, sp, nullptr, err);
       }
     }
     rank0 += total;

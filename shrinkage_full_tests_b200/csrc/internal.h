@@ -62,17 +62,17 @@ inline srk_status cuda_status(cudaError_t e, const char* what) {
 #endif
 struct srk_plan_s {
   int device = 0;
-  int nsm = 0;  // SMs of the device (P1's L2 prefetch distance)
+  int nsm = 0;  // SMs of the device (L2 prefetch distances)
   int N = 0, W = 0, e = 0, B_max = 0, spectra_M = 0;
   float dx = 1.f;
   srk_dtype dtype = SRK_F32;
   srk_adj_convention conv = SRK_ADJ_REFERENCE;
   int M = 0, S = 0, T = 0, Ta = 0;
   int chunk = 0;
-  float2* G[2] = {nullptr, nullptr};   // engine-layout spectra, scaled by dx^2/M^2
+  float4* G[2] = {nullptr, nullptr};   // engine-layout spectra (spec_index), scaled by dx^2/M^2
   bool have_G = false;
   const void* src[2] = {nullptr, nullptr};
-  float2* tw = nullptr;                // W_M^m, float
+  float4* tw = nullptr;                // FFT twiddle quads, float
   // spectrum import / set_kernel workspace, allocated with the plan so that
   // importing spectra needs no allocation and no host synchronisation:
   // FP64 twiddle tables at the tile size and at spectra_M, the column pass
@@ -176,7 +176,7 @@ srk_status tensor_rows_plane_map(const __half* planes, int c, unsigned box_x, un
 
 // Spectrum kernels defined in spectra.cuh (compiled once, in srk_abi.cu) and
 // launched from the other translation units too.
-__global__ void k_relayout(const float2* __restrict__ ref, int M, float scale, float2* __restrict__ full);
-__global__ void k_fft_twiddles(float2* __restrict__ tw, int M);
+__global__ void k_relayout(const float2* __restrict__ ref, int M, float scale, float4* __restrict__ full);
+__global__ void k_fft_twiddles(float4* __restrict__ tw, int M);
 
 }  // namespace srk

@@ -94,9 +94,9 @@ extern "C" srk_status srk_training_forward_noalloc(const float* d_E, const float
   view.N = N; view.W = W; view.e = erosion; view.dx = dx; view.B_max = B; view.spectra_M = N;
   view.dtype = SRK_F32;
   view.M = M; view.S = S; view.T = 1; view.Ta = 1;
-  view.tw = sc;
-  view.G[0] = sc + M;
-  view.G[1] = sc + M + (size_t)M * M;
+  view.tw = reinterpret_cast<float4*>(sc);
+  view.G[0] = reinterpret_cast<float4*>(sc + M);
+  view.G[1] = reinterpret_cast<float4*>(sc + M + (size_t)M * M);
   view.have_G = true;
   view.scratch = sc + fixed;
   view.scratch_bytes = (cap - fixed) * sizeof(float2);

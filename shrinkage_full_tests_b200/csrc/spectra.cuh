@@ -7,12 +7,13 @@
 //     centre sits at index 0:  G(ky,kx) = sum K(dx,dy) exp(-2 pi i (kx dx + ky dy)/M);
 //   * reference layout ("R2C of the column-major buffer"): half spectrum
 //     ref[kx*(M/2+1) + ky], ky in [0, M/2];
-//   * engine layout: full spectrum full[ky*M + kx] (Hermitian extension).
+//   * engine layout: full spectrum, Hermitian extension, quads blocked by four
+//     rows (spec_index in engine.cuh).
 // Twiddles exp(-2 pi i m/M) come from a double table indexed by (a*b) mod M,
 // so no angle is ever reduced in floating point.
 #pragma once
 #include <cuda_runtime.h>
-#include "fft_warp.cuh"
+#include "engine.cuh"
 
 namespace srk {
 
@@ -85,11 +86,17 @@ __global__ void k_dft_cols(const double* __restrict__ Kd, int KW, int M, const d
   P[(long long)j * M + kx] = make_double2(re, im);
 }
 
+__device__ __forceinline__ void spec_store(float4* __restrict__ full, int M, int ky, int kx, float re, float im) {
+  float* p = reinterpret_cast<float*>(full) + spec_index(M, ky, kx);
+  p[0] = re;
+  p[2] = im;
+}
+
 // Pass 2: G(ky,kx) = sum_j P[j][kx] exp(-2 pi i ky (j-c)/M); writes the
 // engine layout scaled by `scale` (if full != null) and the reference layout
 // unscaled (if ref != null).
 __global__ void k_dft_rows(const double2* __restrict__ P, int KW, int M, const double2* __restrict__ tab,
-                           double scale, float2* __restrict__ full, float2* __restrict__ ref) {
+                           double scale, float4* __restrict__ full, float2* __restrict__ ref) {
   const int kx = blockIdx.x * blockDim.x + threadIdx.x;
   const int ky = blockIdx.y;
   if (kx >= M) return;
@@ -101,13 +108,13 @@ __global__ void k_dft_rows(const double2* __restrict__ P, int KW, int M, const d
     re += p.x * w.x - p.y * w.y;
     im += p.x * w.y + p.y * w.x;
   }
-  if (full) full[(long long)ky * M + kx] = make_float2((float)(re * scale), (float)(im * scale));
+  if (full) spec_store(full, M, ky, kx, (float)(re * scale), (float)(im * scale));
   if (ref && ky <= M / 2) ref[(long long)kx * (M / 2 + 1) + ky] = make_float2((float)re, (float)im);
 }
 
 // Re-layout a reference half spectrum of size M into the engine layout with
 // Hermitian extension: G(ky,kx) = conj(G(M-ky, M-kx)) for ky > M/2.
-__global__ void k_relayout(const float2* __restrict__ ref, int M, float scale, float2* __restrict__ full) {
+__global__ void k_relayout(const float2* __restrict__ ref, int M, float scale, float4* __restrict__ full) {
   const int kx = blockIdx.x * blockDim.x + threadIdx.x;
   const int ky = blockIdx.y;
   if (kx >= M) return;
@@ -119,7 +126,7 @@ __global__ void k_relayout(const float2* __restrict__ ref, int M, float scale, f
     const float2 s = ref[(long long)((M - kx) % M) * H + (M - ky)];
     v = make_float2(s.x, -s.y);
   }
-  full[(long long)ky * M + kx] = make_float2(v.x * scale, v.y * scale);
+  spec_store(full, M, ky, kx, v.x * scale, v.y * scale);
 }
 
 // Spatial recovery from a reference half spectrum of size Mr, restricted to
@@ -175,22 +182,18 @@ __global__ void k_twiddles64(double2* __restrict__ tab, int M) {
   tab[m] = make_double2(c, s);
 }
 
-// The FFT engine's float twiddle table (per-pass blocks of tw_entry):
-// exp(-2 pi i num/den) in double, rounded once to float; entries past
-// tw_entries(M) are zero.  Plans and the no-allocation forward both build
+// The FFT engine's twiddle quads (fft_quad.cuh): entry p R + k holds
+// W_M^(j k), j = 2p and 2p + 1, as (re, re, im, im), in double, rounded once
+// to float.  M / 2 quads.  Plans and the no-allocation forward both build
 // their tables with this kernel, so the two paths use identical twiddles.
-__global__ void k_fft_twiddles(float2* __restrict__ tw, int M) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  float2 v = make_float2(0.f, 0.f);
-  if (m < tw_entries(M)) {
-    int num = 0, den = 1;
-    tw_entry(M, m, num, den);
-    double s, c;
-    sincospi(2.0 * (double)num / (double)den, &s, &c);
-    v = make_float2((float)c, (float)-s);
-  }
-  tw[m] = v;
+__global__ void k_fft_twiddles(float4* __restrict__ tw, int M) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int R = M == 128 ? 8 : 16;
+  if (i >= M / 2) return;
+  const int p = i / R, k = i % R;
+  double s[2], c[2];
+  for (int l = 0; l < 2; ++l) sincospi(2.0 * (double)((2 * p + l) * k) / (double)M, &s[l], &c[l]);
+  tw[i] = make_float4((float)c[0], (float)c[1], (float)-s[0], (float)-s[1]);
 }
 
 // A KW x KW float kernel centred on a KWp x KWp support (KWp >= KW, both

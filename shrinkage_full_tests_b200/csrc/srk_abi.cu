@@ -62,6 +62,7 @@ Geom fwd_geom(const srk_plan_s* p, int B) {
   g.M = p->M; g.e = p->e; g.S = p->S; g.T = p->T;
   g.Nin = p->N; g.Wout = p->W; g.TT = p->T * p->T; g.U = B * g.TT;
   g.N = p->N; g.W = p->W; g.wout_n = 0;
+  g.err = p->direct_err;
   return g;
 }
 Geom adj_geom(const srk_plan_s* p, int B) {
@@ -70,6 +71,7 @@ Geom adj_geom(const srk_plan_s* p, int B) {
   g.M = p->M; g.e = p->e; g.S = p->S; g.T = p->Ta;
   g.Nin = p->N + 2 * p->e; g.Wout = p->N; g.TT = p->Ta * p->Ta; g.U = B * g.TT;
   g.N = p->N; g.W = p->W; g.wout_n = 1;
+  g.err = p->direct_err;
   return g;
 }
 
@@ -135,7 +137,7 @@ srk_status build_tab64(double2* tab, int M, cudaStream_t s) {
 // Spatial kernel (double, column-major KW x KW) -> engine spectrum at size M.
 // tab: FP64 twiddles at size M; P: KW x M double2 of workspace.
 srk_status spectrum_from_spatial(const double* Kd, int KW, int M, const double2* tab, double2* P, double scale,
-                                 float2* full, float2* ref, cudaStream_t s) {
+                                 float4* full, float2* ref, cudaStream_t s) {
   k_dft_cols<<<dim3((M + 127) / 128, KW), 128, 0, s>>>(Kd, KW, M, tab, P);
   k_dft_rows<<<dim3((M + 127) / 128, M), 128, 0, s>>>(P, KW, M, tab, scale, full, ref);
   return cuda_status(cudaGetLastError(), "kernel DFT launch");
@@ -146,7 +148,7 @@ srk_status spectrum_from_spatial(const double* Kd, int KW, int M, const double2*
 // (2e+1)^2 support) for the direct schedule.  Stream-ordered; uses only the
 // plan's import workspace (no allocation, no host synchronisation), so it
 // may run under stream capture.
-srk_status import_one(srk_plan_s* p, int k, const float2* ref, float2* full, cudaStream_t s) {
+srk_status import_one(srk_plan_s* p, int k, const float2* ref, float4* full, cudaStream_t s) {
   const int Mr = p->spectra_M;
   // dx^2 / M^2 folded into the spectrum (srkConvOaS applies dx*dx/(M*M), srk_forward.cuh:380)
   const float scale = (p->dx * p->dx) / ((float)p->M * (float)p->M);
@@ -578,8 +580,8 @@ srk_status srk_plan_sync(srk_plan p, srk_stream_t s) {
     if (derr) {
       SRK_CUDA(cudaMemset(p->direct_err, 0, sizeof(derr)));
       return fail(SRK_ERR_TIMEOUT,
-                  "a tensor-core schedule stopped early (site %u: 1-13 a bounded wait gave up, 14-15 a shared "
-                  "memory block off its alignment); outputs incomplete",
+                  "a kernel stopped early (site %u: 1-13 and 16 a bounded wait gave up, 14-15 a shared memory "
+                  "block off its alignment); outputs incomplete",
                   derr);
     }
   }
