@@ -7,12 +7,6 @@
 
 namespace srk {
 
-// L2 prefetch distance of the adjoint-type P1 in launch positions per SM.
-#ifndef SRK_P1_AHEAD
-#define SRK_P1_AHEAD 1
-#endif
-constexpr int kP1Ahead = SRK_P1_AHEAD;
-
 template <typename K>
 srk_status set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024)
@@ -137,7 +131,7 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
   if constexpr (M == kHybM && OpTraits<OP>::K == 1 && OpTraits<OP>::PAIRS && !std::is_same<T, float>::value) {
     if (p->schedule == SRK_SCHEDULE_TENSOR_ROWS && p->hyb_ready) return launch_tensor_rows<OP, T>(p, a, g, nwt, s);
   }
-  constexpr size_t sm1 = p1_smem_bytes<M>(), sm2 = p2_smem_bytes<M>();
+  constexpr size_t sm1 = p1_smem_bytes<M, OP>(), sm2 = p2_smem_bytes<M>();
   constexpr size_t sm3 = p3_smem_bytes<M, OP>();
   constexpr int NG = groups_of<M>();
   const int n3 = (s2_blocks(g.S, g.e - s2_first(g.e)) + NG - 1) / NG;  // P3 CTAs per work tile
@@ -195,12 +189,10 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
   auto launch3 = [&](int w0, int c, float2* base, cudaStream_t s1, cudaStream_t s2, cudaStream_t s3,
                      cudaEvent_t e1, cudaEvent_t e2) -> srk_status {
     const dim3 g1(M / unit_lines<M>(), c);
-    if (kAdj && a.e < 1)
-      k_p1<M, OP, T, false, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, 0);
-    else if (tan)
-      k_p1<M, OP, T, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, p->nsm * kP1Ahead);
+    if (tan)
+      k_p1<M, OP, T, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base);
     else
-      k_p1<M, OP, T><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base, p->nsm * kP1Ahead);
+      k_p1<M, OP, T><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base);
     if (e1) {
       SRK_CUDA(cudaEventRecord(e1, s1));
       SRK_CUDA(cudaStreamWaitEvent(s2, e1, 0));

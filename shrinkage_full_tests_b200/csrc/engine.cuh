@@ -148,23 +148,7 @@ template <> __device__ __forceinline__ void stf<__nv_bfloat16>(__nv_bfloat16* p,
   p[i] = __float2bfloat16_rn(v);
 }
 
-// Central difference along columns (x) / rows (y) with zero outside [0,N),
-// as srk_grad_x / srk_grad_y (srk_forward.cuh:429-445).
-template <typename T>
-__device__ __forceinline__ float grad_x(const T* f, int N, int gx, int gy) {
-  const float r = (gx + 1 < N) ? ldf(f, (long long)(gx + 1) * N + gy) : 0.f;
-  const float l = (gx > 0) ? ldf(f, (long long)(gx - 1) * N + gy) : 0.f;
-  return (r - l) * 0.5f;
-}
-template <typename T>
-__device__ __forceinline__ float grad_y(const T* f, int N, int gx, int gy) {
-  const float d = (gy + 1 < N) ? ldf(f, (long long)gx * N + gy + 1) : 0.f;
-  const float u = (gy > 0) ? ldf(f, (long long)gx * N + gy - 1) : 0.f;
-  return (d - u) * 0.5f;
-}
-
-// a*b + c*d with one fixed rounding sequence, so every kernel that inlines
-// an epilogue produces bit-identical results.
+// a*b + c*d with one fixed rounding sequence (pk_dot2 of scalars).
 __device__ __forceinline__ float dot2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
 
 struct TileRef {
@@ -206,28 +190,6 @@ __device__ __forceinline__ TileRef tile_of(const Geom& g, int u) {
   }
   t.Wout = g.wout_n ? t.N : t.W;
   return t;
-}
-
-// ---- loaders: value of field k of work tile w at local (x, y) ------------
-// Adjoint-type: h_x = v*df/dx (or dv*df/dx + v*d(df)/dx for the
-// tangent-adjoint) on the valid window, zero elsewhere; virtual coords are
-// shifted by +e so that the full N x N output is the valid part of the
-// convolution of the zero-extended (N+2e)^2 field
-// (srk_adj_load_tile, adjoint/srk_adjoint.cuh:169-200).
-template <typename T>
-__device__ __forceinline__ float h_at(const OpArgs& a, const TileRef& t, int k, int px, int py) {
-  const int qx = px - a.e, qy = py - a.e;            // image coords
-  const int ox = qx - a.e, oy = qy - a.e;            // valid-window coords
-  if (ox < 0 || oy < 0 || ox >= t.W || oy >= t.W) return 0.f;
-  const long long vo = t.ow + (long long)ox * t.W + oy;
-  const T* f = static_cast<const T*>(a.I) + t.on;
-  const float v = ldf(static_cast<const T*>(a.v), vo);
-  const float g = (k == 0) ? grad_x(f, t.N, qx, qy) : grad_y(f, t.N, qx, qy);
-  if (a.dI == nullptr) return v * g;
-  const T* df = static_cast<const T*>(a.dI) + t.on;
-  const float dv = ldf(static_cast<const T*>(a.dv), vo);
-  const float dg = (k == 0) ? grad_x(df, t.N, qx, qy) : grad_y(df, t.N, qx, qy);
-  return dot2(dv, g, v, dg);
 }
 
 // ---- blocks, groups and scratch layout -----------------------------------------
@@ -346,23 +308,50 @@ template <> __device__ __forceinline__ pk swin2<__nv_bfloat16>(const __nv_bfloat
   return pk_make(f.x, f.y);
 }
 
-// Two consecutive values as a packed pair; VEC: one aligned access.
+// One value and an aligned pair under a predicate (zero without it): a
+// predicated load, not a branch around one.
+__device__ __forceinline__ unsigned short ldp16(const void* p, bool on) {
+  unsigned short v;
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b16 %0, 0;\n\t@q ld.global.nc.b16 %0, [%1];\n\t}"
+      : "=h"(v) : "l"(p), "r"((unsigned)on));
+  return v;
+}
+__device__ __forceinline__ unsigned ldp32(const void* p, bool on) {
+  unsigned v;
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.b32 %0, [%1];\n\t}"
+      : "=r"(v) : "l"(p), "r"((unsigned)on));
+  return v;
+}
+__device__ __forceinline__ pk ldp64(const void* p, bool on) {
+  pk v;
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b64 %0, 0;\n\t@q ld.global.nc.b64 %0, [%1];\n\t}"
+      : "=l"(v) : "l"(p), "r"((unsigned)on));
+  return v;
+}
+template <typename T> __device__ __forceinline__ float ldp(const T* p, bool on);
+template <> __device__ __forceinline__ float ldp<float>(const float* p, bool on) { return __uint_as_float(ldp32(p, on)); }
+template <> __device__ __forceinline__ float ldp<__half>(const __half* p, bool on) {
+  return __half2float(__ushort_as_half(ldp16(p, on)));
+}
+template <> __device__ __forceinline__ float ldp<__nv_bfloat16>(const __nv_bfloat16* p, bool on) {
+  return __bfloat162float(__ushort_as_bfloat16(ldp16(p, on)));
+}
+// Two consecutive values as a packed pair; VEC: one aligned access under `lo`.
 template <bool VEC, typename T>
 __device__ __forceinline__ pk ld2(const T* __restrict__ p, long long i, bool lo, bool hi) {
-  if constexpr (VEC) {
-    if (!lo) return 0ull;
-    if constexpr (sizeof(T) == 4) {
-      return __ldg(reinterpret_cast<const unsigned long long*>(p + i));
-    } else if constexpr (std::is_same<T, __half>::value) {
-      const float2 f = __half22float2(__ldg(reinterpret_cast<const __half2*>(p + i)));
+  if constexpr (!VEC) {
+    return pk_make(ldp(p + i, lo), ldp(p + i + 1, hi));
+  } else if constexpr (sizeof(T) == 4) {
+    return ldp64(p + i, lo);
+  } else {
+    const unsigned u = ldp32(p + i, lo);
+    if constexpr (std::is_same<T, __half>::value) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u));
       return pk_make(f.x, f.y);
     } else {
-      const float2 f = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162*>(p + i)));
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
       return pk_make(f.x, f.y);
     }
-  } else {
-    const float a = lo ? ldf(p, i) : 0.f, b = hi ? ldf(p, i + 1) : 0.f;
-    return pk_make(a, b);
   }
 }
 template <bool VEC, typename T>
@@ -483,140 +472,273 @@ __device__ __forceinline__ void load_column(const OpArgs& a, const Geom& g, int 
   for (int r = 0; r < R; ++r) z[r] = cpk{re[r], im[r]};
 }
 
-// Central differences (times 2) of f at a pair of rows of the column at fc:
-// gx = f[+n] - f[-n], gy = f[+1] - f[-1].  MODE 1: fc at an even offset of an
-// aligned array of even column length (one access per pair of a side
-// column); 2: at an odd offset (the row pairs around it are aligned); 0:
-// neither.  Predicates as in ld2 (equal in modes 1 and 2).
-template <int MODE, typename T>
-__device__ __forceinline__ void diff2(const T* __restrict__ fc, int n, int o, bool lo, bool hi, pk& gx, pk& gy) {
-  gx = pk_sub(ld2<MODE == 1>(fc + n, o, lo, hi), ld2<MODE == 1>(fc - n, o, lo, hi));
-  if constexpr (MODE == 2) {
-    gy = pk_sub(ld2<true>(fc, o + 1, lo, hi), ld2<true>(fc, o - 1, lo, hi));
-  } else {
-    const float m = lo ? ldf(fc, o - 1) : 0.f, p = hi ? ldf(fc, o + 2) : 0.f;
-    // the pair (f[o], f[o + 1]): f[o] serves the high lane, f[o + 1] the low one
-    const pk c = ld2<MODE == 1>(fc, o, hi, lo);
-    gy = pk_make(__fsub_rn(pk_hi(c), m), __fsub_rn(p, pk_lo(c)));
-  }
+// ---- image windows --------------------------------------------------------------------
+// Columns of an image in shared memory, raw storage values: window column c
+// <-> image column gx0 + c, element i <-> image row gya + i; out-of-image
+// elements are zero (the central-difference rule).  The four columns of a
+// group need the columns and rows around them for the central differences:
+// kWinCols columns.  gya is the first row wanted rounded down to a multiple
+// of the 16-byte chunk (at least of 2): a pair of rows (y, y + 1) of an even
+// image row is one aligned access.  Column pitch: 8 (mod 32) 4-byte words, so
+// the pair reads of a half-warp (four indices of four lines) fall on
+// distinct banks.
+constexpr int kWinCols = kLines + 2;
+// Pitch that holds S + 2 rows from any start inside a chunk.
+template <typename T>
+__host__ __device__ constexpr int win_pitch(int S) {
+  return sizeof(T) == 4 ? (S + 5 + 23) / 32 * 32 + 8 : (S + 9 + 47) / 64 * 64 + 16;
 }
-
-// One tile's adjoint-type fields at tile column x (erosion >= 1: every
-// gradient neighbour of the valid window lies inside the image), written to
-// the re (LANE 0) or im (LANE 1) parts of hx and hy: h = v * df / dx,
-// or dv * df / dx + v * d(df) / dx for the tangent-adjoint (TAN).
-template <int M, typename T, bool TAN, int LANE, int MODE>
-__device__ __forceinline__ void load_adj_tile(const OpArgs& a, const TileRef& tr, int x, int q,
-                                              cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
-  constexpr int R = Quad<M>::R, J = Quad<M>::J;
-  const int qx = tr.x0 + x - a.e, ox = qx - a.e;  // image / valid-window column
-  const bool on = tr.live && ox >= 0 && ox < tr.W;
-  const int qy0 = tr.y0 + 2 * q - a.e, oy0 = qy0 - a.e;
-  const long long vo = tr.ow + (long long)ox * tr.W + oy0;
-  const long long fo = tr.on + (long long)qx * tr.N + qy0;
-  const T* v = static_cast<const T*>(a.v) + vo;
-  const T* f = static_cast<const T*>(a.I) + fo;
-  const T* dv = TAN ? static_cast<const T*>(a.dv) + vo : v;
-  const T* df = TAN ? static_cast<const T*>(a.dI) + fo : f;
-  const pk half = pk_dup(0.5f);
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int o = J * r;
-    const bool lo = on && (unsigned)(oy0 + o) < (unsigned)tr.W;
-    const bool hi = MODE ? lo : on && (unsigned)(oy0 + o + 1) < (unsigned)tr.W;
-    pk gx, gy;
-    diff2<MODE>(f, tr.N, o, lo, hi, gx, gy);
-    gx = pk_mul(gx, half);
-    gy = pk_mul(gy, half);
-    const pk vv = ld2<MODE != 0>(v, o, lo, hi);
-    pk rx, ry;
-    if constexpr (TAN) {
-      pk dgx, dgy;
-      diff2<MODE>(df, tr.N, o, lo, hi, dgx, dgy);
-      const pk dvv = ld2<MODE != 0>(dv, o, lo, hi);
-      rx = pk_dot2(dvv, gx, vv, pk_mul(dgx, half));
-      ry = pk_dot2(dvv, gy, vv, pk_mul(dgy, half));
-    } else {
-      rx = pk_mul(vv, gx);
-      ry = pk_mul(vv, gy);
-    }
-    (LANE ? hx[r].im : hx[r].re) = rx;
-    (LANE ? hy[r].im : hy[r].re) = ry;
-  }
-}
-// The fields of one tile in the tested form: any erosion (0 included, where
-// gradient neighbours may lie outside the image), one value at a time.
-template <int M, typename T, int LANE>
-__device__ __forceinline__ void load_adj_tested(const OpArgs& a, const TileRef& tr, int x, int q,
-                                                cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
-  constexpr int R = Quad<M>::R, J = Quad<M>::J;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int px = tr.x0 + x, py = tr.y0 + 2 * q + J * r;
-    const pk vx = tr.live ? pk_make(h_at<T>(a, tr, 0, px, py), h_at<T>(a, tr, 0, px, py + 1)) : 0ull;
-    const pk vy = tr.live ? pk_make(h_at<T>(a, tr, 1, px, py), h_at<T>(a, tr, 1, px, py + 1)) : 0ull;
-    (LANE ? hx[r].im : hx[r].re) = vx;
-    (LANE ? hy[r].im : hy[r].re) = vy;
-  }
-}
-template <int M, typename T, bool TAN, bool TESTED, int LANE>
-__device__ __forceinline__ void load_adj_lane(const OpArgs& a, const Geom& g, int w, int x, int q,
-                                              cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
-  const TileRef tr = tile_of(g, 2 * w + LANE);
-  if constexpr (TESTED) {
-    load_adj_tested<M, T, LANE>(a, tr, x, q, hx, hy);
-    return;
-  }
-  const bool al = !(tr.N & 1) && pair_aligned(static_cast<const T*>(a.v) + tr.ow) &&
-                  pair_aligned(static_cast<const T*>(a.I) + tr.on) &&
-                  (!TAN || (pair_aligned(static_cast<const T*>(a.dv) + tr.ow) &&
-                            pair_aligned(static_cast<const T*>(a.dI) + tr.on)));
-  if (!al)
-    load_adj_tile<M, T, TAN, LANE, 0>(a, tr, x, q, hx, hy);
-  else if (a.e & 1)
-    load_adj_tile<M, T, TAN, LANE, 2>(a, tr, x, q, hx, hy);
-  else
-    load_adj_tile<M, T, TAN, LANE, 1>(a, tr, x, q, hx, hy);
-}
-
-// ---- P1 ------------------------------------------------------------------------------------
-// L2 prefetch of the inputs of the adjoint-type unit xb2 of WT w2: the v
-// (and dv) columns and the f (and df) columns around them, for both tiles of
-// the pair, one 128-byte line per thread and step; only addresses inside.
 template <int M, typename T>
-__device__ __forceinline__ void p1_prefetch_adj(const OpArgs& a, const Geom& g, int w2, int xb2) {
-  constexpr int C = unit_lines<M>();
-  constexpr int RPL = 128 / (int)sizeof(T);
-  constexpr int LV = (M + RPL - 1) / RPL + 1;      // lines of a v column (start not line-aligned)
-  constexpr int LF = (M + 2 + RPL - 1) / RPL + 1;  // lines of an f column
-  constexpr int PER = C * LV + (C + 2) * LF;       // per tile and array pair
-  const int npair = a.dI != nullptr ? 2 : 1;
-  const int e = a.e;
+__host__ __device__ constexpr size_t win_bytes() { return (size_t)kWinCols * win_pitch<T>(M) * sizeof(T); }
+// Bytes before a window that reads of the rows above the first output reach:
+// less than e <= M / 2 elements.
+template <int M>
+__host__ __device__ constexpr size_t win_lead() { return 2 * (size_t)M; }
+
+// An issued window: `at` is the image row of element 0; the caller waits for
+// it with window_wait.
+struct Window {
+  int at;
+  bool bulk;   // copied by the TMA engine, on the group's barrier
+  bool sync;   // elements written by the threads
+};
+
+// Starts the copy of nc (at most the group's threads) columns from gx0 and nr
+// rows from gy0 of the N x N image at img (any of them outside the image; not
+// live: nothing) on the group's barrier i.  One bulk copy per column where
+// every 16-byte chunk lies wholly inside or outside the image (N a multiple
+// of the chunk, an aligned image): a loop of 16-byte cp.async over the
+// threads cost P3 and the adjoint's P1 several hundred instructions.  Else
+// the threads copy value by value.  The group is past gm.open().
+template <int M, typename T>
+__device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, int gy0,
+                                               int nr, int HP, T* __restrict__ win, const GroupMem<M>& gm, int i) {
+  constexpr int EPC = 16 / (int)sizeof(T);
+  constexpr int GT = Quad<M>::GT;
+  static_assert(kWinCols <= GT, "one thread per column");
+  const int t = threadIdx.x % GT;
+  Window w;
+  w.bulk = live && N % EPC == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
+  w.at = gy0 & (w.bulk ? -EPC : -2);
+  w.sync = live;
+  if (!live) return w;
+  if (w.bulk) {
+    // rows wanted: whole chunks; r0 .. r1 of them and columns c0 .. c1 - 1 lie in the image
+    const int n = (gy0 - w.at + nr + EPC - 1) & -EPC;
+    const int r0 = max(0, -w.at), r1 = max(r0, min(n, N - w.at));
+    const int c0 = min(nc, max(0, -gx0)), c1 = max(c0, min(nc, N - gx0));
+    const unsigned bytes = (unsigned)((r1 - r0) * sizeof(T));
+    if (t == 0) tc::mbar_expect_tx(gm.bar + i, (unsigned)(c1 - c0) * bytes);
+    __syncwarp();
+    if (t >= c0 && t < c1 && bytes)
+      tc::bulk_g2s(win + t * HP + r0, img + (long long)(gx0 + t) * N + w.at + r0, bytes, gm.bar + i);
+    w.sync = c1 - c0 < nc || r1 - r0 < n;
+    if (w.sync)
+      for (int c = 0; c < nc; ++c) {
+        const bool in = c >= c0 && c < c1;
+        for (int k = t; k < n; k += GT)
+          if (!in || k < r0 || k >= r1) win[c * HP + k] = T(0.f);
+      }
+  } else {
+    const int n = gy0 - w.at + nr;
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
-    const TileRef tr = tile_of(g, 2 * w2 + h);
-    if (!tr.live) continue;
-    const int x = tr.x0 + xb2 * C;
-    for (int idx = threadIdx.x; idx < PER * npair; idx += kThreads) {
-      const int d = idx / PER, r = idx % PER;
-      if (r < C * LV) {
-        const int col = x + r / LV - 2 * e, row0 = tr.y0 - 2 * e;
-        const int row = max(row0, 0) + (r % LV) * RPL;
-        if (col < 0 || col >= tr.W || row >= tr.W || row >= row0 + M) continue;
-        const T* v = static_cast<const T*>(d ? a.dv : a.v);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(v + tr.ow + (long long)col * tr.W + row));
-      } else {
-        const int rf = r - C * LV;
-        const int col = x + rf / LF - e - 1, row0 = tr.y0 - e - 1;
-        const int row = max(row0, 0) + (rf % LF) * RPL;
-        if (col < 0 || col >= tr.N || row >= tr.N || row >= row0 + M + 2) continue;
-        const T* f = static_cast<const T*>(d ? a.dI : a.I);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(f + tr.on + (long long)col * tr.N + row));
+    for (int c = 0; c < nc; ++c) {
+      const int gx = gx0 + c;
+      const bool colin = gx >= 0 && gx < N;
+      const T* col = img + (long long)(colin ? gx : 0) * N + w.at;
+      T* d = win + c * HP;
+      for (int k = t; k < n; k += GT) {
+        const bool in = colin && (unsigned)(w.at + k) < (unsigned)N;
+        if constexpr (sizeof(T) == 4)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                           static_cast<unsigned>(__cvta_generic_to_shared(d + k))),
+                       "l"(in ? col + k : img), "r"(in ? 4 : 0)
+                       : "memory");
+        else
+          d[k] = in ? col[k] : T(0.f);
       }
     }
   }
+  return w;
+}
+// The window has arrived for every thread of the group (group-uniform).
+template <int M>
+__device__ __forceinline__ void window_wait(const Window& w, GroupMem<M>& gm, int i) {
+  if (w.bulk)
+    gm.wait(i);
+  else
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (w.sync) group_sync<M>();
 }
 
+// This thread's column of one tile in a W- or N-sized array: rows y = 2q + l
+// + J r of the tile column lie in the array for 0 <= rel + l + J r < cnt.
+struct OutCol {
+  bool on;        // the column lies in the array
+  unsigned cnt;   // rows
+  int rel;        // row 2q relative to the first
+  long long off;  // element offset of row 2q in the batch array
+};
+// Adjoint-type fields h_x = v * df/dx, h_y = v * df/dy on the valid window,
+// zero elsewhere (or dv * df/dx + v * d(df)/dx for the tangent-adjoint).
+// Virtual coordinates are shifted by +e so that the full N x N output is the
+// valid part of the convolution of the zero-extended (N + 2e)^2 field
+// (srk_adj_load_tile, adjoint/srk_adjoint.cuh:169-200).
+//
+// Twice the central differences of a staged image at the pair of rows `row`,
+// row + 1 of window column 1 (win: the column left of this thread's).  ODD:
+// `row` is odd, the row pairs around it are aligned.
+template <bool ODD, typename T>
+__device__ __forceinline__ void diff2(const T* __restrict__ win, int HP, int row, pk& gx, pk& gy) {
+  const T* cm = win + row;
+  const T* cc = cm + HP;
+  const T* cp = cc + HP;
+  if constexpr (ODD) {
+    const pk lm = swin2(cm - 1), lp = swin2(cm + 1), rm = swin2(cp - 1), rp = swin2(cp + 1);
+    gx = pk_sub(pk_make(pk_hi(rm), pk_lo(rp)), pk_make(pk_hi(lm), pk_lo(lp)));
+    gy = pk_sub(swin2(cc + 1), swin2(cc - 1));
+  } else {
+    gx = pk_sub(swin2(cp), swin2(cm));
+    const pk c = swin2(cc);
+    gy = pk_make(__fsub_rn(pk_hi(c), swin(cc - 1)), __fsub_rn(swin(cc + 2), pk_lo(c)));
+  }
+}
+
+// v / 2 (the differences' factor; halving is exact) at this thread's rows of
+// the valid-window column o, zero outside.
+template <int M, typename T>
+__device__ __forceinline__ void load_cotangent(const T* __restrict__ v, const TileRef& t, const OutCol& o,
+                                               pk (&vv)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  const pk half = pk_dup(0.5f);
+  if (!((t.W | o.rel) & 1) && pair_aligned(v + t.ow)) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      vv[r] = ld2<true>(v + o.off, J * r, o.on && (unsigned)(o.rel + J * r) < o.cnt, true);
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      vv[r] = ld2<false>(v + o.off, J * r, o.on && (unsigned)(o.rel + J * r) < o.cnt,
+                         o.on && (unsigned)(o.rel + J * r + 1) < o.cnt);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) vv[r] = pk_mul(vv[r], half);
+}
+
+// One tile's h_x, h_y in the re (LANE 0) or im (LANE 1) parts: v * gradient
+// of the window wf, or (TAN) dv * gradient of wf + v * gradient of wd.  MASK:
+// some of the group's values lie outside the valid window.
+template <int M, typename T, bool TAN, int LANE, bool ODD, bool MASK>
+__device__ __forceinline__ void adj_fields(const pk (&vv)[Quad<M>::R], const pk (&dv)[Quad<M>::R], const OutCol& o,
+                                           const T* __restrict__ wf, const T* __restrict__ wd, int row,
+                                           cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J, HP = win_pitch<T>(M);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = J * r;
+    pk gx, gy;
+    diff2<ODD>(wf, HP, row + i, gx, gy);
+    if constexpr (TAN) {
+      pk dgx, dgy;
+      diff2<ODD>(wd, HP, row + i, dgx, dgy);
+      gx = pk_dot2(dv[r], gx, vv[r], dgx);
+      gy = pk_dot2(dv[r], gy, vv[r], dgy);
+    } else {
+      gx = pk_mul(vv[r], gx);
+      gy = pk_mul(vv[r], gy);
+    }
+    if constexpr (MASK) {
+      // outside the valid window exactly zero, whatever the image holds there
+      const bool lo = o.on && (unsigned)(o.rel + i) < o.cnt, hi = o.on && (unsigned)(o.rel + i + 1) < o.cnt;
+      gx = pk_make(lo ? pk_lo(gx) : 0.f, hi ? pk_hi(gx) : 0.f);
+      gy = pk_make(lo ? pk_lo(gy) : 0.f, hi ? pk_hi(gy) : 0.f);
+    }
+    (LANE ? hx[r].im : hx[r].re) = gx;
+    (LANE ? hy[r].im : hy[r].re) = gy;
+  }
+}
+template <int M, typename T, bool TAN, int LANE>
+__device__ __forceinline__ void adj_lane(const GroupMem<M>& gm, bool cols, const pk (&vv)[Quad<M>::R],
+                                         const pk (&dv)[Quad<M>::R], const OutCol& o,
+                                         const T* __restrict__ wf, const T* __restrict__ wd, int row,
+                                         cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  const int y0 = o.rel - 2 * gm.t.q;  // first tile row in the valid window (group-uniform, like `inside`)
+  const bool inside = cols && y0 >= 0 && y0 + M <= (int)o.cnt;
+  if (!inside) {
+    if (row & 1)
+      adj_fields<M, T, TAN, LANE, true, true>(vv, dv, o, wf, wd, row, hx, hy);
+    else
+      adj_fields<M, T, TAN, LANE, false, true>(vv, dv, o, wf, wd, row, hx, hy);
+  } else if (row & 1) {
+    adj_fields<M, T, TAN, LANE, true, false>(vv, dv, o, wf, wd, row, hx, hy);
+  } else {
+    adj_fields<M, T, TAN, LANE, false, false>(vv, dv, o, wf, wd, row, hx, hy);
+  }
+}
+
+// h_x, h_y of the group's columns for both tiles of the pair.  Two windows at
+// a time, in the exchange and the buffer: f of both tiles, or f and df of one
+// tile after the other; the cotangents are loaded while they arrive.
+template <int M, typename T, bool TAN>
+__device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, int blk, GroupMem<M>& gm,
+                                         cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
+  constexpr int HP = win_pitch<T>(M);
+  static_assert(win_bytes<M, T>() <= exch_bytes<M>() && win_bytes<M, T>() <= block_bytes<M>(), "window size");
+  const TileRef tr[2] = {tile_of(g, 2 * w), tile_of(g, 2 * w + 1)};
+  const int x = blk * kLines + gm.t.line, q2 = 2 * gm.t.q;
+  T* const w0 = reinterpret_cast<T*>(gm.ex);
+  T* const w1 = reinterpret_cast<T*>(gm.buf);
+  auto column = [&](const TileRef& t) {  // this thread's column of the tile in the valid window
+    const int ox = t.x0 + x - 2 * a.e;
+    OutCol o;
+    o.on = t.live && (unsigned)ox < (unsigned)t.W;
+    o.cnt = (unsigned)t.W;
+    o.rel = t.y0 - 2 * a.e + q2;
+    o.off = t.ow + (long long)ox * t.W + o.rel;
+    return o;
+  };
+  auto stage = [&](const TileRef& t, const void* img, int i) {
+    return issue_window<M, T>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
+                              t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, gm, i);
+  };
+  auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
+    const int ox = t.x0 + blk * kLines - 2 * a.e;
+    return t.live && ox >= 0 && ox + kLines <= t.W;
+  };
+  auto row = [&](const TileRef& t, const Window& wn) { return t.y0 - a.e + q2 - wn.at; };  // this thread's first row
+  gm.open();
+  const T* const f0 = w0 + gm.t.line * HP;
+  const T* const f1 = w1 + gm.t.line * HP;
+  const OutCol o0 = column(tr[0]), o1 = column(tr[1]);
+  if constexpr (TAN) {
+    pk vv[Quad<M>::R], dv[Quad<M>::R];
+    Window f = stage(tr[0], a.I, 0), d = stage(tr[0], a.dI, 1);
+    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, vv);
+    load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[0], o0, dv);
+    window_wait(f, gm, 0);
+    window_wait(d, gm, 1);
+    adj_lane<M, T, true, 0>(gm, inside(tr[0]), vv, dv, o0, f0, f1, row(tr[0], f), hx, hy);
+    gm.open();  // the windows are read
+    f = stage(tr[1], a.I, 0);
+    d = stage(tr[1], a.dI, 1);
+    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[1], o1, vv);
+    load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[1], o1, dv);
+    window_wait(f, gm, 0);
+    window_wait(d, gm, 1);
+    adj_lane<M, T, true, 1>(gm, inside(tr[1]), vv, dv, o1, f0, f1, row(tr[1], f), hx, hy);
+  } else {
+    pk v0[Quad<M>::R], v1[Quad<M>::R];
+    const Window f = stage(tr[0], a.I, 0), s = stage(tr[1], a.I, 1);
+    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, v0);
+    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[1], o1, v1);
+    window_wait(f, gm, 0);
+    window_wait(s, gm, 1);
+    adj_lane<M, T, false, 0>(gm, inside(tr[0]), v0, v0, o0, f0, f0, row(tr[0], f), hx, hy);
+    adj_lane<M, T, false, 1>(gm, inside(tr[1]), v1, v1, o1, f1, f1, row(tr[1], s), hx, hy);
+  }
+}
+
+// ---- P1 ------------------------------------------------------------------------------------
 // The transform of column x (ky = k_i + R m) -> S1[ky/4][x][ky%4].
 template <int M>
 __device__ __forceinline__ void p1_store(const float2 (&X)[Quad<M>::VPT], float2* __restrict__ S1k, int x, int q) {
@@ -631,8 +753,8 @@ __device__ __forceinline__ void p1_store(const float2 (&X)[Quad<M>::VPT], float2
 }
 
 // P1: the group transforms columns 4 blk .. 4 blk + 3 of every field along y.
-// OP_ADJ: TAN when dv and df are given; TESTED for erosion 0 (any TAN).
-template <int M, int OP, typename T, bool TAN = false, bool TESTED = false>
+// OP_ADJ: TAN when dv and df are given.
+template <int M, int OP, typename T, bool TAN = false>
 __device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, int blk, float2* __restrict__ S1,
                                        GroupMem<M>& gm, const float4* __restrict__ tw) {
   using Q = Quad<M>;
@@ -642,8 +764,7 @@ __device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, in
   if constexpr (OP == OP_ADJ) {
     // both fields from one pass over the inputs; h_y waits in registers
     cpk hx[Q::R], hy[Q::R];
-    load_adj_lane<M, T, TAN, TESTED, 0>(a, g, w, x, t.q, hx, hy);
-    load_adj_lane<M, T, TAN, TESTED, 1>(a, g, w, x, t.q, hx, hy);
+    load_adj<M, T, TAN>(a, g, w, blk, gm, hx, hy);
     fft_dit<M, false>(hx, X, gm.ex, tw, t);
     p1_store<M>(X, S1, x, t.q);
     fft_dit<M, false>(hy, X, gm.ex, tw, t);
@@ -678,11 +799,10 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
 #pragma unroll
       for (int m = 0; m < Q::J; ++m) X[i * Q::J + m] = src[4 * (Q::TPL * i + Q::R * m)];
   };
-  // spectrum quad of kx = 2q, 2q + 1 (+ J r): quad index 4 (q + J r / 2) + line of the block
-  const int go = 4 * t.q + t.line;
-  auto spec = [&](const float4* __restrict__ G, int r) {
-    cpk v = cpk_load(__ldg(G + row / 2 + go + r * (2 * Q::J)));
-    if (conjG) v.im = pk_neg(v.im);
+  // staged spectrum quad of kx = 2q, 2q + 1 (+ J r): quad 4 (q + J r / 2) + line of the block
+  auto spec = [&](int r) {
+    cpk v = cpk_load(gb[4 * t.q + t.line + r * (2 * Q::J)]);
+    if (K == 2 && conjG) v.im = pk_neg(v.im);
     return v;
   };
   auto emit = [&](const float2 (&X)[Q::VPT], int l) {
@@ -708,31 +828,37 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
     fft_dif_finish<M, false>(z);
     gm.wait(1);
 #pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], cpk_load(gb[go + r * (2 * Q::J)]));
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
     gm.open();
     gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the first inverse
     fft_dit<M, true>(b, X, gm.ex, tw, t);
     emit(X, 0);
     gm.wait(1);
 #pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], cpk_load(gb[go + r * (2 * Q::J)]));
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
     fft_dit<M, true>(b, X, gm.ex, tw, t);
     emit(X, 1);
   } else {
-    gm.fetch(1, gm.buf, S1 + (size_t)M * M + row, BB);
+    gm.fetch(1, gm.buf, Gx + row / 2, BB);
+    gm.wait(0);
+    load(gm.ex, X);
+    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
+    gm.open();  // the exchange is read: the second field takes its place
+    gm.fetch(0, gm.ex, S1 + (size_t)M * M + row, BB);
+    fft_dif_finish<M, false>(z);
+    gm.wait(1);
+#pragma unroll
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
+    gm.open();
+    gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the second transform
     gm.wait(0);
     load(gm.ex, X);
     fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
     fft_dif_finish<M, false>(z);
-#pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(Gx, r));
     gm.wait(1);
-    load(gm.buf, X);
-    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
-    fft_dif_finish<M, false>(z);
 #pragma unroll
     for (int r = 0; r < Q::R; ++r) {
-      const cpk c = cpk_mul<false>(z[r], spec(Gy, r));
+      const cpk c = cpk_mul<false>(z[r], spec(r));
       b[r] = cpk{pk_add(b[r].re, c.re), pk_add(b[r].im, c.im)};
     }
     fft_dit<M, true>(b, X, gm.ex, tw, t);
@@ -741,33 +867,14 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
 }
 
 // ---- P3 ------------------------------------------------------------------------------------
-// Gradient windows (forward and tangent).  The four output columns of a
-// group need the image columns gx - 1 .. gx + 4 and rows y0 + e - 1 ..
-// y0 + e + S: kWinCols columns of raw storage values in shared memory,
-// window column c <-> image column gx0 + c, element i <-> image row gya + i,
-// gya <= y0 + e - 1 even, so that the pair of rows (y, y + 1), y even, is one
-// aligned access.  Out-of-image elements are zero (the central-difference
-// rule).  Column pitch: 8 (mod 32) 4-byte words, so the pair reads of a
-// half-warp (four indices of four lines) fall on distinct banks.
-constexpr int kWinCols = kLines + 2;
-// Bytes before a window that reads of the rows above the first output reach:
-// less than e <= M / 2 elements.
-template <int M>
-__host__ __device__ constexpr size_t win_lead() { return 2 * (size_t)M; }
-template <typename T>
-__host__ __device__ constexpr int win_pitch(int S) {
-  // holds off + S + 2 elements, off = y0 + e - 1 - gya < 16 / sizeof(T)
-  return sizeof(T) == 4 ? (S + 5 + 23) / 32 * 32 + 8 : (S + 9 + 47) / 64 * 64 + 16;
-}
-template <int M, typename T>
-__host__ __device__ constexpr size_t win_bytes() { return (size_t)kWinCols * win_pitch<T>(M) * sizeof(T); }
-
 template <int OP>
 __host__ __device__ constexpr bool grad_op() { return OP == OP_FWD || OP == OP_JVP; }
-// Shared memory of a block in each pass (P1 has one landing zone, P3 of the
-// adjoint one field).
-template <int M>
-__host__ __device__ constexpr size_t p1_smem_bytes() { return groups_of<M>() * group_bytes<M, false>(); }
+// Shared memory of a block in each pass (P1 of the single-field ops has one
+// landing zone, P3 of the adjoint one field).
+template <int OP>
+__host__ __device__ constexpr bool p1_buf() { return OP == OP_ADJ; }
+template <int M, int OP>
+__host__ __device__ constexpr size_t p1_smem_bytes() { return groups_of<M>() * group_bytes<M, p1_buf<OP>()>(); }
 template <int M>
 __host__ __device__ constexpr size_t p2_smem_bytes() { return groups_of<M>() * group_bytes<M, true>(); }
 template <int OP>
@@ -775,68 +882,6 @@ __host__ __device__ constexpr bool p3_buf() { return OpTraits<OP>::L == 2; }
 template <int M, int OP>
 __host__ __device__ constexpr size_t p3_smem_bytes() { return groups_of<M>() * group_bytes<M, p3_buf<OP>()>(); }
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// Starts the copy of one window (16-byte asynchronous chunks where every
-// chunk lies wholly inside or outside the image: N a multiple of the chunk,
-// an aligned image, first row inside; else 4-byte asynchronous copies, or
-// plain ones for 2-byte values) and returns gya.  One commit group.
-template <int M, typename T>
-__device__ __forceinline__ int issue_window(const T* __restrict__ img, const TileRef& tr, int gx0, int e, int S,
-                                            T* __restrict__ win) {
-  constexpr int EPC = 16 / (int)sizeof(T);
-  constexpr int GT = Quad<M>::GT;
-  const int N = tr.N, HP = win_pitch<T>(S);
-  const int gy0 = tr.y0 + e - 1;
-  const int t = threadIdx.x % GT;
-  const bool vec = N % EPC == 0 && gy0 >= 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
-  const int gya = vec ? gy0 - gy0 % EPC : gy0 - (gy0 & 1);
-  const int nel = gy0 - gya + S + 2;
-  if (tr.live) {
-#pragma unroll 1
-    for (int c = 0; c < kWinCols; ++c) {
-      const int gx = gx0 + c;
-      const bool colin = gx >= 0 && gx < N;
-      const T* col = img + (long long)(colin ? gx : 0) * N + gya;
-      T* d = win + c * HP;
-      if (vec) {
-        const int lim = colin ? N - gya : 0;  // elements of this column inside the image
-        for (int i = EPC * t; i < nel; i += EPC * GT) {
-          const bool in = i < lim;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                           static_cast<unsigned>(__cvta_generic_to_shared(d + i))),
-                       "l"(in ? col + i : img), "r"(in ? 16 : 0)
-                       : "memory");
-        }
-      } else {
-        for (int i = t; i < nel; i += GT) {
-          const int gy = gya + i;
-          const bool in = colin && gy >= 0 && gy < N;
-          if constexpr (sizeof(T) == 4)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                             static_cast<unsigned>(__cvta_generic_to_shared(d + i))),
-                         "l"(in ? col + i : img), "r"(in ? 4 : 0)
-                         : "memory");
-          else
-            d[i] = in ? col[i] : T(0.f);
-        }
-      }
-    }
-  }
-  cp_async_commit();
-  return gya;
-}
-
-// This thread's output column of one tile: rows y = 2q + l + J r of tile
-// column x are outputs for e <= y < e + cnt.
-struct OutCol {
-  bool on;        // the column has outputs
-  unsigned cnt;   // valid rows
-  int rel;        // 2q - e: row 2q relative to the first valid one
-  long long off;  // element offset of row 2q in the output batch array
-};
 template <int M>
 __device__ __forceinline__ OutCol out_col(const Geom& g, const TileRef& tr, int x, int q, bool nsized) {
   OutCol o;
@@ -953,10 +998,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
   // the windows take the place of the second field (once every thread has
   // read it) and of the last exchange
   T* win[2] = {reinterpret_cast<T*>(gm.buf), reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(gm.ex) + win_lead<M>())};
-  int gya[2] = {0, 0};
+  Window wn[2];
   auto window = [&](int h) {
     const TileRef tr = tile_h(h);
-    gya[h] = issue_window<M, T>(image_h(h, tr), tr, tr.x0 + xg - 1, g.e, g.S, win[h]);
+    wn[h] = issue_window<M, T>(image_h(h, tr), tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2,
+                               win_pitch<T>(g.S), win[h], gm, 1 - h);
   };
   // column x of a staged S2 block: ky = k_i + R m
   auto load = [&](const void* blkmem, float2 (&X)[Q::VPT]) {
@@ -981,24 +1027,21 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     fft_dif_finish<M, true>(u0);
     gm.wait(1);
     load(gm.buf, X);
+    tc::fence_async_smem();  // the buffer's next copy comes after these reads
     fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
       if constexpr (GRAD) window(0);
     });
   }
   if constexpr (GRAD) {
-    group_sync<M>();  // the exchange is read: window 1 takes its place
+    gm.open();  // the exchange is read: window 1 takes its place
     window(1);
     fft_dif_finish<M, true>(u1);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      if (h == 0)
-        cp_async_wait<1>();
-      else
-        cp_async_wait<0>();
-      group_sync<M>();
+      window_wait(wn[h], gm, 1 - h);
       const TileRef tr = tile_h(h);
       const OutCol o = out_col<M>(g, tr, x, t.q, false);
-      const int row0 = tr.y0 + 2 * t.q - gya[h], HP = win_pitch<T>(g.S);
+      const int row0 = tr.y0 + 2 * t.q - wn[h].at, HP = win_pitch<T>(g.S);
       if (!o.on) continue;
       auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
       const bool vec = out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy);
@@ -1038,23 +1081,16 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
 template <int M>
 __device__ __forceinline__ int group_index() { return threadIdx.x / Quad<M>::GT; }
 
-// ahead (OP_ADJ): launch positions between this CTA and the one whose inputs
-// it prefetches into L2 (0: none).
-template <int M, int OP, typename T, bool TAN = false, bool TESTED = false>
+// TAN (adjoint-type op of the tangent-adjoint, dv and df given) is chosen by
+// the launch.
+template <int M, int OP, typename T, bool TAN = false>
 __global__ void __launch_bounds__(kThreads, OP == OP_ADJ ? SRK_P1_ADJ_MIN_BLOCKS : SRK_P1_MIN_BLOCKS)
-k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict__ scratch, int ahead) {
-  // TAN and TESTED (adjoint-type op) are chosen by the launch: TESTED for
-  // erosion 0, else TAN exactly when dv and df are given
+k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict__ scratch) {
   extern __shared__ __align__(16) unsigned char sm[];
-  GroupMem<M> gm = group_mem<M, false>(sm, g.err);
+  GroupMem<M> gm = group_mem<M, p1_buf<OP>()>(sm, g.err);
   const int wl = blockIdx.y;
-  if constexpr (OP == OP_ADJ && !TESTED) {
-    const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x) + ahead;
-    const int by2 = lin / (int)gridDim.x, bx2 = lin % (int)gridDim.x;
-    if (ahead > 0 && by2 < (int)gridDim.y) p1_prefetch_adj<M, T>(a, g, w0 + by2, bx2);
-  }
-  phase1<M, OP, T, TAN, TESTED>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
-                                scratch + wl * wt_elems<M, OP>(g.S), gm, tw);
+  phase1<M, OP, T, TAN>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
+                        scratch + wl * wt_elems<M, OP>(g.S), gm, tw);
 }
 
 template <int M, int OP>
@@ -1184,7 +1220,10 @@ k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restr
       float2* base = scratch + (size_t)slot * slot_elems;
       const int blk = unit * NG + group_index<M>();
       if (phase == 1) {
-        phase1<M, OP, T, false, OP == OP_ADJ>(a, g, w, blk, base, gm, tw);
+        if (OP == OP_ADJ && a.dI != nullptr)
+          phase1<M, OP, T, OP == OP_ADJ>(a, g, w, blk, base, gm, tw);
+        else
+          phase1<M, OP, T>(a, g, w, blk, base, gm, tw);
       } else if (phase == 2) {
         phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blk, gm, tw);
       } else if (blk < nblk) {
