@@ -104,8 +104,9 @@ struct RagImage {
 // its tiles in `rtile` (image, x0, y0) and its images in `rimg`.
 struct Geom {
   int M;      // FFT tile size
-  int e;      // erosion (kernel half width bound)
-  int S;      // valid outputs per tile per axis (<= M - 2e)
+  int e;      // first valid local output of a tile (the erosion, or 0: see adj_geom)
+  int S;      // valid outputs per tile per axis
+  int org;    // origin of the first tile in virtual coordinates (uniform batch)
   int T;      // tiles per axis (uniform batch)
   int Nin;    // virtual input size (N for forward-type, N + 2e for adjoint)
   int Wout;   // output size (W for forward-type, N for adjoint)
@@ -174,8 +175,8 @@ __device__ __forceinline__ TileRef tile_of(const Geom& g, int u) {
   } else {
     if (g.TT == 1) {  // one tile per image (tile size >= image): no divisions
       t.b = uu;
-      t.x0 = 0;
-      t.y0 = 0;
+      t.x0 = g.org;
+      t.y0 = g.org;
     } else {
       t.b = uu / g.TT;
       const int r = uu - t.b * g.TT;
@@ -882,17 +883,19 @@ __host__ __device__ constexpr bool p3_buf() { return OpTraits<OP>::L == 2; }
 template <int M, int OP>
 __host__ __device__ constexpr size_t p3_smem_bytes() { return groups_of<M>() * group_bytes<M, p3_buf<OP>()>(); }
 
+// Virtual coordinates are output coordinates + the erosion.
 template <int M>
-__device__ __forceinline__ OutCol out_col(const Geom& g, const TileRef& tr, int x, int q, bool nsized) {
+__device__ __forceinline__ OutCol out_col(const Geom& g, int erosion, const TileRef& tr, int x, int q, bool nsized) {
   OutCol o;
-  const int ox = tr.x0 + x - g.e;
+  const int ox = tr.x0 + x - erosion, oy = tr.y0 + g.e - erosion;  // output column, first valid output row
   o.on = tr.live && x >= g.e && x < g.e + g.S && ox < tr.Wout;
-  o.cnt = (unsigned)max(0, min(g.S, tr.Wout - tr.y0));
+  o.cnt = (unsigned)max(0, min(g.S, tr.Wout - oy));
   o.rel = 2 * q - g.e;
-  o.off = (nsized ? tr.on + (long long)ox * tr.N : tr.ow + (long long)ox * tr.W) + tr.y0 + o.rel;
+  o.off = (nsized ? tr.on + (long long)ox * tr.N : tr.ow + (long long)ox * tr.W) + oy + o.rel;
   return o;
 }
-// Every pair of rows is one aligned access, wholly valid or wholly not.
+// Every pair of rows is one aligned access, wholly valid or wholly not (the
+// first valid output row of a tile is even).
 __device__ __forceinline__ bool out_even(const Geom& g, const TileRef& tr) { return !((g.e | tr.Wout) & 1); }
 
 // Forward / tangent epilogue, round h, with the central differences read
@@ -1040,7 +1043,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     for (int h = 0; h < 2; ++h) {
       window_wait(wn[h], gm, 1 - h);
       const TileRef tr = tile_h(h);
-      const OutCol o = out_col<M>(g, tr, x, t.q, false);
+      const OutCol o = out_col<M>(g, a.e, tr, x, t.q, false);
       const int row0 = tr.y0 + 2 * t.q - wn[h].at, HP = win_pitch<T>(g.S);
       if (!o.on) continue;
       auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
@@ -1057,7 +1060,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     for (int h = 0; h < NH; ++h) {
       const TileRef tr = tile_h(h);
       constexpr bool NS = OP == OP_ADJ;
-      const OutCol o = out_col<M>(g, tr, x, t.q, NS);
+      const OutCol o = out_col<M>(g, a.e, tr, x, t.q, NS);
       if (!o.on) continue;
       bool vec = out_even(g, tr);
       if constexpr (NS) {

@@ -65,20 +65,37 @@ Geom fwd_geom(const srk_plan_s* p, int B) {
   g.err = p->direct_err;
   return g;
 }
-Geom adj_geom(const srk_plan_s* p, int B) {
+// Tiles per axis of the adjoint geometry.  Its input is zero outside the
+// valid window [e, N - e) of the image, so for N <= M one circular transform
+// of the whole image wraps only zeros into the N outputs: the conv of a
+// support of N - 2e with 2e + 1 taps is N <= M long.  One tile then yields all
+// N outputs (valid range 0 .. N), where overlapping tiles of stride M - 2e
+// need ceil(N / (M - 2e)) per axis (four tiles for N = M).
+bool adj_single(const srk_plan_s* p) { return p->N <= p->M; }
+// General (overlapping) adjoint tiles, also for ragged batches and slabs.
+Geom adj_tiles_geom(const srk_plan_s* p, int B) {
   Geom g;
   std::memset(&g, 0, sizeof(g));
-  g.M = p->M; g.e = p->e; g.S = p->S; g.T = p->Ta;
-  g.Nin = p->N + 2 * p->e; g.Wout = p->N; g.TT = p->Ta * p->Ta; g.U = B * g.TT;
+  g.M = p->M; g.e = p->e; g.S = p->S; g.T = (p->N + p->S - 1) / p->S;
+  g.Nin = p->N + 2 * p->e; g.Wout = p->N; g.TT = g.T * g.T; g.U = B * g.TT;
   g.N = p->N; g.W = p->W; g.wout_n = 1;
   g.err = p->direct_err;
   return g;
 }
+Geom adj_geom(const srk_plan_s* p, int B) {
+  Geom g = adj_tiles_geom(p, B);
+  if (adj_single(p)) {
+    g.e = 0; g.S = p->N; g.org = p->e; g.T = g.TT = 1; g.U = B;
+  }
+  return g;
+}
 
-size_t wt_bytes(int M, int S) {
+// Scratch of the largest work tile: the forward's fields at stride S, the
+// adjoint's at S or (single) with every column valid.
+size_t wt_bytes(int M, int S, bool single) {
   const size_t P = (size_t)s2_pitch(S);
   const size_t fwd = (size_t)M * M + 2 * P * M;
-  const size_t adj = 2 * (size_t)M * M + P * M;
+  const size_t adj = 2 * (size_t)M * M + (single ? (size_t)M : P) * M;
   return sizeof(float2) * (fwd > adj ? fwd : adj);
 }
 
@@ -377,11 +394,11 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
   p->M = M; p->S = M - 2 * erosion;
   p->schedule = sched;
   p->T = (W + p->S - 1) / p->S;
-  p->Ta = (N + p->S - 1) / p->S;
+  p->Ta = adj_single(p) ? 1 : (N + p->S - 1) / p->S;
   const size_t nwt_max = std::max<size_t>({(size_t)(B_max * (size_t)p->T * p->T + 1) / 2,
                                            (size_t)B_max * p->T * p->T,
                                            (size_t)(B_max * (size_t)p->Ta * p->Ta + 1) / 2});
-  const size_t per = wt_bytes(M, p->S);
+  const size_t per = wt_bytes(M, p->S, adj_single(p));
   // default scratch: 8 GiB, at most 1/16 of the device memory, at least
   // 256 MiB.  At B=5000 on the B200 it holds the whole N=256 batch (one
   // chunk: -4% against 1 GiB) and N=512 runs in 15 launches (-1.3%); the
@@ -1002,7 +1019,7 @@ srk_status slab_tables_ta(srk_plan_s* p, int N, int c0, int c1, int* r0o, int* r
 }
 
 Geom ragged_geom(const srk_plan_s* p, bool adj) {
-  Geom g = adj ? adj_geom(p, 1) : fwd_geom(p, 1);
+  Geom g = adj ? adj_tiles_geom(p, 1) : fwd_geom(p, 1);
   g.U = adj ? p->rag_ntiles_adj : p->rag_ntiles_fwd;
   g.rtile = p->rag_tiles + (adj ? p->rag_ntiles_fwd : 0);
   g.rimg = p->rag_imgs;

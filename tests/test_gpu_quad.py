@@ -93,3 +93,35 @@ def test_storage_types_equal_the_fp32_routes(torch_cuda, tile, N, KW, B, dt):
         res.append([x.to(T) for x in (h, df, dg)])
     for x, y in zip(*res):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("conv", [srk.SRK_ADJ_REFERENCE, srk.SRK_ADJ_TRUE])
+@pytest.mark.parametrize("tile,N,KW", [(128, 128, 1), (128, 128, 3), (128, 101, 33), (128, 128, 113), (256, 256, 61),
+                                       (256, 255, 31), (256, 200, 121), (512, 512, 121), (512, 509, 31)])
+def test_adjoint_of_an_image_within_one_tile(torch_cuda, tile, N, KW, conv):
+    """N <= tile: the adjoint with respect to g runs as one circular tile per
+    image, up to N = tile, where the outputs fill the transform; against the
+    oracle and against the overlapping tiles of a ragged call."""
+    torch = torch_cuda
+    e = (KW - 1) // 2
+    W = N - 2 * e
+    rng = np.random.default_rng(N + KW)
+    Kx, Ky = (rng.standard_normal((KW, KW)).astype(np.float32) / KW for _ in range(2))
+    B = 3
+    f = np.stack(fields(N, B, 50 + N))
+    v = rng.standard_normal((B, W, W)).astype(np.float32)
+    plan = srk.SrkPlan(N, W, e, 1.0, B, spectra_M=tile, tile_M=tile)
+    plan.set_adj_convention(conv)
+    plan.set_kernel(dev(Kx, torch), dev(Ky, torch))
+    fd, vd = dev(f, torch), dev(v, torch)
+    u = torch.zeros((B, W, W), device="cuda")
+    dI, dE, rE = (torch.full((B, N, N), float("nan"), device="cuda") for _ in range(3))
+    for b in range(B):
+        srk.adjointSRK(vd[b], u[b], u[b], fd[b], None, None, N, W, e, 1.0, None, dI[b], dE[b], plan)
+    srk.adjointSRKRagged(vd, u, u, fd, None, None, [N] * B, e, 1.0, None, dI, rE, plan)
+    plan.sync()
+    name = "true" if conv == srk.SRK_ADJ_TRUE else "reference"
+    for b in range(B):
+        ref = O.adj_wrt_E(v[b], f[b], Kx, Ky, e, 1.0, name)
+        assert rel_max_err(host(dE[b]), ref) < TOL
+        assert rel_max_err(host(rE[b]), ref) < TOL
