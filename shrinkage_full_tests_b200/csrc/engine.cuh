@@ -504,13 +504,41 @@ struct Window {
   bool sync;   // elements written by the threads
 };
 
+// Rows [at, end) of the nc columns from gx0 in asynchronous pieces of BYTES (2:
+// plain copies of single values), each wholly inside or outside the image.
+template <int M, typename T, int BYTES>
+__device__ __forceinline__ void window_pieces(const T* __restrict__ img, int N, int gx0, int nc, int at, int end, int HP,
+                                              T* __restrict__ win) {
+  constexpr int E = BYTES / (int)sizeof(T) ? BYTES / (int)sizeof(T) : 1;
+  constexpr int GT = Quad<M>::GT;
+  const int t = threadIdx.x % GT;
+#pragma unroll 1
+  for (int c = 0; c < nc; ++c) {
+    const int gx = gx0 + c;
+    const bool colin = gx >= 0 && gx < N;
+    const T* col = img + (long long)(colin ? gx : 0) * N + at;
+    T* d = win + c * HP;
+    for (int k = E * t; k < end - at; k += E * GT) {
+      const bool in = colin && (unsigned)(at + k) < (unsigned)N;
+      if constexpr (BYTES > 2)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;\n" ::"r"(
+                         static_cast<unsigned>(__cvta_generic_to_shared(d + k))),
+                     "l"(in ? col + k : img), "r"(in ? BYTES : 0), "n"(BYTES)
+                     : "memory");
+      else
+        d[k] = in ? col[k] : T(0.f);
+    }
+  }
+}
+
 // Starts the copy of nc (at most the group's threads) columns from gx0 and nr
 // rows from gy0 of the N x N image at img (any of them outside the image; not
 // live: nothing) on the group's barrier i.  One bulk copy per column where
 // every 16-byte chunk lies wholly inside or outside the image (N a multiple
 // of the chunk, an aligned image): a loop of 16-byte cp.async over the
 // threads cost P3 and the adjoint's P1 several hundred instructions.  Else
-// the threads copy value by value.  The group is past gm.open().
+// the threads copy the largest pieces that N and the image allow.  The group
+// is past gm.open().
 template <int M, typename T>
 __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, int gy0,
                                                int nr, int HP, T* __restrict__ win, const GroupMem<M>& gm, int i) {
@@ -522,7 +550,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   w.bulk = live && N % EPC == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
   w.at = gy0 & (w.bulk ? -EPC : -2);
   w.sync = live;
-  if (!live) return w;
+  if (!live) return w;  // (nothing reads the window of a dead tile)
   if (w.bulk) {
     // rows wanted: whole chunks; r0 .. r1 of them and columns c0 .. c1 - 1 lie in the image
     const int n = (gy0 - w.at + nr + EPC - 1) & -EPC;
@@ -540,25 +568,13 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
         for (int k = t; k < n; k += GT)
           if (!in || k < r0 || k >= r1) win[c * HP + k] = T(0.f);
       }
+  } else if ((N * (int)sizeof(T)) % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 7) == 0) {
+    window_pieces<M, T, 8>(img, N, gx0, nc, w.at & (sizeof(T) == 4 ? -2 : -4), gy0 + nr, HP, win);
+    w.at &= sizeof(T) == 4 ? -2 : -4;
+  } else if ((N * (int)sizeof(T)) % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3) == 0) {
+    window_pieces<M, T, 4>(img, N, gx0, nc, w.at, gy0 + nr, HP, win);
   } else {
-    const int n = gy0 - w.at + nr;
-#pragma unroll 1
-    for (int c = 0; c < nc; ++c) {
-      const int gx = gx0 + c;
-      const bool colin = gx >= 0 && gx < N;
-      const T* col = img + (long long)(colin ? gx : 0) * N + w.at;
-      T* d = win + c * HP;
-      for (int k = t; k < n; k += GT) {
-        const bool in = colin && (unsigned)(w.at + k) < (unsigned)N;
-        if constexpr (sizeof(T) == 4)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                           static_cast<unsigned>(__cvta_generic_to_shared(d + k))),
-                       "l"(in ? col + k : img), "r"(in ? 4 : 0)
-                       : "memory");
-        else
-          d[k] = in ? col[k] : T(0.f);
-      }
-    }
+    window_pieces<M, T, 2>(img, N, gx0, nc, w.at, gy0 + nr, HP, win);
   }
   return w;
 }
@@ -870,6 +886,9 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
 // ---- P3 ------------------------------------------------------------------------------------
 template <int OP>
 __host__ __device__ constexpr bool grad_op() { return OP == OP_FWD || OP == OP_JVP; }
+// Operators whose epilogue multiplies by cotangents (W-sized images).
+template <int OP>
+__host__ __device__ constexpr bool cot_op() { return OP == OP_VJP_F || OP == OP_TANADJ_F; }
 // Shared memory of a block in each pass (P1 of the single-field ops has one
 // landing zone, P3 of the adjoint one field).
 template <int OP>
@@ -943,33 +962,47 @@ __device__ __forceinline__ void grad_round(const OpArgs& a, const OutCol& o, int
   }
 }
 
-// The other epilogues.  VJP (f): w = u * v of image h; tangent-adjoint (f):
-// w = dlam * Re + lam * Im; adjoint: the full N x N output of image h.
-template <int M, int OP, typename T, bool VEC>
-__device__ __forceinline__ void plain_epilogue(const OpArgs& a, const OutCol& o, int h, const cpk (&u0)[Quad<M>::R],
-                                               const cpk (&u1)[Quad<M>::R]) {
+// Epilogue of the cotangent ops, from the staged window(s) of the cotangent
+// (element `row` = tile row 2q of this line's column).  VJP (f): w = u * v of
+// image h; tangent-adjoint (f): w = dlam * Re + lam * Im.  ODD: row is odd.
+template <int M, int OP, typename T, bool VEC, bool ODD>
+__device__ __forceinline__ void cot_epilogue(const OpArgs& a, const OutCol& o, int h, const T* __restrict__ v,
+                                             const T* __restrict__ dv, const cpk (&u0)[Quad<M>::R],
+                                             const cpk (&u1)[Quad<M>::R]) {
+  constexpr int R = Quad<M>::R, J = Quad<M>::J;
+  float* __restrict__ WX = static_cast<float*>(a.out0) + o.off;
+  float* __restrict__ WY = static_cast<float*>(a.out1) + o.off;
+  auto pair = [](const T* p) { return ODD ? pk_make(swin(p), swin(p + 1)) : swin2(p); };
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = J * r;
+    const bool lo = (unsigned)(o.rel + i) < o.cnt;
+    const bool hi = VEC ? lo : (unsigned)(o.rel + i + 1) < o.cnt;
+    const pk vv = pair(v + i);
+    pk wx, wy;
+    if constexpr (OP == OP_VJP_F) {
+      wx = pk_mul(h ? u0[r].im : u0[r].re, vv);
+      wy = pk_mul(h ? u1[r].im : u1[r].re, vv);
+    } else {
+      const pk dd = pair(dv + i);
+      wx = pk_dot2(dd, u0[r].re, vv, u0[r].im);
+      wy = pk_dot2(dd, u1[r].re, vv, u1[r].im);
+    }
+    st2<VEC>(WX, i, wx, lo, hi);
+    st2<VEC>(WY, i, wy, lo, hi);
+  }
+}
+
+// Epilogue of the adjoint: the full N x N output of image h.
+template <int M, typename T, bool VEC>
+__device__ __forceinline__ void adj_epilogue(const OpArgs& a, const OutCol& o, int h, const cpk (&u)[Quad<M>::R]) {
   constexpr int R = Quad<M>::R, J = Quad<M>::J;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int i = J * r;
     const bool lo = (unsigned)(o.rel + i) < o.cnt;
     const bool hi = VEC ? lo : (unsigned)(o.rel + i + 1) < o.cnt;
-    if constexpr (OP == OP_ADJ) {
-      st2<VEC>(static_cast<T*>(a.out0) + o.off, i, h ? u0[r].im : u0[r].re, lo, hi);
-    } else {
-      const pk v = ld2<VEC>(static_cast<const T*>(a.v) + o.off, i, lo, hi);
-      pk wx, wy;
-      if constexpr (OP == OP_VJP_F) {
-        wx = pk_mul(h ? u0[r].im : u0[r].re, v);
-        wy = pk_mul(h ? u1[r].im : u1[r].re, v);
-      } else {
-        const pk dv = ld2<VEC>(static_cast<const T*>(a.dv) + o.off, i, lo, hi);
-        wx = pk_dot2(dv, u0[r].re, v, u0[r].im);
-        wy = pk_dot2(dv, u1[r].re, v, u1[r].im);
-      }
-      st2<VEC>(static_cast<float*>(a.out0) + o.off, i, wx, lo, hi);
-      st2<VEC>(static_cast<float*>(a.out1) + o.off, i, wy, lo, hi);
-    }
+    st2<VEC>(static_cast<T*>(a.out0) + o.off, i, h ? u[r].im : u[r].re, lo, hi);
   }
 }
 
@@ -984,10 +1017,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
                                        GroupMem<M>& gm, const float4* __restrict__ tw) {
   using Q = Quad<M>;
   constexpr int L = OpTraits<OP>::L;
-  constexpr bool GRAD = grad_op<OP>();
+  constexpr bool GRAD = grad_op<OP>(), WIN = L == 2;
+  static_assert(GRAD || cot_op<OP>() || L == 1, "two-field ops have windows");
   constexpr unsigned BB = (unsigned)block_bytes<M>();
   // rows below the last output reach less than e elements past a window
-  static_assert(!GRAD || (win_bytes<M, T>() + 2 * win_lead<M>() <= exch_bytes<M>() &&
+  static_assert(!WIN || (win_bytes<M, T>() + 2 * win_lead<M>() <= exch_bytes<M>() &&
                           win_bytes<M, T>() + win_lead<M>() <= block_bytes<M>()),
                 "the windows reuse the buffer (behind the exchange) and the exchange");
   const QuadThread t = gm.t;
@@ -995,17 +1029,22 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
   const int xg = (S2L == kS2Rotated ? g.e : s2_first(g.e)) + blk * kLines;  // the group's first tile column
   const int x = xg + t.line;
   auto tile_h = [&](int h) { return tile_of(g, OpTraits<OP>::PAIRS ? 2 * w + h : w); };
-  auto image_h = [&](int h, const TileRef& tr) {
-    return static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
-  };
   // the windows take the place of the second field (once every thread has
-  // read it) and of the last exchange
+  // read it) and of the last exchange: f (and df) around the group's columns,
+  // or v (lam and dlam) at the group's output columns
   T* win[2] = {reinterpret_cast<T*>(gm.buf), reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(gm.ex) + win_lead<M>())};
   Window wn[2];
+  const int HP = win_pitch<T>(g.S);
   auto window = [&](int h) {
     const TileRef tr = tile_h(h);
-    wn[h] = issue_window<M, T>(image_h(h, tr), tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2,
-                               win_pitch<T>(g.S), win[h], gm, 1 - h);
+    if constexpr (GRAD) {
+      const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
+      wn[h] = issue_window<M, T>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2, HP, win[h],
+                                 gm, 1 - h);
+    } else {
+      const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
+      wn[h] = issue_window<M, T>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], gm, 1 - h);
+    }
   };
   // column x of a staged S2 block: ky = k_i + R m
   auto load = [&](const void* blkmem, float2 (&X)[Q::VPT]) {
@@ -1032,49 +1071,56 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     load(gm.buf, X);
     tc::fence_async_smem();  // the buffer's next copy comes after these reads
     fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
-      if constexpr (GRAD) window(0);
+      window(0);
     });
   }
-  if constexpr (GRAD) {
+  if constexpr (WIN) {
     gm.open();  // the exchange is read: window 1 takes its place
     window(1);
     fft_dif_finish<M, true>(u1);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       window_wait(wn[h], gm, 1 - h);
+      if (OP == OP_TANADJ_F && h == 0) continue;  // both windows at once
       const TileRef tr = tile_h(h);
       const OutCol o = out_col<M>(g, a.e, tr, x, t.q, false);
-      const int row0 = tr.y0 + 2 * t.q - wn[h].at, HP = win_pitch<T>(g.S);
       if (!o.on) continue;
-      auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
-      const bool vec = out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy);
-      if (vec)
-        grad_round<M, OP, T, true>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
-      else
-        grad_round<M, OP, T, false>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
+      if constexpr (GRAD) {
+        const int row0 = tr.y0 + 2 * t.q - wn[h].at;
+        auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
+        const bool vec = out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy);
+        if (vec)
+          grad_round<M, OP, T, true>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
+        else
+          grad_round<M, OP, T, false>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
+      } else {
+        constexpr int H1 = OP == OP_TANADJ_F ? 0 : 1;  // the window of v
+        const int hv = H1 ? h : 0;
+        const int row = tr.y0 + o.rel - wn[hv].at, drow = tr.y0 + o.rel - wn[1].at;
+        const T* v = win[hv] + t.line * HP + row;
+        const T* dv = win[1] + t.line * HP + drow;
+        const bool vec = out_even(g, tr) && pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
+                         pair_aligned(static_cast<const float*>(a.out1) + tr.ow);
+        // both windows start at even rows: one parity
+        if ((row & 1) == 0 && vec)
+          cot_epilogue<M, OP, T, true, false>(a, o, h, v, dv, u0, u1);
+        else if ((row & 1) == 0)
+          cot_epilogue<M, OP, T, false, false>(a, o, h, v, dv, u0, u1);
+        else
+          cot_epilogue<M, OP, T, false, true>(a, o, h, v, dv, u0, u1);
+      }
     }
   } else {
-    fft_dif_finish<M, true>(L == 2 ? u1 : u0);
-    constexpr int NH = OpTraits<OP>::PAIRS ? 2 : 1;
+    fft_dif_finish<M, true>(u0);
 #pragma unroll
-    for (int h = 0; h < NH; ++h) {
+    for (int h = 0; h < 2; ++h) {
       const TileRef tr = tile_h(h);
-      constexpr bool NS = OP == OP_ADJ;
-      const OutCol o = out_col<M>(g, a.e, tr, x, t.q, NS);
+      const OutCol o = out_col<M>(g, a.e, tr, x, t.q, true);
       if (!o.on) continue;
-      bool vec = out_even(g, tr);
-      if constexpr (NS) {
-        vec = vec && pair_aligned(static_cast<const T*>(a.out0) + tr.on);
-      } else {
-        vec = vec && pair_aligned(static_cast<const T*>(a.v) + tr.ow) &&
-              pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
-              pair_aligned(static_cast<const float*>(a.out1) + tr.ow);
-        if (OP == OP_TANADJ_F) vec = vec && pair_aligned(static_cast<const T*>(a.dv) + tr.ow);
-      }
-      if (vec)
-        plain_epilogue<M, OP, T, true>(a, o, h, u0, u1);
+      if (out_even(g, tr) && pair_aligned(static_cast<const T*>(a.out0) + tr.on))
+        adj_epilogue<M, T, true>(a, o, h, u0);
       else
-        plain_epilogue<M, OP, T, false>(a, o, h, u0, u1);
+        adj_epilogue<M, T, false>(a, o, h, u0);
     }
   }
 }
@@ -1258,68 +1304,176 @@ static __global__ void k_wait_selftest(Ctl* ctl, unsigned long long spin_limit) 
 // window (zero outside); adjoint of the central difference
 // (adjointWrtI_kernel, adjoint/srk_adjoint.cuh:25-59).  With ux, uy, v
 // given instead (the reference contract) w = u*v is formed on the fly.
-// A thread computes kStencilCols consecutive columns of one row: the
-// kStencilCols + 2 values of wx it needs are loaded once, and every load is
-// issued before the first use.
-constexpr int kStencilCols = 4;
-template <typename T, bool FROM_U>
-__device__ __forceinline__ void adj_wrt_f_cols(const float* __restrict__ wx, const float* __restrict__ wy,
-                                               const T* __restrict__ v, const T* __restrict__ ux,
-                                               const T* __restrict__ uy, long long wo, long long oo, int N, int W,
-                                               int e, int gx0, int gx1, int gy, T* __restrict__ out) {
-  constexpr int CX = kStencilCols;
-  if (gy >= N) return;
-  const int oy = gy - e;
-  auto w_at = [&](const float* w, const T* u, int r, int c, bool in) -> float {
-    const long long i = wo + (long long)c * W + r;
-    if constexpr (FROM_U) return in ? __fmul_rn(ldf(u, i), ldf(v, i)) : 0.f;
-    else return in ? w[i] : 0.f;
+// Every element is loaded once: a warp owns kStencilWarpRows rows and marches
+// over the columns, CX per step with every load of a step in flight; the
+// column neighbours of wx stay in registers, the row neighbours of wy come
+// from the neighbouring lanes (the first and last lane load one row more).
+// With one row per lane the march is bound by instruction issue (N = 4096:
+// 58 us FP32, the same at FP16 storage), so a lane owns a pair of rows, one
+// aligned access each, where the window's rows allow (W even, aligned
+// arrays; the pairs start at even window rows), and single rows in two
+// strips elsewhere.  N = 4096 from u and v: 62 us with blocks that loaded
+// every neighbour, 47 us (5.6 TB/s) so, FP16 38; B = 256, N = 512 from wx,
+// wy: 141 -> 108 us (6.3 TB/s).  16 columns a block: 32 and 64 measured 3 to
+// 10 % slower (fewer blocks in flight), 8 for small images.
+constexpr int kStencilThreads = 128;
+constexpr int kStencilWarpRows = 64;
+constexpr int kStencilRows = kStencilThreads / 32 * kStencilWarpRows;  // rows of a block
+constexpr int kStencilCols = 16;  // columns of a block
+// Row blocks of an image: pairs start at even window rows, one row above the
+// image for odd erosion.
+__host__ __device__ inline int stencil_row_blocks(int N, int e) { return (N + (e & 1) + kStencilRows - 1) / kStencilRows; }
+
+template <bool PAIR>
+struct StencilVal;  // a lane's value(s): one float or a packed pair
+template <>
+struct StencilVal<false> {
+  using V = float;
+  template <typename T>
+  static __device__ __forceinline__ V load(const T* p, bool on) { return ldp(p, on); }
+  static __device__ __forceinline__ V mul(V a, V b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return __fsub_rn(a, b); }
+  static __device__ __forceinline__ V add(V a, V b) { return __fadd_rn(a, b); }
+  static __device__ __forceinline__ V half() { return 0.5f; }
+  // rows above and below, h: the edge lanes' halo value
+  static __device__ __forceinline__ void neighbours(V y, float h, int lane, V& up, V& dn) {
+    up = __shfl_up_sync(0xffffffffu, y, 1);
+    dn = __shfl_down_sync(0xffffffffu, y, 1);
+    if (lane == 0) up = h;
+    if (lane == 31) dn = h;
+  }
+};
+template <>
+struct StencilVal<true> {
+  using V = pk;
+  template <typename T>
+  static __device__ __forceinline__ V load(const T* p, bool on) { return ld2<true>(p, 0, on, on); }
+  static __device__ __forceinline__ V mul(V a, V b) { return pk_mul(a, b); }
+  static __device__ __forceinline__ V sub(V a, V b) { return pk_sub(a, b); }
+  static __device__ __forceinline__ V add(V a, V b) { return pk_add(a, b); }
+  static __device__ __forceinline__ V half() { return pk_dup(0.5f); }
+  static __device__ __forceinline__ void neighbours(V y, float h, int lane, V& up, V& dn) {
+    float u = __shfl_up_sync(0xffffffffu, pk_hi(y), 1), d = __shfl_down_sync(0xffffffffu, pk_lo(y), 1);
+    if (lane == 0) u = h;
+    if (lane == 31) d = h;
+    up = pk_make(u, pk_lo(y));
+    dn = pk_make(pk_hi(y), d);
+  }
+};
+
+// Columns [gx0, gx1) of the lane's row gy (PAIR: rows gy, gy + 1).
+template <typename T, bool FROM_U, bool PAIR>
+__device__ __forceinline__ void adj_wrt_f_strip(const float* __restrict__ wx, const float* __restrict__ wy,
+                                                const T* __restrict__ v, const T* __restrict__ ux,
+                                                const T* __restrict__ uy, long long wo, long long oo, int N, int W,
+                                                int e, int gx0, int gx1, int gy, T* __restrict__ out) {
+  using O = StencilVal<PAIR>;
+  using V = typename O::V;
+  constexpr int CX = FROM_U ? 4 : 8;  // 8 loads a step with two arrays, 4 with three (47 us; 54 with 8)
+  const int lane = threadIdx.x & 31;
+  const int oy = gy - e;  // the lane's (first) row in the window; PAIR: even, W even
+  const int hd = lane == 0 ? -1 : PAIR ? 2 : 1;
+  const bool rin = (unsigned)oy < (unsigned)W, hin = (lane == 0 || lane == 31) && (unsigned)(oy + hd) < (unsigned)W;
+  const long long base = wo + oy;
+  int c = gx0 - e;  // window column of the first output
+  // window columns read: up to that of gx1 (a slab's arrays end there)
+  const int cend = gx1 - e;
+  auto in = [&](int k) { return (unsigned)k < (unsigned)W && k <= cend; };
+  auto load_x = [&](int k, V& vk) -> V {
+    const bool on = rin && in(k);
+    const long long i = base + (long long)k * W;
+    if constexpr (FROM_U) {
+      vk = O::load(v + i, on);
+      return O::mul(O::load(ux + i, on), vk);
+    } else {
+      return O::load(wx + i, on);
+    }
   };
-  const bool rin = (unsigned)oy < (unsigned)W;
-  const bool uin = (unsigned)(oy - 1) < (unsigned)W, din = (unsigned)(oy + 1) < (unsigned)W;
-  float wxv[CX + 2];
+  const bool o0 = (unsigned)gy < (unsigned)N, o1 = PAIR && (unsigned)(gy + 1) < (unsigned)N;
+  const bool opair = PAIR && o0 && o1 && !((N | gy) & 1) && pair_aligned(out + oo);
+  V vc{};  // v at column c (FROM_U)
+  V xm = load_x(c - 1, vc), x0 = load_x(c, vc);
+  for (int gx = gx0; gx < gx1; gx += CX, c += CX) {
+    V xn[CX], vn[CX], y[CX];
+    float h[CX];
 #pragma unroll
-  for (int j = 0; j < CX + 2; ++j) {
-    const int c = gx0 - e - 1 + j;
-    wxv[j] = w_at(wx, ux, oy, c, rin && (unsigned)c < (unsigned)W);
+    for (int j = 0; j < CX; ++j) {
+      xn[j] = load_x(c + 1 + j, vn[j]);
+      const bool cin = in(c + j) && c + j < cend;
+      const long long i = base + (long long)(c + j) * W;
+      if constexpr (FROM_U) {
+        y[j] = O::load(uy + i, rin && cin);
+        h[j] = __fmul_rn(ldp(uy + i + hd, hin && cin), ldp(v + i + hd, hin && cin));
+      } else {
+        y[j] = O::load(wy + i, rin && cin);
+        h[j] = ldp(wy + i + hd, hin && cin);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < CX; ++j) {
+      if constexpr (FROM_U) y[j] = O::mul(y[j], j ? vn[j - 1] : vc);
+      V up, dn;
+      O::neighbours(y[j], h[j], lane, up, dn);
+      const V left = j == 0 ? xm : j == 1 ? x0 : xn[j - 2];
+      const V r = O::add(O::mul(O::sub(left, xn[j]), O::half()), O::mul(O::sub(up, dn), O::half()));
+      if (gx + j < gx1) {
+        T* __restrict__ p = out + oo + (long long)(gx + j) * N + gy;
+        if constexpr (PAIR) {
+          if (opair)
+            st2<true>(p, 0, r, true, true);
+          else
+            st2<false>(p, 0, r, o0, o1);
+        } else if (o0) {
+          stf(p, 0, r);
+        }
+      }
+    }
+    xm = xn[CX - 2];
+    x0 = xn[CX - 1];
+    if constexpr (FROM_U) vc = vn[CX - 1];
   }
-  float wyu[CX], wyd[CX];
-#pragma unroll
-  for (int j = 0; j < CX; ++j) {
-    const int c = gx0 - e + j;
-    const bool cin = (unsigned)c < (unsigned)W;
-    wyu[j] = w_at(wy, uy, oy - 1, c, uin && cin);
-    wyd[j] = w_at(wy, uy, oy + 1, c, din && cin);
-  }
-#pragma unroll
-  for (int j = 0; j < CX; ++j) {
-    const int gx = gx0 + j;
-    if (gx >= gx1) break;
-    const float val = __fadd_rn(__fmul_rn(__fsub_rn(wxv[j], wxv[j + 2]), 0.5f),
-                                __fmul_rn(__fsub_rn(wyu[j], wyd[j]), 0.5f));
-    stf(out, oo + (long long)gx * N + gy, val);
+}
+// Columns [gx0, gx1) of row block rb of one image.
+template <typename T, bool FROM_U>
+__device__ __forceinline__ void adj_wrt_f_block(const float* __restrict__ wx, const float* __restrict__ wy,
+                                                const T* __restrict__ v, const T* __restrict__ ux,
+                                                const T* __restrict__ uy, long long wo, long long oo, int N, int W,
+                                                int e, int gx0, int gx1, int rb, T* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int r0 = rb * kStencilRows + (threadIdx.x >> 5) * kStencilWarpRows - (e & 1);  // the warp's first row
+  if (r0 >= N) return;
+  bool pair = !(W & 1);
+  if constexpr (FROM_U)
+    pair = pair && pair_aligned(v + wo) && pair_aligned(ux + wo) && pair_aligned(uy + wo);
+  else
+    pair = pair && pair_aligned(wx + wo) && pair_aligned(wy + wo);
+  if (pair) {
+    adj_wrt_f_strip<T, FROM_U, true>(wx, wy, v, ux, uy, wo, oo, N, W, e, gx0, gx1, r0 + 2 * lane, out);
+  } else {
+#pragma unroll 1
+    for (int s = 0; s < kStencilWarpRows; s += 32)
+      adj_wrt_f_strip<T, FROM_U, false>(wx, wy, v, ux, uy, wo, oo, N, W, e, gx0, gx1, r0 + s + lane, out);
   }
 }
 
-// Uniform batch: grid (N/32, N/(8*kStencilCols), B) of 32 x 8 blocks.
+// Uniform batch: grid (row blocks, columns / cols, B).
 template <typename T, bool FROM_U>
-__global__ void k_adj_wrt_f(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
-                            const T* __restrict__ ux, const T* __restrict__ uy, int N, int W, int e, int B,
-                            T* __restrict__ out) {
-  const int gy = blockIdx.x * blockDim.x + threadIdx.x;
-  const int gx0 = (blockIdx.y * blockDim.y + threadIdx.y) * kStencilCols;
+__global__ void __launch_bounds__(kStencilThreads)
+k_adj_wrt_f(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
+            const T* __restrict__ ux, const T* __restrict__ uy, int N, int W, int e, int cols, T* __restrict__ out) {
+  const int gx0 = blockIdx.y * cols;
   const int b = blockIdx.z;
-  adj_wrt_f_cols<T, FROM_U>(wx, wy, v, ux, uy, (long long)b * W * W, (long long)b * N * N, N, W, e, gx0, N, gy,
-                            out);
+  adj_wrt_f_block<T, FROM_U>(wx, wy, v, ux, uy, (long long)b * W * W, (long long)b * N * N, N, W, e, gx0,
+                             min(gx0 + cols, N), blockIdx.x, out);
 }
 
-// The same for a ragged batch or a column slab: 32 x 8 blocks over the
-// pixel columns [cx0, cx1) of each image, the blocks of image b starting at
-// rimg[b].blk0.
+// The same for a ragged batch or a column slab over the pixel columns
+// [cx0, cx1) of each image, the blocks of image b starting at rimg[b].blk0.
 template <typename T, bool FROM_U>
-__global__ void k_adj_wrt_f_rag(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
-                                const T* __restrict__ ux, const T* __restrict__ uy,
-                                const RagImage* __restrict__ rimg, int B, int e, T* __restrict__ out) {
+__global__ void __launch_bounds__(kStencilThreads)
+k_adj_wrt_f_rag(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
+                const T* __restrict__ ux, const T* __restrict__ uy, const RagImage* __restrict__ rimg, int B, int e,
+                T* __restrict__ out) {
   int lo = 0, hi = B - 1;
   const int blk = blockIdx.x;
   while (lo < hi) {
@@ -1327,11 +1481,11 @@ __global__ void k_adj_wrt_f_rag(const float* __restrict__ wx, const float* __res
     if (rimg[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
   }
   const RagImage im = rimg[lo];
-  const int nby = (im.N + 31) / 32;
+  const int nby = stencil_row_blocks(im.N, e);
   const int k = blk - im.blk0;
-  const int gy = (k % nby) * 32 + threadIdx.x;
-  const int gx0 = im.cx0 + ((k / nby) * 8 + threadIdx.y) * kStencilCols;
-  adj_wrt_f_cols<T, FROM_U>(wx, wy, v, ux, uy, im.ow, im.on, im.N, im.W, e, gx0, im.cx1, gy, out);
+  const int gx0 = im.cx0 + (k / nby) * kStencilCols;
+  adj_wrt_f_block<T, FROM_U>(wx, wy, v, ux, uy, im.ow, im.on, im.N, im.W, e, gx0, min(gx0 + kStencilCols, im.cx1),
+                             k % nby, out);
 }
 
 }  // namespace srk

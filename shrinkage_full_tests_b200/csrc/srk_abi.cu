@@ -124,13 +124,15 @@ srk_status ensure_wbuf(srk_plan_s* p, size_t bytes, cudaStream_t) {
 template <typename T>
 void adj_wrt_f_t(srk_plan_s* p, const float* wx, const float* wy, const void* v, const void* ux, const void* uy, int B,
                  void* out, cudaStream_t s) {
-  const dim3 blk(32, 8);
-  const dim3 grd((p->N + 31) / 32, (p->N + 8 * kStencilCols - 1) / (8 * kStencilCols), B);
+  const int nby = stencil_row_blocks(p->N, p->e);
+  // a small image: shorter marches on more SMs
+  const int cols = (long long)nby * (p->N / kStencilCols) * B >= 8ll * std::max(p->nsm, 1) ? kStencilCols : 8;
+  const dim3 grd(nby, (p->N + cols - 1) / cols, B), blk(kStencilThreads);
   if (ux)
     k_adj_wrt_f<T, true><<<grd, blk, 0, s>>>(nullptr, nullptr, static_cast<const T*>(v), static_cast<const T*>(ux),
-                                             static_cast<const T*>(uy), p->N, p->W, p->e, B, static_cast<T*>(out));
+                                             static_cast<const T*>(uy), p->N, p->W, p->e, cols, static_cast<T*>(out));
   else
-    k_adj_wrt_f<T, false><<<grd, blk, 0, s>>>(wx, wy, nullptr, nullptr, nullptr, p->N, p->W, p->e, B,
+    k_adj_wrt_f<T, false><<<grd, blk, 0, s>>>(wx, wy, nullptr, nullptr, nullptr, p->N, p->W, p->e, cols,
                                               static_cast<T*>(out));
 }
 
@@ -902,6 +904,11 @@ srk_status upload_tables(srk_plan_s* p, std::vector<int> key, std::vector<int4> 
 }
 
 
+// Blocks of the ragged stencil launch over the pixel columns [c0, c1) of an image.
+long long stencil_blocks(int N, int e, int c0, int c1) {
+  return (long long)stencil_row_blocks(N, e) * ((c1 - c0 + kStencilCols - 1) / kStencilCols);
+}
+
 // B images of sizes Ns[b] (each 2*erosion+1 <= N_b <= the plan's N; same
 // erosion, dx, tile size and spectra), concatenated column-major in every
 // buffer: N-sized arrays hold N_b^2 elements per image, W-sized ones W_b^2.
@@ -932,7 +939,7 @@ srk_status ragged_tables(srk_plan_s* p, int B, const int* Ns, cudaStream_t s) {
     imgs[b].pad = 0;
     on += (long long)N * N;
     ow += (long long)W * W;
-    blk += (long long)((N + 31) / 32) * ((N + 8 * kStencilCols - 1) / (8 * kStencilCols));
+    blk += stencil_blocks(N, e, 0, N);
     const int Tf = (W + S - 1) / S, Ta = (N + S - 1) / S;
     for (int tx = 0; tx < Tf; ++tx)
       for (int ty = 0; ty < Tf; ++ty) fwd.push_back(make_int4(b, tx * S, ty * S, 0));
@@ -974,7 +981,7 @@ srk_status slab_tables(srk_plan_s* p, int N, int c0, int c1, bool adj, cudaStrea
   imgs[0].cx0 = adj ? c0 : 0;
   imgs[0].cx1 = adj ? c1 : 0;
   imgs[0].pad = 0;
-  const int nblk = adj ? ((N + 31) / 32) * ((c1 - c0 + 8 * kStencilCols - 1) / (8 * kStencilCols)) : 0;
+  const int nblk = adj ? (int)stencil_blocks(N, e, c0, c1) : 0;
   std::vector<int4> none;
   return adj ? upload_tables(p, std::move(key), std::move(none), tiles, imgs, nblk, 0, 0, s)
              : upload_tables(p, std::move(key), std::move(tiles), none, imgs, nblk, 0, 0, s);
@@ -1014,7 +1021,7 @@ srk_status slab_tables_ta(srk_plan_s* p, int N, int c0, int c1, int* r0o, int* r
   imgs[0].cx0 = c0;
   imgs[0].cx1 = c1;
   imgs[0].pad = 0;
-  const int nblk = ((N + 31) / 32) * ((c1 - c0 + 8 * kStencilCols - 1) / (8 * kStencilCols));
+  const int nblk = (int)stencil_blocks(N, e, c0, c1);
   return upload_tables(p, std::move(key), std::move(fwd), adj, imgs, nblk, 0, 0, s);
 }
 
@@ -1029,7 +1036,7 @@ Geom ragged_geom(const srk_plan_s* p, bool adj) {
 template <typename T>
 void adj_wrt_f_rag_t(srk_plan_s* p, const float* wx, const float* wy, const void* v, const void* ux, const void* uy,
                      int B, void* out, cudaStream_t s) {
-  const dim3 blk(32, 8);
+  const int blk = kStencilThreads;
   if (ux)
     k_adj_wrt_f_rag<T, true><<<p->rag_nblk, blk, 0, s>>>(nullptr, nullptr, static_cast<const T*>(v),
                                                          static_cast<const T*>(ux), static_cast<const T*>(uy),
