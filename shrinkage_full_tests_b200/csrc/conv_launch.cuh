@@ -189,20 +189,22 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
   auto launch3 = [&](int w0, int c, float2* base, cudaStream_t s1, cudaStream_t s2, cudaStream_t s3,
                      cudaEvent_t e1, cudaEvent_t e2) -> srk_status {
     const dim3 g1(M / unit_lines<M>(), c);
+    const bool chain = !e1;  // one stream: programmatic dependent launches
     if (tan)
-      k_p1<M, OP, T, kAdj><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base);
+      SRK_TRY(launch(k_p1<M, OP, T, kAdj>, g1, kThreads, sm1, s1, chain, a, g, p->tw, w0, base));
     else
-      k_p1<M, OP, T><<<g1, kThreads, sm1, s1>>>(a, g, p->tw, w0, base);
+      SRK_TRY(launch(k_p1<M, OP, T>, g1, kThreads, sm1, s1, chain, a, g, p->tw, w0, base));
     if (e1) {
       SRK_CUDA(cudaEventRecord(e1, s1));
       SRK_CUDA(cudaStreamWaitEvent(s2, e1, 0));
     }
-    k_p2<M, OP><<<dim3(M / unit_lines<M>(), c), kThreads, sm2, s2>>>(base, p->G[0], p->G[1], conjG ? 1 : 0, g, p->tw);
+    SRK_TRY(launch(k_p2<M, OP>, dim3(M / unit_lines<M>(), c), kThreads, sm2, s2, chain, base, p->G[0], p->G[1],
+                   conjG ? 1 : 0, g, p->tw));
     if (e2) {
       SRK_CUDA(cudaEventRecord(e2, s2));
       SRK_CUDA(cudaStreamWaitEvent(s3, e2, 0));
     }
-    k_p3<M, OP, T><<<dim3(n3, c), kThreads, sm3, s3>>>(base, a, g, p->tw, w0);
+    SRK_TRY(launch(k_p3<M, OP, T>, dim3(n3, c), kThreads, sm3, s3, chain, base, a, g, p->tw, w0));
     return SRK_OK;
   };
   const int whole = (int)std::min<size_t>(std::max<size_t>(cap, 1), 65535);

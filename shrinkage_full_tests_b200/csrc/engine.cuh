@@ -504,29 +504,55 @@ struct Window {
   bool sync;   // elements written by the threads
 };
 
-// Rows [at, end) of the nc columns from gx0 in asynchronous pieces of BYTES (2:
-// plain copies of single values), each wholly inside or outside the image.
+// Elements [0, n) of the nc columns that bulk copies or window_pieces do not
+// write (outside the image): zero.  Columns c0 .. c1 - 1, elements r0 .. r1 - 1
+// lie in the image.  Returns whether there are any.
+template <int M, typename T>
+__device__ __forceinline__ bool window_zero(int nc, int n, int c0, int c1, int r0, int r1, int HP, T* __restrict__ win) {
+  constexpr int GT = Quad<M>::GT;
+  const int t = threadIdx.x % GT;
+  if (c1 - c0 == nc && r1 - r0 == n) return false;
+  for (int c = 0; c < nc; ++c) {
+    const bool in = c >= c0 && c < c1;
+    for (int k = t; k < n; k += GT)
+      if (!in || k < r0 || k >= r1) win[c * HP + k] = T(0.f);
+  }
+  return true;
+}
+
+// Columns [c0, c1) and elements [r0, r1) (whole pieces) of a window in
+// asynchronous pieces of BYTES; 2: single values through registers, a batch
+// of loads in flight.
 template <int M, typename T, int BYTES>
-__device__ __forceinline__ void window_pieces(const T* __restrict__ img, int N, int gx0, int nc, int at, int end, int HP,
+__device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, int c0, int c1, int r0, int r1, int HP,
                                               T* __restrict__ win) {
   constexpr int E = BYTES / (int)sizeof(T) ? BYTES / (int)sizeof(T) : 1;
   constexpr int GT = Quad<M>::GT;
   const int t = threadIdx.x % GT;
+  if constexpr (BYTES > 2) {
 #pragma unroll 1
-  for (int c = 0; c < nc; ++c) {
-    const int gx = gx0 + c;
-    const bool colin = gx >= 0 && gx < N;
-    const T* col = img + (long long)(colin ? gx : 0) * N + at;
-    T* d = win + c * HP;
-    for (int k = E * t; k < end - at; k += E * GT) {
-      const bool in = colin && (unsigned)(at + k) < (unsigned)N;
-      if constexpr (BYTES > 2)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;\n" ::"r"(
-                         static_cast<unsigned>(__cvta_generic_to_shared(d + k))),
-                     "l"(in ? col + k : img), "r"(in ? BYTES : 0), "n"(BYTES)
-                     : "memory");
-      else
-        d[k] = in ? col[k] : T(0.f);
+    for (int c = c0; c < c1; ++c) {
+      const T* p = src + (long long)c * N + r0 + E * t;
+      unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(win + c * HP + r0 + E * t));
+#pragma unroll 4
+      for (int k = r0 + E * t; k < r1; k += E * GT, p += E * GT, d += BYTES * GT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(p), "n"(BYTES) : "memory");
+    }
+  } else {
+    constexpr int KS = 3;  // rows per batch and column: kWinCols KS loads in flight
+#pragma unroll 1
+    for (int k = r0 + t; k < r1; k += KS * GT) {
+      T v[kWinCols][KS];
+#pragma unroll
+      for (int c = 0; c < kWinCols; ++c)
+#pragma unroll
+        for (int s = 0; s < KS; ++s)
+          if (c >= c0 && c < c1 && k + s * GT < r1) v[c][s] = src[(long long)c * N + k + s * GT];
+#pragma unroll
+      for (int c = 0; c < kWinCols; ++c)
+#pragma unroll
+        for (int s = 0; s < KS; ++s)
+          if (c >= c0 && c < c1 && k + s * GT < r1) win[c * HP + k + s * GT] = v[c][s];
     }
   }
 }
@@ -546,36 +572,32 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   constexpr int GT = Quad<M>::GT;
   static_assert(kWinCols <= GT, "one thread per column");
   const int t = threadIdx.x % GT;
+  const int mis = (int)(reinterpret_cast<uintptr_t>(img) & 15) | (N * (int)sizeof(T));  // alignment of every column
+  const int bytes = !(mis & 15) ? 16 : !(mis & 7) ? 8 : !(mis & 3) ? 4 : 2;              // the piece that it allows
+  const int E = max(bytes / (int)sizeof(T), 1);
   Window w;
-  w.bulk = live && N % EPC == 0 && (reinterpret_cast<uintptr_t>(img) & 15) == 0;
-  w.at = gy0 & (w.bulk ? -EPC : -2);
-  w.sync = live;
+  w.bulk = live && bytes == 16;
+  w.at = gy0 & -max(E, 2);
+  w.sync = live && !w.bulk;
   if (!live) return w;  // (nothing reads the window of a dead tile)
+  // whole pieces; elements r0 .. r1 - 1 and columns c0 .. c1 - 1 lie in the image
+  const int n = (gy0 - w.at + nr + E - 1) & -E;
+  const int r0 = max(0, -w.at), r1 = max(r0, min(n, N - w.at));
+  const int c0 = min(nc, max(0, -gx0)), c1 = max(c0, min(nc, N - gx0));
+  const T* src = img + (long long)gx0 * N + w.at;  // (dereferenced inside the image only)
   if (w.bulk) {
-    // rows wanted: whole chunks; r0 .. r1 of them and columns c0 .. c1 - 1 lie in the image
-    const int n = (gy0 - w.at + nr + EPC - 1) & -EPC;
-    const int r0 = max(0, -w.at), r1 = max(r0, min(n, N - w.at));
-    const int c0 = min(nc, max(0, -gx0)), c1 = max(c0, min(nc, N - gx0));
-    const unsigned bytes = (unsigned)((r1 - r0) * sizeof(T));
-    if (t == 0) tc::mbar_expect_tx(gm.bar + i, (unsigned)(c1 - c0) * bytes);
+    const unsigned len = (unsigned)((r1 - r0) * sizeof(T));
+    if (t == 0) tc::mbar_expect_tx(gm.bar + i, (unsigned)(c1 - c0) * len);
     __syncwarp();
-    if (t >= c0 && t < c1 && bytes)
-      tc::bulk_g2s(win + t * HP + r0, img + (long long)(gx0 + t) * N + w.at + r0, bytes, gm.bar + i);
-    w.sync = c1 - c0 < nc || r1 - r0 < n;
-    if (w.sync)
-      for (int c = 0; c < nc; ++c) {
-        const bool in = c >= c0 && c < c1;
-        for (int k = t; k < n; k += GT)
-          if (!in || k < r0 || k >= r1) win[c * HP + k] = T(0.f);
-      }
-  } else if ((N * (int)sizeof(T)) % 8 == 0 && (reinterpret_cast<uintptr_t>(img) & 7) == 0) {
-    window_pieces<M, T, 8>(img, N, gx0, nc, w.at & (sizeof(T) == 4 ? -2 : -4), gy0 + nr, HP, win);
-    w.at &= sizeof(T) == 4 ? -2 : -4;
-  } else if ((N * (int)sizeof(T)) % 4 == 0 && (reinterpret_cast<uintptr_t>(img) & 3) == 0) {
-    window_pieces<M, T, 4>(img, N, gx0, nc, w.at, gy0 + nr, HP, win);
+    if (t >= c0 && t < c1 && len) tc::bulk_g2s(win + t * HP + r0, src + (long long)t * N + r0, len, gm.bar + i);
+  } else if (bytes == 8) {
+    window_pieces<M, T, 8>(src, N, c0, c1, r0, r1, HP, win);
+  } else if (bytes == 4) {
+    window_pieces<M, T, 4>(src, N, c0, c1, r0, r1, HP, win);
   } else {
-    window_pieces<M, T, 2>(img, N, gx0, nc, w.at, gy0 + nr, HP, win);
+    window_pieces<M, T, 2>(src, N, c0, c1, r0, r1, HP, win);
   }
+  w.sync |= window_zero<M, T>(nc, n, c0, c1, r0, r1, HP, win);
   return w;
 }
 // The window has arrived for every thread of the group (group-uniform).
@@ -797,10 +819,13 @@ __device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, in
 // ---- P2 ------------------------------------------------------------------------------------
 // P2: rows ky = 4 blk .. 4 blk + 3: FFT along x, spectral map, inverse, keep
 // the valid columns.
-template <int M, int OP>
+// The spectra are older than the pass before: ready() is called between their
+// fetch and that of S1.
+template <int M, int OP, typename F>
 __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __restrict__ S2,
                                        const float4* __restrict__ Gx, const float4* __restrict__ Gy, int conjG,
-                                       const Geom& g, int blk, GroupMem<M>& gm, const float4* __restrict__ tw) {
+                                       const Geom& g, int blk, GroupMem<M>& gm, const float4* __restrict__ tw,
+                                       F&& ready) {
   using Q = Quad<M>;
   constexpr int K = OpTraits<OP>::K;
   constexpr unsigned BB = (unsigned)block_bytes<M>();
@@ -836,9 +861,10 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
   float2 X[Q::VPT];
   cpk z[Q::R], b[Q::R];
   gm.open();
+  gm.fetch(1, gm.buf, Gx + row / 2, BB);
+  ready();
   gm.fetch(0, gm.ex, S1 + row, BB);
   if constexpr (K == 1) {
-    gm.fetch(1, gm.buf, Gx + row / 2, BB);
     gm.wait(0);
     load(gm.ex, X);
     fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
@@ -856,7 +882,6 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
     fft_dit<M, true>(b, X, gm.ex, tw, t);
     emit(X, 1);
   } else {
-    gm.fetch(1, gm.buf, Gx + row / 2, BB);
     gm.wait(0);
     load(gm.ex, X);
     fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
@@ -1126,6 +1151,16 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
 }
 
 // ---- three-launch schedule (one kernel per phase over a chunk of WTs) ------
+// The kernels of one call run back to back on one stream by programmatic
+// dependent launch: a kernel's blocks are placed while the last blocks of the
+// one before finish, set up their barriers and wait there (grid_wait: every
+// kernel before is complete and visible).  Every kernel waits before it lets
+// the next one start (grid_next), so at most two kernels overlap and what a
+// kernel does before its wait may use anything older than its predecessor.
+// A no-op where the launch is an ordinary one.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Index of this thread's group in its block.
 template <int M>
 __device__ __forceinline__ int group_index() { return threadIdx.x / Quad<M>::GT; }
@@ -1138,6 +1173,8 @@ k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict
   extern __shared__ __align__(16) unsigned char sm[];
   GroupMem<M> gm = group_mem<M, p1_buf<OP>()>(sm, g.err);
   const int wl = blockIdx.y;
+  grid_wait();
+  grid_next();
   phase1<M, OP, T, TAN>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
                         scratch + wl * wt_elems<M, OP>(g.S), gm, tw);
 }
@@ -1150,7 +1187,10 @@ k_p2(float2* __restrict__ scratch, const float4* __restrict__ Gx, const float4* 
   GroupMem<M> gm = group_mem<M, true>(sm, g.err);
   float2* base = scratch + blockIdx.y * wt_elems<M, OP>(g.S);
   phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blockIdx.x * groups_of<M>() + group_index<M>(), gm,
-                tw);
+                tw, [] {
+                  grid_wait();
+                  grid_next();
+                });
 }
 
 template <int M, int OP, typename T, int S2L = kS2Engine>
@@ -1161,6 +1201,8 @@ k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ 
   const int wl = blockIdx.y;
   const int nblk = s2_blocks(g.S, S2L == kS2Rotated ? 0 : g.e - s2_first(g.e));
   const int blk = blockIdx.x * groups_of<M>() + group_index<M>();
+  grid_wait();
+  grid_next();
   if (blk < nblk)
     phase3<M, OP, T, S2L>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blk, gm, tw);
 }
@@ -1274,7 +1316,7 @@ k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restr
         else
           phase1<M, OP, T>(a, g, w, blk, base, gm, tw);
       } else if (phase == 2) {
-        phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blk, gm, tw);
+        phase2<M, OP>(base, base + s1_elems<M, OP>(), Gx, Gy, conjG, g, blk, gm, tw, [] {});
       } else if (blk < nblk) {
         phase3<M, OP, T>(base + s1_elems<M, OP>(), a, g, w, blk, gm, tw);
       }
@@ -1463,6 +1505,8 @@ k_adj_wrt_f(const float* __restrict__ wx, const float* __restrict__ wy, const T*
             const T* __restrict__ ux, const T* __restrict__ uy, int N, int W, int e, int cols, T* __restrict__ out) {
   const int gx0 = blockIdx.y * cols;
   const int b = blockIdx.z;
+  grid_wait();
+  grid_next();
   adj_wrt_f_block<T, FROM_U>(wx, wy, v, ux, uy, (long long)b * W * W, (long long)b * N * N, N, W, e, gx0,
                              min(gx0 + cols, N), blockIdx.x, out);
 }
@@ -1474,6 +1518,8 @@ __global__ void __launch_bounds__(kStencilThreads)
 k_adj_wrt_f_rag(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
                 const T* __restrict__ ux, const T* __restrict__ uy, const RagImage* __restrict__ rimg, int B, int e,
                 T* __restrict__ out) {
+  grid_wait();
+  grid_next();
   int lo = 0, hi = B - 1;
   const int blk = blockIdx.x;
   while (lo < hi) {

@@ -55,6 +55,23 @@ inline srk_status cuda_status(cudaError_t e, const char* what) {
   } while (0)
 #define SRK_CUDA(expr) SRK_TRY(cuda_status((expr), #expr))
 
+// Launch as a programmatic dependent of the kernel before it on the stream
+// (`chain`; see grid_wait in engine.cuh), or an ordinary launch.
+template <typename... P, typename... A>
+srk_status launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool chain, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = chain ? 1 : 0;
+  return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "kernel launch");
+}
+
 }  // namespace srk
 
 #ifndef SRK_RING

@@ -39,19 +39,27 @@ struct NvtxRange {
 namespace {
 
 // ---- tile choice -------------------------------------------------------------
-// FFT work per image ~ T^2 * M^2 * log2(M) for the forward geometry; choose
-// the cheapest M whose valid stride S = M - 2e keeps at least 16 outputs.
-int choose_tile(int N, int W, int e) {
-  const int cand[3] = {128, 256, 512};
+// Time of a forward call in microseconds, fitted to the engine on a B200:
+//   launch(M) + B T^2 M^2 7.2e-6 (0.35 + 0.65 S / M).
+// The second term is the throughput limit (the passes cost the same per point
+// of a tile at every M; the row pass's stores and the last pass only touch the
+// S valid columns): B=300 N=256 KW=31 measures 270 / 141 / 594 us at M = 128 /
+// 256 / 512, B=64 N=333 KW=31 119 / 148 / 158, B=100 N=512 KW=31 240 / 422 /
+// 191.  The first is the latency of the three dependent kernels when the
+// tiles do not fill the device: shorter for small tiles, whose lines have
+// fewer values per thread (N=1024 KW=31 B=1: 22 / 35 / 36 us; N=256 KW=31
+// B=1: 15.1 / 15.7 / 21.7, its adjoint 18 / 23 / 24).
+// The valid stride S = M - 2e keeps at least 16 outputs.
+int choose_tile(int N, int W, int e, int B) {
   int best = 0;
   double best_cost = 0;
-  for (int M : cand) {
+  for (int M : {128, 256, 512}) {
     const int S = M - 2 * e;
     if (S < 16) continue;
     const int T = (W + S - 1) / S;
-    const double lg = std::log2((double)M);
-    const double cost = (double)T * T * M * M * lg;
-    if (best == 0 || cost < best_cost * 0.98) { best = M; best_cost = cost; }
+    const double launch = M == 128 ? 14.5 : M == 256 ? (T == 1 ? 15.5 : 20.0) : 21.0;
+    const double cost = launch + (double)B * T * T * M * M * 7.2e-6 * (0.35 + 0.65 * S / M);
+    if (best == 0 || cost < best_cost) { best = M; best_cost = cost; }
   }
   return best;
 }
@@ -122,28 +130,25 @@ srk_status ensure_wbuf(srk_plan_s* p, size_t bytes, cudaStream_t) {
 }
 
 template <typename T>
-void adj_wrt_f_t(srk_plan_s* p, const float* wx, const float* wy, const void* v, const void* ux, const void* uy, int B,
-                 void* out, cudaStream_t s) {
+srk_status adj_wrt_f_t(srk_plan_s* p, const float* wx, const float* wy, const void* v, const void* ux, const void* uy,
+                       int B, void* out, cudaStream_t s) {
   const int nby = stencil_row_blocks(p->N, p->e);
   // a small image: shorter marches on more SMs
   const int cols = (long long)nby * (p->N / kStencilCols) * B >= 8ll * std::max(p->nsm, 1) ? kStencilCols : 8;
-  const dim3 grd(nby, (p->N + cols - 1) / cols, B), blk(kStencilThreads);
-  if (ux)
-    k_adj_wrt_f<T, true><<<grd, blk, 0, s>>>(nullptr, nullptr, static_cast<const T*>(v), static_cast<const T*>(ux),
-                                             static_cast<const T*>(uy), p->N, p->W, p->e, cols, static_cast<T*>(out));
-  else
-    k_adj_wrt_f<T, false><<<grd, blk, 0, s>>>(wx, wy, nullptr, nullptr, nullptr, p->N, p->W, p->e, cols,
-                                              static_cast<T*>(out));
+  const dim3 grd(nby, (p->N + cols - 1) / cols, B);
+  const T *tv = static_cast<const T*>(v), *tx = static_cast<const T*>(ux), *ty = static_cast<const T*>(uy);
+  return launch(ux ? k_adj_wrt_f<T, true> : k_adj_wrt_f<T, false>, grd, kStencilThreads, 0, s, true, wx, wy, tv, tx, ty,
+                p->N, p->W, p->e, cols, static_cast<T*>(out));
 }
 
 srk_status adj_wrt_f(srk_plan_s* p, const float* wx, const float* wy, const void* v, const void* ux,
                      const void* uy, int B, void* out, cudaStream_t s) {
   switch (p->dtype) {
-    case SRK_F32: adj_wrt_f_t<float>(p, wx, wy, v, ux, uy, B, out, s); break;
-    case SRK_F16: adj_wrt_f_t<__half>(p, wx, wy, v, ux, uy, B, out, s); break;
-    case SRK_BF16: adj_wrt_f_t<__nv_bfloat16>(p, wx, wy, v, ux, uy, B, out, s); break;
+    case SRK_F32: return adj_wrt_f_t<float>(p, wx, wy, v, ux, uy, B, out, s);
+    case SRK_F16: return adj_wrt_f_t<__half>(p, wx, wy, v, ux, uy, B, out, s);
+    case SRK_BF16: return adj_wrt_f_t<__nv_bfloat16>(p, wx, wy, v, ux, uy, B, out, s);
   }
-  return cuda_status(cudaGetLastError(), "adj_wrt_f launch");
+  return fail(SRK_ERR_UNSUPPORTED, "dtype %d", (int)p->dtype);
 }
 
 // ---- spectra -----------------------------------------------------------------------
@@ -383,7 +388,7 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
     const srk_status st = srk_autotune(N, W, erosion, dx, B_max, dtype, &M, &sched);
     if (st != SRK_OK) return st;
   }
-  if (M == 0) M = choose_tile(N, W, erosion);
+  if (M == 0) M = choose_tile(N, W, erosion, B_max);
   if (M == 0)
     return fail(SRK_ERR_UNSUPPORTED, "erosion=%d too large for the 512 tile (needs stride >= 16)", erosion);
   if (!(M == 128 || M == 256 || M == 512)) return fail(SRK_ERR_INVALID_ARG, "tile_M=%d not in {128,256,512}", M);
