@@ -66,6 +66,10 @@
 #ifndef SRK_P3_ADJ_MIN_BLOCKS
 #define SRK_P3_ADJ_MIN_BLOCKS 8
 #endif
+// M = 128 has half the values per thread: every pass fits 128 registers.
+#ifndef SRK_SMALL_MIN_BLOCKS
+#define SRK_SMALL_MIN_BLOCKS 8
+#endif
 
 namespace srk {
 
@@ -1168,7 +1172,7 @@ __device__ __forceinline__ int group_index() { return threadIdx.x / Quad<M>::GT;
 // TAN (adjoint-type op of the tangent-adjoint, dv and df given) is chosen by
 // the launch.
 template <int M, int OP, typename T, bool TAN = false>
-__global__ void __launch_bounds__(kThreads, OP == OP_ADJ ? SRK_P1_ADJ_MIN_BLOCKS : SRK_P1_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, OP == OP_ADJ && M > 128 ? SRK_P1_ADJ_MIN_BLOCKS : SRK_P1_MIN_BLOCKS)
 k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict__ scratch) {
   extern __shared__ __align__(16) unsigned char sm[];
   GroupMem<M> gm = group_mem<M, p1_buf<OP>()>(sm, g.err);
@@ -1180,7 +1184,7 @@ k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict
 }
 
 template <int M, int OP>
-__global__ void __launch_bounds__(kThreads, SRK_P2_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, M > 128 ? SRK_P2_MIN_BLOCKS : SRK_SMALL_MIN_BLOCKS)
 k_p2(float2* __restrict__ scratch, const float4* __restrict__ Gx, const float4* __restrict__ Gy, int conjG, Geom g,
      const float4* __restrict__ tw) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -1194,7 +1198,9 @@ k_p2(float2* __restrict__ scratch, const float4* __restrict__ Gx, const float4* 
 }
 
 template <int M, int OP, typename T, int S2L = kS2Engine>
-__global__ void __launch_bounds__(kThreads, OpTraits<OP>::L == 1 ? SRK_P3_ADJ_MIN_BLOCKS : SRK_P3_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, M == 128                ? SRK_SMALL_MIN_BLOCKS
+                                           : OpTraits<OP>::L == 1 ? SRK_P3_ADJ_MIN_BLOCKS
+                                                                  : SRK_P3_MIN_BLOCKS)
 k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ tw, int w0) {
   extern __shared__ __align__(16) unsigned char sm[];
   GroupMem<M> gm = group_mem<M, p3_buf<OP>()>(sm, g.err);
