@@ -563,7 +563,10 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 
 // Starts the copy of nc (at most the group's threads) columns from gx0 and nr
 // rows from gy0 of the N x N image at img (any of them outside the image; not
-// live: nothing) on the group's barrier i.  One bulk copy per column where
+// live: nothing) on the group's barrier i.  edge: elements outside the image
+// become zero; else they keep whatever the memory held (with erosion >= 1
+// only values that are never stored read them, and zeroing them was the
+// longest step of a tile at the image's edge).  One bulk copy per column where
 // every 16-byte chunk lies wholly inside or outside the image (N a multiple
 // of the chunk, an aligned image): a loop of 16-byte cp.async over the
 // threads cost P3 and the adjoint's P1 several hundred instructions.  Else
@@ -571,7 +574,8 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 // is past gm.open().
 template <int M, typename T>
 __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, int gy0,
-                                               int nr, int HP, T* __restrict__ win, const GroupMem<M>& gm, int i) {
+                                               int nr, int HP, T* __restrict__ win, bool edge, const GroupMem<M>& gm,
+                                               int i) {
   constexpr int EPC = 16 / (int)sizeof(T);
   constexpr int GT = Quad<M>::GT;
   static_assert(kWinCols <= GT, "one thread per column");
@@ -601,7 +605,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   } else {
     window_pieces<M, T, 2>(src, N, c0, c1, r0, r1, HP, win);
   }
-  w.sync |= window_zero<M, T>(nc, n, c0, c1, r0, r1, HP, win);
+  if (edge) w.sync |= window_zero<M, T>(nc, n, c0, c1, r0, r1, HP, win);
   return w;
 }
 // The window has arrived for every thread of the group (group-uniform).
@@ -742,7 +746,7 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
   };
   auto stage = [&](const TileRef& t, const void* img, int i) {
     return issue_window<M, T>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
-                              t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, gm, i);
+                              t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
   };
   auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
     const int ox = t.x0 + blk * kLines - 2 * a.e;
@@ -1069,10 +1073,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     if constexpr (GRAD) {
       const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
       wn[h] = issue_window<M, T>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2, HP, win[h],
-                                 gm, 1 - h);
+                                 a.e < 1, gm, 1 - h);
     } else {
       const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
-      wn[h] = issue_window<M, T>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], gm, 1 - h);
+      wn[h] = issue_window<M, T>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], false, gm,
+                                 1 - h);
     }
   };
   // column x of a staged S2 block: ky = k_i + R m
