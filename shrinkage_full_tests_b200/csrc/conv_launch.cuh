@@ -14,6 +14,39 @@ srk_status set_smem(K kernel, size_t bytes) {
   return SRK_OK;
 }
 
+// Form of a launch's images (engine.cuh) in P1 of the adjoint and in P3.  A
+// ragged batch mixes sizes and is kAny; so is erosion 0.
+template <typename T>
+bool rows16(const void* img, int n) {  // every column of the images starts on 16 bytes (no image: true)
+  return !img || ((reinterpret_cast<uintptr_t>(img) & 15) == 0 && (size_t)n * sizeof(T) % 16 == 0);
+}
+template <typename T>
+bool pairs(const void* out) { return (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(T) - 1)) == 0; }
+template <typename T>
+int p1_adj_form(const OpArgs& a, const Geom& g) {
+  if (g.rtile || a.e < 1 || !rows16<T>(a.I, g.N) || !rows16<T>(a.dI, g.N) || (g.TT > 1 && (g.S & 1))) return kAny;
+  return ((g.TT == 1 ? g.org : 0) - a.e) & 1 ? kOdd : kEven;
+}
+template <int OP, typename T>
+int p3_form(const OpArgs& a, const Geom& g) {
+  if (g.rtile || (g.TT > 1 && (g.S & 1)) || (((g.TT == 1 ? g.org : 0) + g.e - a.e) & 1)) return kAny;  // first output row
+  const bool even = !((g.e | g.Wout) & 1);
+  if constexpr (OpTraits<OP>::L == 1) {
+    return even && pairs<T>(a.out0) ? kEven : kAny;
+  } else {
+    if (a.e < 1 || g.e != a.e) return kAny;
+    bool out;
+    if constexpr (grad_op<OP>()) {
+      if (!rows16<T>(a.I, g.N) || (OP == OP_JVP && !rows16<T>(a.dI, g.N))) return kAny;
+      out = pairs<T>(a.out0) && pairs<T>(a.out_ux) && pairs<T>(a.out_uy);
+    } else {
+      if (!rows16<T>(a.v, g.W) || (OP == OP_TANADJ_F && !rows16<T>(a.dv, g.W))) return kAny;
+      out = pairs<float>(a.out0) && pairs<float>(a.out1);
+    }
+    return g.e & 1 ? kOdd : even && out ? kEven : kAny;
+  }
+}
+
 // Three-pass schedule with the tensor-core row pass (SRK_SCHEDULE_TENSOR_ROWS):
 // per chunk the column pass (-> FP16 planes, with each work tile's largest
 // |Z|: the column DFT on the tensor cores, k_p1g, where its TMA boxes apply,
@@ -30,7 +63,11 @@ srk_status launch_tensor_rows(srk_plan_s* p, const OpArgs& a, const Geom& g, int
   const size_t smp1 = p1h_smem_bytes();
   constexpr size_t sm3 = p3_smem_bytes<M, OP>();
   SRK_TRY(set_smem(k_p1h<OP, T>, smp1));
-  SRK_TRY(set_smem(k_p3<M, OP, T, kS2Rotated>, sm3));
+  static_assert(sm3 <= 48 * 1024, "no shared-memory opt-in needed");
+  const int form = p3_form<OP, T>(a, g);
+  auto kp3 = form == kEven  ? k_p3<M, OP, T, kS2Rotated, kEven>
+             : form == kOdd ? k_p3<M, OP, T, kS2Rotated, kOdd>
+                            : k_p3<M, OP, T, kS2Rotated>;
   SRK_TRY(set_smem(k_p1h_refit<OP, T>, smp1));
   static_assert(OpTraits<OP>::PAIRS, "the tensor-row schedule serves the pair ops");
   // k_p1g (column DFT on the tensor cores): a uniform batch, N % 8 == 0
@@ -75,7 +112,7 @@ srk_status launch_tensor_rows(srk_plan_s* p, const OpArgs& a, const Geom& g, int
     return SRK_OK;
   };
   auto p3 = [&](int w0, int c, float2* base, cudaStream_t st) {
-    k_p3<M, OP, T, kS2Rotated><<<dim3(s2_blocks(g.S, 0), c), kThreads, sm3, st>>>(base, a, g, p->tw, w0);
+    kp3<<<dim3(s2_blocks(g.S, 0), c), kThreads, sm3, st>>>(base, a, g, p->tw, w0);
   };
   const int whole = (int)std::min<size_t>(std::max<size_t>(cap, 1), 65535);
   int launches = 0;
@@ -186,14 +223,23 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
   const bool tan = OP == OP_ADJ && a.dI != nullptr;  // the tangent-adjoint's adjoint-type pass
   constexpr bool kAdj = OP == OP_ADJ;
   static_assert(sm1 <= 48 * 1024 && sm2 <= 48 * 1024 && sm3 <= 48 * 1024, "no shared-memory opt-in needed");
+  auto kp1 = k_p1<M, OP, T>;
+  if constexpr (kAdj) {
+    switch (p1_adj_form<T>(a, g)) {
+      case kEven: kp1 = tan ? k_p1<M, OP, T, true, kEven> : k_p1<M, OP, T, false, kEven>; break;
+      case kOdd: kp1 = tan ? k_p1<M, OP, T, true, kOdd> : k_p1<M, OP, T, false, kOdd>; break;
+      default: kp1 = tan ? k_p1<M, OP, T, true> : k_p1<M, OP, T>;
+    }
+  }
+  const int form = p3_form<OP, T>(a, g);
+  auto kp3 = form == kEven ? k_p3<M, OP, T, kS2Engine, kEven> : k_p3<M, OP, T>;
+  if constexpr (!kAdj)
+    if (form == kOdd) kp3 = k_p3<M, OP, T, kS2Engine, kOdd>;
   auto launch3 = [&](int w0, int c, float2* base, cudaStream_t s1, cudaStream_t s2, cudaStream_t s3,
                      cudaEvent_t e1, cudaEvent_t e2) -> srk_status {
     const dim3 g1(M / unit_lines<M>(), c);
     const bool chain = !e1;  // one stream: programmatic dependent launches
-    if (tan)
-      SRK_TRY(launch(k_p1<M, OP, T, kAdj>, g1, kThreads, sm1, s1, chain, a, g, p->tw, w0, base));
-    else
-      SRK_TRY(launch(k_p1<M, OP, T>, g1, kThreads, sm1, s1, chain, a, g, p->tw, w0, base));
+    SRK_TRY(launch(kp1, g1, kThreads, sm1, s1, chain, a, g, p->tw, w0, base));
     if (e1) {
       SRK_CUDA(cudaEventRecord(e1, s1));
       SRK_CUDA(cudaStreamWaitEvent(s2, e1, 0));
@@ -204,7 +250,7 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
       SRK_CUDA(cudaEventRecord(e2, s2));
       SRK_CUDA(cudaStreamWaitEvent(s3, e2, 0));
     }
-    SRK_TRY(launch(k_p3<M, OP, T>, dim3(n3, c), kThreads, sm3, s3, chain, base, a, g, p->tw, w0));
+    SRK_TRY(launch(kp3, dim3(n3, c), kThreads, sm3, s3, chain, base, a, g, p->tw, w0));
     return SRK_OK;
   };
   const int whole = (int)std::min<size_t>(std::max<size_t>(cap, 1), 65535);

@@ -500,6 +500,16 @@ __host__ __device__ constexpr size_t win_bytes() { return (size_t)kWinCols * win
 template <int M>
 __host__ __device__ constexpr size_t win_lead() { return 2 * (size_t)M; }
 
+// What a launch knows of the images that its blocks stage: nothing, or that
+// every column starts on 16 bytes, the erosion is at least 1 and the first row
+// that a thread works on is even / odd in every tile (P3: even also means that
+// every pair of outputs is one aligned store).  The kernels of the two known
+// forms hold neither the copies in smaller pieces nor the other parity's
+// arithmetic.  The passes are short of instruction cache and registers, so
+// the paths not taken cost: P3 of 150 image pairs at M = 512 177 -> 149 us
+// (erosion 60), 241 -> 198 (15); of 600 at M = 256 179 -> 153 and 220 -> 189.
+enum Form : int { kAny = 0, kEven = 1, kOdd = 2 };
+
 // An issued window: `at` is the image row of element 0; the caller waits for
 // it with window_wait.
 struct Window {
@@ -571,8 +581,8 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 // of the chunk, an aligned image): a loop of 16-byte cp.async over the
 // threads cost P3 and the adjoint's P1 several hundred instructions.  Else
 // the threads copy the largest pieces that N and the image allow.  The group
-// is past gm.open().
-template <int M, typename T>
+// is past gm.open().  FORM: what the launch knows of the images (Form).
+template <int M, int FORM, typename T>
 __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, int gy0,
                                                int nr, int HP, T* __restrict__ win, bool edge, const GroupMem<M>& gm,
                                                int i) {
@@ -581,7 +591,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   static_assert(kWinCols <= GT, "one thread per column");
   const int t = threadIdx.x % GT;
   const int mis = (int)(reinterpret_cast<uintptr_t>(img) & 15) | (N * (int)sizeof(T));  // alignment of every column
-  const int bytes = !(mis & 15) ? 16 : !(mis & 7) ? 8 : !(mis & 3) ? 4 : 2;              // the piece that it allows
+  const int bytes = FORM != kAny || !(mis & 15) ? 16 : !(mis & 7) ? 8 : !(mis & 3) ? 4 : 2;  // the piece that it allows
   const int E = max(bytes / (int)sizeof(T), 1);
   Window w;
   w.bulk = live && bytes == 16;
@@ -598,6 +608,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
     if (t == 0) tc::mbar_expect_tx(gm.bar + i, (unsigned)(c1 - c0) * len);
     __syncwarp();
     if (t >= c0 && t < c1 && len) tc::bulk_g2s(win + t * HP + r0, src + (long long)t * N + r0, len, gm.bar + i);
+    if constexpr (FORM != kAny) return w;
   } else if (bytes == 8) {
     window_pieces<M, T, 8>(src, N, c0, c1, r0, r1, HP, win);
   } else if (bytes == 4) {
@@ -609,13 +620,13 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   return w;
 }
 // The window has arrived for every thread of the group (group-uniform).
-template <int M>
+template <int FORM, int M>
 __device__ __forceinline__ void window_wait(const Window& w, GroupMem<M>& gm, int i) {
   if (w.bulk)
     gm.wait(i);
-  else
+  else if (FORM == kAny)
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (w.sync) group_sync<M>();
+  if (FORM == kAny && w.sync) group_sync<M>();
 }
 
 // This thread's column of one tile in a W- or N-sized array: rows y = 2q + l
@@ -704,19 +715,20 @@ __device__ __forceinline__ void adj_fields(const pk (&vv)[Quad<M>::R], const pk 
     (LANE ? hy[r].im : hy[r].re) = gy;
   }
 }
-template <int M, typename T, bool TAN, int LANE>
+template <int M, typename T, bool TAN, int LANE, int FORM>
 __device__ __forceinline__ void adj_lane(const GroupMem<M>& gm, bool cols, const pk (&vv)[Quad<M>::R],
                                          const pk (&dv)[Quad<M>::R], const OutCol& o,
                                          const T* __restrict__ wf, const T* __restrict__ wd, int row,
                                          cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
   const int y0 = o.rel - 2 * gm.t.q;  // first tile row in the valid window (group-uniform, like `inside`)
   const bool inside = cols && y0 >= 0 && y0 + M <= (int)o.cnt;
+  const bool odd = FORM == kAny ? row & 1 : FORM == kOdd;
   if (!inside) {
-    if (row & 1)
+    if (odd)
       adj_fields<M, T, TAN, LANE, true, true>(vv, dv, o, wf, wd, row, hx, hy);
     else
       adj_fields<M, T, TAN, LANE, false, true>(vv, dv, o, wf, wd, row, hx, hy);
-  } else if (row & 1) {
+  } else if (odd) {
     adj_fields<M, T, TAN, LANE, true, false>(vv, dv, o, wf, wd, row, hx, hy);
   } else {
     adj_fields<M, T, TAN, LANE, false, false>(vv, dv, o, wf, wd, row, hx, hy);
@@ -726,7 +738,7 @@ __device__ __forceinline__ void adj_lane(const GroupMem<M>& gm, bool cols, const
 // h_x, h_y of the group's columns for both tiles of the pair.  Two windows at
 // a time, in the exchange and the buffer: f of both tiles, or f and df of one
 // tile after the other; the cotangents are loaded while they arrive.
-template <int M, typename T, bool TAN>
+template <int M, typename T, bool TAN, int FORM>
 __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, int blk, GroupMem<M>& gm,
                                          cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
   constexpr int HP = win_pitch<T>(M);
@@ -745,7 +757,7 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
     return o;
   };
   auto stage = [&](const TileRef& t, const void* img, int i) {
-    return issue_window<M, T>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
+    return issue_window<M, FORM>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
                               t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
   };
   auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
@@ -762,26 +774,26 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
     Window f = stage(tr[0], a.I, 0), d = stage(tr[0], a.dI, 1);
     load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, vv);
     load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[0], o0, dv);
-    window_wait(f, gm, 0);
-    window_wait(d, gm, 1);
-    adj_lane<M, T, true, 0>(gm, inside(tr[0]), vv, dv, o0, f0, f1, row(tr[0], f), hx, hy);
+    window_wait<FORM>(f, gm, 0);
+    window_wait<FORM>(d, gm, 1);
+    adj_lane<M, T, true, 0, FORM>(gm, inside(tr[0]), vv, dv, o0, f0, f1, row(tr[0], f), hx, hy);
     gm.open();  // the windows are read
     f = stage(tr[1], a.I, 0);
     d = stage(tr[1], a.dI, 1);
     load_cotangent<M, T>(static_cast<const T*>(a.v), tr[1], o1, vv);
     load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[1], o1, dv);
-    window_wait(f, gm, 0);
-    window_wait(d, gm, 1);
-    adj_lane<M, T, true, 1>(gm, inside(tr[1]), vv, dv, o1, f0, f1, row(tr[1], f), hx, hy);
+    window_wait<FORM>(f, gm, 0);
+    window_wait<FORM>(d, gm, 1);
+    adj_lane<M, T, true, 1, FORM>(gm, inside(tr[1]), vv, dv, o1, f0, f1, row(tr[1], f), hx, hy);
   } else {
     pk v0[Quad<M>::R], v1[Quad<M>::R];
     const Window f = stage(tr[0], a.I, 0), s = stage(tr[1], a.I, 1);
     load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, v0);
     load_cotangent<M, T>(static_cast<const T*>(a.v), tr[1], o1, v1);
-    window_wait(f, gm, 0);
-    window_wait(s, gm, 1);
-    adj_lane<M, T, false, 0>(gm, inside(tr[0]), v0, v0, o0, f0, f0, row(tr[0], f), hx, hy);
-    adj_lane<M, T, false, 1>(gm, inside(tr[1]), v1, v1, o1, f1, f1, row(tr[1], s), hx, hy);
+    window_wait<FORM>(f, gm, 0);
+    window_wait<FORM>(s, gm, 1);
+    adj_lane<M, T, false, 0, FORM>(gm, inside(tr[0]), v0, v0, o0, f0, f0, row(tr[0], f), hx, hy);
+    adj_lane<M, T, false, 1, FORM>(gm, inside(tr[1]), v1, v1, o1, f1, f1, row(tr[1], s), hx, hy);
   }
 }
 
@@ -801,7 +813,7 @@ __device__ __forceinline__ void p1_store(const float2 (&X)[Quad<M>::VPT], float2
 
 // P1: the group transforms columns 4 blk .. 4 blk + 3 of every field along y.
 // OP_ADJ: TAN when dv and df are given.
-template <int M, int OP, typename T, bool TAN = false>
+template <int M, int OP, typename T, bool TAN = false, int FORM = kAny>
 __device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, int blk, float2* __restrict__ S1,
                                        GroupMem<M>& gm, const float4* __restrict__ tw) {
   using Q = Quad<M>;
@@ -811,11 +823,16 @@ __device__ __forceinline__ void phase1(const OpArgs& a, const Geom& g, int w, in
   if constexpr (OP == OP_ADJ) {
     // both fields from one pass over the inputs; h_y waits in registers
     cpk hx[Q::R], hy[Q::R];
-    load_adj<M, T, TAN>(a, g, w, blk, gm, hx, hy);
-    fft_dit<M, false>(hx, X, gm.ex, tw, t);
-    p1_store<M>(X, S1, x, t.q);
-    fft_dit<M, false>(hy, X, gm.ex, tw, t);
-    p1_store<M>(X, S1 + (size_t)M * M, x, t.q);
+    load_adj<M, T, TAN, FORM>(a, g, w, blk, gm, hx, hy);
+    // one copy of the transform: the pass is short of instruction cache
+    // (adjoint N = 4096, KW = 61: 262 -> 242 us with P2's)
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      fft_dit<M, false>(hx, X, gm.ex, tw, t);
+      p1_store<M>(X, S1 + (size_t)k * M * M, x, t.q);
+#pragma unroll
+      for (int r = 0; r < Q::R; ++r) hx[r] = hy[r];
+    }
   } else {
     cpk z[Q::R];
     load_column<M, OP, T>(a, g, w, blk, gm, z);
@@ -877,39 +894,43 @@ __device__ __forceinline__ void phase2(const float2* __restrict__ S1, float2* __
     load(gm.ex, X);
     fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
     fft_dif_finish<M, false>(z);
-    gm.wait(1);
+    // (one copy of the inverse at M = 512: 171 -> 167 us per 150 work tiles;
+    // at M = 256 it spills, 159 -> 163 per 600)
+#pragma unroll (M == 512 ? 1 : 2)
+    for (int l = 0; l < 2; ++l) {
+      gm.wait(1);
 #pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
-    gm.open();
-    gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the first inverse
-    fft_dit<M, true>(b, X, gm.ex, tw, t);
-    emit(X, 0);
-    gm.wait(1);
-#pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
-    fft_dit<M, true>(b, X, gm.ex, tw, t);
-    emit(X, 1);
+      for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
+      if (l == 0) {
+        gm.open();
+        gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the first inverse
+      }
+      fft_dit<M, true>(b, X, gm.ex, tw, t);
+      emit(X, l);
+    }
   } else {
-    gm.wait(0);
-    load(gm.ex, X);
-    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
-    gm.open();  // the exchange is read: the second field takes its place
-    gm.fetch(0, gm.ex, S1 + (size_t)M * M + row, BB);
-    fft_dif_finish<M, false>(z);
-    gm.wait(1);
 #pragma unroll
-    for (int r = 0; r < Q::R; ++r) b[r] = cpk_mul<false>(z[r], spec(r));
-    gm.open();
-    gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the second transform
-    gm.wait(0);
-    load(gm.ex, X);
-    fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
-    fft_dif_finish<M, false>(z);
-    gm.wait(1);
+    for (int r = 0; r < Q::R; ++r) b[r] = cpk{0ull, 0ull};
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      gm.wait(0);
+      load(gm.ex, X);
+      fft_dif_begin<M, false>(X, z, gm.ex, tw, t);
+      if (k == 0) {
+        gm.open();  // the exchange is read: the second field takes its place
+        gm.fetch(0, gm.ex, S1 + (size_t)M * M + row, BB);
+      }
+      fft_dif_finish<M, false>(z);
+      gm.wait(1);
 #pragma unroll
-    for (int r = 0; r < Q::R; ++r) {
-      const cpk c = cpk_mul<false>(z[r], spec(r));
-      b[r] = cpk{pk_add(b[r].re, c.re), pk_add(b[r].im, c.im)};
+      for (int r = 0; r < Q::R; ++r) {
+        const cpk c = cpk_mul<false>(z[r], spec(r));
+        b[r] = cpk{pk_add(b[r].re, c.re), pk_add(b[r].im, c.im)};
+      }
+      if (k == 0) {
+        gm.open();
+        gm.fetch(1, gm.buf, Gy + row / 2, BB);  // in flight during the second transform
+      }
     }
     fft_dit<M, true>(b, X, gm.ex, tw, t);
     emit(X, 0);
@@ -1045,7 +1066,7 @@ __device__ __forceinline__ void adj_epilogue(const OpArgs& a, const OutCol& o, i
 enum S2Layout : int { kS2Engine = 0, kS2Rotated = 1 };
 
 // P3: columns 4 blk .. of S2: inverse FFT along ky, epilogue.
-template <int M, int OP, typename T, int S2L = kS2Engine>
+template <int M, int OP, typename T, int S2L = kS2Engine, int FORM = kAny>
 __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpArgs& a, const Geom& g, int w, int blk,
                                        GroupMem<M>& gm, const float4* __restrict__ tw) {
   using Q = Quad<M>;
@@ -1072,11 +1093,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     const TileRef tr = tile_h(h);
     if constexpr (GRAD) {
       const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
-      wn[h] = issue_window<M, T>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2, HP, win[h],
+      wn[h] = issue_window<M, FORM>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2, HP, win[h],
                                  a.e < 1, gm, 1 - h);
     } else {
       const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
-      wn[h] = issue_window<M, T>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], false, gm,
+      wn[h] = issue_window<M, FORM>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], false, gm,
                                  1 - h);
     }
   };
@@ -1091,30 +1112,57 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
         X[i * Q::J + m] = src[4 * (S2L == kS2Rotated ? (ky + blk) & (M - 1) : ky)];
       }
   };
+  // One copy of the transform for both fields where that does not spill: at
+  // M = 512 159 -> 148 us per 150 work tiles with pairs of stores, 208 -> 198
+  // with single ones; at M = 256 and 128 two copies are as fast or faster (153
+  // against 156, 161 against 162), and beside the copies in smaller pieces of
+  // kAny one copy spills (177 against 181, 241 against 269).
+  constexpr bool LOOP = M == 512 && FORM != kAny;
   float2 X[Q::VPT];
   cpk u0[Q::R], u1[Q::R];
   gm.open();
   gm.fetch(0, gm.ex, S2 + (size_t)blk * (kLines * M), BB);
   if constexpr (L == 2) gm.fetch(1, gm.buf, S2 + (size_t)M * P + (size_t)blk * (kLines * M), BB);
-  gm.wait(0);
-  load(gm.ex, X);
-  fft_dif_begin<M, true>(X, u0, gm.ex, tw, t);
-  if constexpr (L == 2) {
-    fft_dif_finish<M, true>(u0);
-    gm.wait(1);
-    load(gm.buf, X);
-    tc::fence_async_smem();  // the buffer's next copy comes after these reads
-    fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
-      window(0);
-    });
+  if constexpr (L == 2 && LOOP) {
+#pragma unroll 1
+    for (int l = 0; l < 2; ++l) {
+      gm.wait(l);
+      load(l ? static_cast<const void*>(gm.buf) : gm.ex, X);
+      tc::fence_async_smem();  // the buffer's next copy comes after these reads
+      fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
+        if (l) window(0);
+      });
+      if (l) {
+        gm.open();  // the exchange is read: window 1 takes its place
+        window(1);
+      }
+      fft_dif_finish<M, true>(u1);
+      if (l == 0) {
+#pragma unroll
+        for (int r = 0; r < Q::R; ++r) u0[r] = u1[r];
+      }
+    }
+  } else {
+    gm.wait(0);
+    load(gm.ex, X);
+    fft_dif_begin<M, true>(X, u0, gm.ex, tw, t);
+    if constexpr (L == 2) {
+      fft_dif_finish<M, true>(u0);
+      gm.wait(1);
+      load(gm.buf, X);
+      tc::fence_async_smem();  // the buffer's next copy comes after these reads
+      fft_dif_begin<M, true>(X, u1, gm.ex, tw, t, [&] {
+        window(0);
+      });
+      gm.open();  // the exchange is read: window 1 takes its place
+      window(1);
+      fft_dif_finish<M, true>(u1);
+    }
   }
   if constexpr (WIN) {
-    gm.open();  // the exchange is read: window 1 takes its place
-    window(1);
-    fft_dif_finish<M, true>(u1);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      window_wait(wn[h], gm, 1 - h);
+      window_wait<FORM>(wn[h], gm, 1 - h);
       if (OP == OP_TANADJ_F && h == 0) continue;  // both windows at once
       const TileRef tr = tile_h(h);
       const OutCol o = out_col<M>(g, a.e, tr, x, t.q, false);
@@ -1122,7 +1170,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
       if constexpr (GRAD) {
         const int row0 = tr.y0 + 2 * t.q - wn[h].at;
         auto al = [&](const void* p) { return !p || pair_aligned(static_cast<const T*>(p) + tr.ow); };
-        const bool vec = out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy);
+        const bool vec = FORM == kAny ? out_even(g, tr) && al(a.out0) && al(a.out_ux) && al(a.out_uy) : FORM == kEven;
         if (vec)
           grad_round<M, OP, T, true>(a, o, t.line, t.q, h, row0, win[h], HP, u0, u1);
         else
@@ -1133,12 +1181,13 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
         const int row = tr.y0 + o.rel - wn[hv].at, drow = tr.y0 + o.rel - wn[1].at;
         const T* v = win[hv] + t.line * HP + row;
         const T* dv = win[1] + t.line * HP + drow;
-        const bool vec = out_even(g, tr) && pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
-                         pair_aligned(static_cast<const float*>(a.out1) + tr.ow);
-        // both windows start at even rows: one parity
-        if ((row & 1) == 0 && vec)
+        const bool vec = FORM == kAny ? out_even(g, tr) && pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
+                                            pair_aligned(static_cast<const float*>(a.out1) + tr.ow)
+                                      : FORM == kEven;
+        const bool even = FORM == kAny ? (row & 1) == 0 : FORM == kEven;  // (both windows start at even rows)
+        if (even && vec)
           cot_epilogue<M, OP, T, true, false>(a, o, h, v, dv, u0, u1);
-        else if ((row & 1) == 0)
+        else if (even)
           cot_epilogue<M, OP, T, false, false>(a, o, h, v, dv, u0, u1);
         else
           cot_epilogue<M, OP, T, false, true>(a, o, h, v, dv, u0, u1);
@@ -1151,7 +1200,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
       const TileRef tr = tile_h(h);
       const OutCol o = out_col<M>(g, a.e, tr, x, t.q, true);
       if (!o.on) continue;
-      if (out_even(g, tr) && pair_aligned(static_cast<const T*>(a.out0) + tr.on))
+      if (FORM == kEven || (out_even(g, tr) && pair_aligned(static_cast<const T*>(a.out0) + tr.on)))
         adj_epilogue<M, T, true>(a, o, h, u0);
       else
         adj_epilogue<M, T, false>(a, o, h, u0);
@@ -1176,7 +1225,7 @@ __device__ __forceinline__ int group_index() { return threadIdx.x / Quad<M>::GT;
 
 // TAN (adjoint-type op of the tangent-adjoint, dv and df given) is chosen by
 // the launch.
-template <int M, int OP, typename T, bool TAN = false>
+template <int M, int OP, typename T, bool TAN = false, int FORM = kAny>
 __global__ void __launch_bounds__(kThreads, OP == OP_ADJ && M > 128 ? SRK_P1_ADJ_MIN_BLOCKS : SRK_P1_MIN_BLOCKS)
 k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict__ scratch) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -1184,7 +1233,7 @@ k_p1(OpArgs a, Geom g, const float4* __restrict__ tw, int w0, float2* __restrict
   const int wl = blockIdx.y;
   grid_wait();
   grid_next();
-  phase1<M, OP, T, TAN>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
+  phase1<M, OP, T, TAN, FORM>(a, g, w0 + wl, blockIdx.x * groups_of<M>() + group_index<M>(),
                         scratch + wl * wt_elems<M, OP>(g.S), gm, tw);
 }
 
@@ -1202,7 +1251,7 @@ k_p2(float2* __restrict__ scratch, const float4* __restrict__ Gx, const float4* 
                 });
 }
 
-template <int M, int OP, typename T, int S2L = kS2Engine>
+template <int M, int OP, typename T, int S2L = kS2Engine, int FORM = kAny>
 __global__ void __launch_bounds__(kThreads, M == 128                ? SRK_SMALL_MIN_BLOCKS
                                            : OpTraits<OP>::L == 1 ? SRK_P3_ADJ_MIN_BLOCKS
                                                                   : SRK_P3_MIN_BLOCKS)
@@ -1215,7 +1264,7 @@ k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ 
   grid_wait();
   grid_next();
   if (blk < nblk)
-    phase3<M, OP, T, S2L>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blk, gm, tw);
+    phase3<M, OP, T, S2L, FORM>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blk, gm, tw);
 }
 
 // ---- persistent schedule ---------------------------------------------------------

@@ -125,3 +125,13 @@ def test_adjoint_of_an_image_within_one_tile(torch_cuda, tile, N, KW, conv):
         ref = O.adj_wrt_E(v[b], f[b], Kx, Ky, e, 1.0, name)
         assert rel_max_err(host(dE[b]), ref) < TOL
         assert rel_max_err(host(rE[b]), ref) < TOL
+
+
+@pytest.mark.parametrize("tile,N,KW", [(128, 128, 15), (128, 304, 15), (128, 304, 33), (256, 256, 31), (256, 464, 31),
+                                       (512, 512, 63), (512, 912, 31), (512, 912, 61)])
+def test_aligned_forms(torch_cuda, tile, N, KW):
+    """Images in 16-byte columns take kernels that know it and the parity of
+    the first row (odd and even erosion); every operator, one tile and
+    several, against the oracle, and 2-byte storage against FP32."""
+    test_every_route(torch_cuda, tile, N, KW, 0)
+    test_storage_types_equal_the_fp32_routes(torch_cuda, tile, N, KW, 2, "float16")
