@@ -97,7 +97,7 @@ typedef struct srk_plan_info {
   int tile_M;       /* FFT tile size of the forward geometry */
   int tile_stride;  /* valid outputs per tile per axis */
   int tiles;        /* tiles per axis, forward geometry */
-  int tiles_adj;    /* tiles per axis, adjoint (full N x N output) geometry */
+  int tiles_adj;    /* tiles per axis, adjoint (full N x N output) geometry; 1 where N <= tile_M */
   int chunk_wt;     /* work tiles per scratch chunk */
   size_t scratch_bytes;
   srk_dtype dtype;
@@ -121,12 +121,12 @@ const char* srk_last_error(void);
  * B_max: largest batch a call may pass.
  * spectra_M: FFT size of the caller's spectra (N for srkTrainingForward,
  *            the reference's M_TILE for the OaS operators).
- * tile_M: 0 = choose by a cost model, SRK_TILE_AUTOTUNE = time every
+ * tile_M: 0 = choose by a cost model of N, W and B_max, SRK_TILE_AUTOTUNE = time every
  *         (tile, schedule) candidate once per device and configuration
  *         (cached on disk, see srk_autotune), else 128, 256 or 512.
  * scratch_budget_bytes: 0 = default (8 GiB, at most 1/16 of the device
  *         memory, at least 256 MiB); the scratch holds the work tiles in
- *         flight (5.8 MB each at N = 512), never more than B_max needs.
+ *         flight (5.3 MB each at N = 512, KW = 121), never more than B_max needs.
  * The plan also holds 2 W^2 B_max floats for the intermediate of the VJP
  * and the tangent-adjoint (u*v between the FFT passes and the transposed
  * stencil): every device buffer an operator uses is allocated here (plus the

@@ -24,6 +24,7 @@ template <typename T>
 bool pairs(const void* out) { return (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(T) - 1)) == 0; }
 template <typename T>
 int p1_adj_form(const OpArgs& a, const Geom& g) {
+  if (!g.rtile && a.e >= 1 && (g.N & 1)) return kOddN;
   if (g.rtile || a.e < 1 || !rows16<T>(a.I, g.N) || !rows16<T>(a.dI, g.N) || (g.TT > 1 && (g.S & 1))) return kAny;
   return ((g.TT == 1 ? g.org : 0) - a.e) & 1 ? kOdd : kEven;
 }
@@ -35,6 +36,7 @@ int p3_form(const OpArgs& a, const Geom& g) {
     return even && pairs<T>(a.out0) ? kEven : kAny;
   } else {
     if (a.e < 1 || g.e != a.e) return kAny;
+    if (g.N & 1) return kOddN;
     bool out;
     if constexpr (grad_op<OP>()) {
       if (!rows16<T>(a.I, g.N) || (OP == OP_JVP && !rows16<T>(a.dI, g.N))) return kAny;
@@ -228,13 +230,16 @@ srk_status launch_conv_m(srk_plan_s* p, const OpArgs& a, const Geom& g, int nwt,
     switch (p1_adj_form<T>(a, g)) {
       case kEven: kp1 = tan ? k_p1<M, OP, T, true, kEven> : k_p1<M, OP, T, false, kEven>; break;
       case kOdd: kp1 = tan ? k_p1<M, OP, T, true, kOdd> : k_p1<M, OP, T, false, kOdd>; break;
+      case kOddN: kp1 = tan ? k_p1<M, OP, T, true, kOddN> : k_p1<M, OP, T, false, kOddN>; break;
       default: kp1 = tan ? k_p1<M, OP, T, true> : k_p1<M, OP, T>;
     }
   }
   const int form = p3_form<OP, T>(a, g);
   auto kp3 = form == kEven ? k_p3<M, OP, T, kS2Engine, kEven> : k_p3<M, OP, T>;
-  if constexpr (!kAdj)
+  if constexpr (!kAdj) {
     if (form == kOdd) kp3 = k_p3<M, OP, T, kS2Engine, kOdd>;
+    if (form == kOddN) kp3 = k_p3<M, OP, T, kS2Engine, kOddN>;
+  }
   auto launch3 = [&](int w0, int c, float2* base, cudaStream_t s1, cudaStream_t s2, cudaStream_t s3,
                      cudaEvent_t e1, cudaEvent_t e2) -> srk_status {
     const dim3 g1(M / unit_lines<M>(), c);

@@ -26,9 +26,10 @@
 // xa = e rounded down to a multiple of four (s2_first).
 //
 // A group of one (M = 128, 256) or two (M = 512) warps transforms four lines
-// with 32 (M = 128: 16) complex values per thread, straight from global
-// memory into registers and back; shared memory holds one exchange per
-// transform and the gradient windows of P3.  A second field (P2's Z*Gy, P3's
+// with 32 (M = 128: 16) complex values per thread.  Its inputs (columns,
+// spectra, blocks of S1 and S2, image windows) arrive in shared memory by
+// bulk copies, which free the group's exchange and one more buffer hold in
+// turn; results are stored from registers.  A second field (P2's Z*Gy, P3's
 // and the adjoint's second field) stays in registers: at 168 registers and
 // 12 warps per SM that costs less than its round trip through shared memory
 // at a higher occupancy, since the packed transforms have 16 independent
@@ -500,15 +501,18 @@ __host__ __device__ constexpr size_t win_bytes() { return (size_t)kWinCols * win
 template <int M>
 __host__ __device__ constexpr size_t win_lead() { return 2 * (size_t)M; }
 
-// What a launch knows of the images that its blocks stage: nothing, or that
+// What a launch knows of the images that its blocks stage: nothing; or that
 // every column starts on 16 bytes, the erosion is at least 1 and the first row
 // that a thread works on is even / odd in every tile (P3: even also means that
-// every pair of outputs is one aligned store).  The kernels of the two known
-// forms hold neither the copies in smaller pieces nor the other parity's
-// arithmetic.  The passes are short of instruction cache and registers, so
-// the paths not taken cost: P3 of 150 image pairs at M = 512 177 -> 149 us
-// (erosion 60), 241 -> 198 (15); of 600 at M = 256 179 -> 153 and 220 -> 189.
-enum Form : int { kAny = 0, kEven = 1, kOdd = 2 };
+// every pair of outputs is one aligned store); or that N is odd (element-wise
+// windows, single stores) and the erosion at least 1.  The kernels of the known
+// forms hold neither the copies in other pieces nor the other stores and, of
+// the 16-byte forms, the other parity.  The passes are short of instruction
+// cache and registers, so the paths not taken cost: P3 of 150 image pairs at
+// M = 512 177 -> 149 us (erosion 60), 241 -> 198 (15); of 600 at M = 256
+// 179 -> 153 and 220 -> 189; forward of 100 images of 511, KW 31: 206 -> 193.
+enum Form : int { kAny = 0, kEven = 1, kOdd = 2, kOddN = 3 };
+__host__ __device__ constexpr bool rows16_form(int form) { return form == kEven || form == kOdd; }
 
 // An issued window: `at` is the image row of element 0; the caller waits for
 // it with window_wait.
@@ -535,8 +539,9 @@ __device__ __forceinline__ bool window_zero(int nc, int n, int c0, int c1, int r
 }
 
 // Columns [c0, c1) and elements [r0, r1) (whole pieces) of a window in
-// asynchronous pieces of BYTES; 2: single values through registers, a batch
-// of loads in flight.
+// asynchronous pieces of BYTES; 2: through registers, a batch of loads in
+// flight, in aligned words (forward of 100 FP16 images of 511, KW 31: 262 us
+// with single values, 195 so).
 template <int M, typename T, int BYTES>
 __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, int c0, int c1, int r0, int r1, int HP,
                                               T* __restrict__ win) {
@@ -553,21 +558,50 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(p), "n"(BYTES) : "memory");
     }
   } else {
-    constexpr int KS = 3;  // rows per batch and column: kWinCols KS loads in flight
-#pragma unroll 1
-    for (int k = r0 + t; k < r1; k += KS * GT) {
-      T v[kWinCols][KS];
+    // Four elements per thread and column from the aligned words around them,
+    // where these lie wholly inside the column's elements; the up to four at
+    // either end of a column one by one, each by a thread of its own.
+    static_assert(win_pitch<T>(M) % 4 == 0, "8-byte stores");
+    const int K0 = r0 & -4;
+    const unsigned odd0 = (unsigned)(reinterpret_cast<uintptr_t>(src) >> 1);
+    auto shift = [&](int c) { return (int)((odd0 + (unsigned)(c * N)) & 1); };  // of column c against the words
+    constexpr int ENDS = (8 * kWinCols + GT - 1) / GT;
+    T ev[ENDS];
+    int ek[ENDS];  // window element, or -1
 #pragma unroll
-      for (int c = 0; c < kWinCols; ++c)
-#pragma unroll
-        for (int s = 0; s < KS; ++s)
-          if (c >= c0 && c < c1 && k + s * GT < r1) v[c][s] = src[(long long)c * N + k + s * GT];
-#pragma unroll
-      for (int c = 0; c < kWinCols; ++c)
-#pragma unroll
-        for (int s = 0; s < KS; ++s)
-          if (c >= c0 && c < c1 && k + s * GT < r1) win[c * HP + k + s * GT] = v[c][s];
+    for (int i = 0; i < ENDS; ++i) {
+      const int j = (t + i * GT) & 7, c = (t + i * GT) >> 3, s = shift(c);
+      const int first = min(K0 - s >= r0 ? K0 : K0 + 4, r1);             // the words begin
+      const int last = max(K0 + ((r1 - s - K0) >> 2) * 4, first);        // and end here
+      const int k = j < 4 ? r0 + j : last + j - 4;
+      const bool on = c >= c0 && c < c1 && (j < 4 ? k < first : k < r1);
+      ek[i] = on ? c * HP + k : -1;
+      if (on) ev[i] = src[(long long)c * N + k];
     }
+#pragma unroll 1
+    for (int k = K0 + 4 * t; k < r1; k += 4 * GT) {
+      unsigned w[kWinCols][3];
+#pragma unroll
+      for (int c = 0; c < kWinCols; ++c) {
+        const int s = shift(c);
+        const unsigned* q = reinterpret_cast<const unsigned*>(src + (long long)c * N + k - s);
+        if (c >= c0 && c < c1 && k - s >= r0 && k + 4 + s <= r1) {
+          w[c][0] = q[0];
+          w[c][1] = q[1];
+          if (s) w[c][2] = q[2];
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < kWinCols; ++c) {
+        const int s = shift(c);
+        if (c >= c0 && c < c1 && k - s >= r0 && k + 4 + s <= r1)
+          *reinterpret_cast<uint2*>(win + c * HP + k) =
+              make_uint2(__funnelshift_r(w[c][0], w[c][1], 16 * s), __funnelshift_r(w[c][1], w[c][2], 16 * s));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ENDS; ++i)
+      if (ek[i] >= 0) win[ek[i]] = ev[i];
   }
 }
 
@@ -591,10 +625,10 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   static_assert(kWinCols <= GT, "one thread per column");
   const int t = threadIdx.x % GT;
   const int mis = (int)(reinterpret_cast<uintptr_t>(img) & 15) | (N * (int)sizeof(T));  // alignment of every column
-  const int bytes = FORM != kAny || !(mis & 15) ? 16 : !(mis & 7) ? 8 : !(mis & 3) ? 4 : 2;  // the piece that it allows
+  const int bytes = FORM == kOddN ? (int)sizeof(T) : FORM != kAny || !(mis & 15) ? 16 : !(mis & 7) ? 8 : !(mis & 3) ? 4 : 2;  // the piece that it allows
   const int E = max(bytes / (int)sizeof(T), 1);
   Window w;
-  w.bulk = live && bytes == 16;
+  w.bulk = FORM != kOddN && live && bytes == 16;
   w.at = gy0 & -max(E, 2);
   w.sync = live && !w.bulk;
   if (!live) return w;  // (nothing reads the window of a dead tile)
@@ -603,6 +637,10 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   const int r0 = max(0, -w.at), r1 = max(r0, min(n, N - w.at));
   const int c0 = min(nc, max(0, -gx0)), c1 = max(c0, min(nc, N - gx0));
   const T* src = img + (long long)gx0 * N + w.at;  // (dereferenced inside the image only)
+  if constexpr (FORM == kOddN) {
+    window_pieces<M, T, (int)sizeof(T)>(src, N, c0, c1, r0, r1, HP, win);
+    return w;
+  }
   if (w.bulk) {
     const unsigned len = (unsigned)((r1 - r0) * sizeof(T));
     if (t == 0) tc::mbar_expect_tx(gm.bar + i, (unsigned)(c1 - c0) * len);
@@ -622,11 +660,11 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
 // The window has arrived for every thread of the group (group-uniform).
 template <int FORM, int M>
 __device__ __forceinline__ void window_wait(const Window& w, GroupMem<M>& gm, int i) {
-  if (w.bulk)
+  if (FORM != kOddN && w.bulk)
     gm.wait(i);
-  else if (FORM == kAny)
+  else if (!rows16_form(FORM))
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (FORM == kAny && w.sync) group_sync<M>();
+  if (!rows16_form(FORM) && w.sync) group_sync<M>();
 }
 
 // This thread's column of one tile in a W- or N-sized array: rows y = 2q + l
@@ -722,7 +760,7 @@ __device__ __forceinline__ void adj_lane(const GroupMem<M>& gm, bool cols, const
                                          cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
   const int y0 = o.rel - 2 * gm.t.q;  // first tile row in the valid window (group-uniform, like `inside`)
   const bool inside = cols && y0 >= 0 && y0 + M <= (int)o.cnt;
-  const bool odd = FORM == kAny ? row & 1 : FORM == kOdd;
+  const bool odd = rows16_form(FORM) ? FORM == kOdd : row & 1;
   if (!inside) {
     if (odd)
       adj_fields<M, T, TAN, LANE, true, true>(vv, dv, o, wf, wd, row, hx, hy);
@@ -1116,8 +1154,8 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
   // M = 512 159 -> 148 us per 150 work tiles with pairs of stores, 208 -> 198
   // with single ones; at M = 256 and 128 two copies are as fast or faster (153
   // against 156, 161 against 162), and beside the copies in smaller pieces of
-  // kAny one copy spills (177 against 181, 241 against 269).
-  constexpr bool LOOP = M == 512 && FORM != kAny;
+  // kAny and kOddN one copy spills (177 against 181, 241 against 269).
+  constexpr bool LOOP = M == 512 && rows16_form(FORM);
   float2 X[Q::VPT];
   cpk u0[Q::R], u1[Q::R];
   gm.open();
@@ -1184,7 +1222,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
         const bool vec = FORM == kAny ? out_even(g, tr) && pair_aligned(static_cast<const float*>(a.out0) + tr.ow) &&
                                             pair_aligned(static_cast<const float*>(a.out1) + tr.ow)
                                       : FORM == kEven;
-        const bool even = FORM == kAny ? (row & 1) == 0 : FORM == kEven;  // (both windows start at even rows)
+        const bool even = rows16_form(FORM) ? FORM == kEven : (row & 1) == 0;  // (both windows start at even rows)
         if (even && vec)
           cot_epilogue<M, OP, T, true, false>(a, o, h, v, dv, u0, u1);
         else if (even)

@@ -79,7 +79,7 @@ srk_status launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 #endif
 struct srk_plan_s {
   int device = 0;
-  int nsm = 0;  // SMs of the device (L2 prefetch distances)
+  int nsm = 0;  // SMs of the device
   int N = 0, W = 0, e = 0, B_max = 0, spectra_M = 0;
   float dx = 1.f;
   srk_dtype dtype = SRK_F32;

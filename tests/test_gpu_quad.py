@@ -135,3 +135,12 @@ def test_aligned_forms(torch_cuda, tile, N, KW):
     several, against the oracle, and 2-byte storage against FP32."""
     test_every_route(torch_cuda, tile, N, KW, 0)
     test_storage_types_equal_the_fp32_routes(torch_cuda, tile, N, KW, 2, "float16")
+
+
+@pytest.mark.parametrize("tile,N,KW,B", [(128, 127, 3, 3), (128, 301, 33, 2), (256, 255, 61, 3), (512, 509, 121, 2),
+                                         (512, 905, 31, 1)])
+def test_odd_columns_of_two_byte_storage(torch_cuda, tile, N, KW, B):
+    """Odd N, 2-byte storage: windows from the words around each column, whose
+    alignment changes from column to column and from image to image."""
+    for dt in ("float16", "bfloat16"):
+        test_storage_types_equal_the_fp32_routes(torch_cuda, tile, N, KW, B, dt)
