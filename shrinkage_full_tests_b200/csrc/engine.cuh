@@ -49,6 +49,7 @@
 #include <type_traits>
 #include "fft_quad.cuh"
 #include "tc.cuh"
+#include "tile_cols.h"
 
 // CTAs of kThreads threads per SM the kernels are compiled for (register cap
 // 65536 / (kThreads n), in steps of 8): 8 -> 128 registers, 6 -> 168.
@@ -523,7 +524,7 @@ struct Window {
 };
 
 // Elements [0, n) of the nc columns that bulk copies or window_pieces do not
-// write (outside the image): zero.  Columns c0 .. c1 - 1, elements r0 .. r1 - 1
+// write (outside the image, or needed by no valid output): zero.  Columns c0 .. c1 - 1, elements r0 .. r1 - 1
 // lie in the image.  Returns whether there are any.
 template <int M, typename T>
 __device__ __forceinline__ bool window_zero(int nc, int n, int c0, int c1, int r0, int r1, int HP, T* __restrict__ win) {
@@ -605,9 +606,9 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
   }
 }
 
-// Starts the copy of nc (at most the group's threads) columns from gx0 and nr
-// rows from gy0 of the N x N image at img (any of them outside the image; not
-// live: nothing) on the group's barrier i.  edge: elements outside the image
+// Starts the copy of nc (at most the group's threads) columns from gx0, of
+// them those of `need`, and nr rows from gy0 of the N x N image at img (any of
+// them outside the image; not live: nothing) on the group's barrier i.  edge: elements outside the image
 // become zero; else they keep whatever the memory held (with erosion >= 1
 // only values that are never stored read them, and zeroing them was the
 // longest step of a tile at the image's edge).  One bulk copy per column where
@@ -617,9 +618,9 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 // the threads copy the largest pieces that N and the image allow.  The group
 // is past gm.open().  FORM: what the launch knows of the images (Form).
 template <int M, int FORM, typename T>
-__device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, int gy0,
-                                               int nr, int HP, T* __restrict__ win, bool edge, const GroupMem<M>& gm,
-                                               int i) {
+__device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, ColSpan need,
+                                               int gy0, int nr, int HP, T* __restrict__ win, bool edge,
+                                               const GroupMem<M>& gm, int i) {
   constexpr int EPC = 16 / (int)sizeof(T);
   constexpr int GT = Quad<M>::GT;
   static_assert(kWinCols <= GT, "one thread per column");
@@ -635,7 +636,8 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   // whole pieces; elements r0 .. r1 - 1 and columns c0 .. c1 - 1 lie in the image
   const int n = (gy0 - w.at + nr + E - 1) & -E;
   const int r0 = max(0, -w.at), r1 = max(r0, min(n, N - w.at));
-  const int c0 = min(nc, max(0, -gx0)), c1 = max(c0, min(nc, N - gx0));
+  const ColSpan cs = clip_span(need, gx0, N);
+  const int c0 = cs.lo, c1 = cs.hi;
   const T* src = img + (long long)gx0 * N + w.at;  // (dereferenced inside the image only)
   if constexpr (FORM == kOddN) {
     window_pieces<M, T, (int)sizeof(T)>(src, N, c0, c1, r0, r1, HP, win);
@@ -796,7 +798,7 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
   };
   auto stage = [&](const TileRef& t, const void* img, int i) {
     return issue_window<M, FORM>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
-                              t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
+                              ColSpan{0, kWinCols}, t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
   };
   auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
     const int ox = t.x0 + blk * kLines - 2 * a.e;
@@ -1131,12 +1133,12 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     const TileRef tr = tile_h(h);
     if constexpr (GRAD) {
       const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
-      wn[h] = issue_window<M, FORM>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, tr.y0 + g.e - 1, g.S + 2, HP, win[h],
-                                 a.e < 1, gm, 1 - h);
+      wn[h] = issue_window<M, FORM>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, window_span(xg, g.e, g.S, 1),
+                                 tr.y0 + g.e - 1, g.S + 2, HP, win[h], a.e < 1, gm, 1 - h);
     } else {
       const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
-      wn[h] = issue_window<M, FORM>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, tr.y0, g.S, HP, win[h], false, gm,
-                                 1 - h);
+      wn[h] = issue_window<M, FORM>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, window_span(xg, g.e, g.S, 0), tr.y0, g.S,
+                                 HP, win[h], false, gm, 1 - h);
     }
   };
   // column x of a staged S2 block: ky = k_i + R m
