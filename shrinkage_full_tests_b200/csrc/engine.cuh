@@ -1317,6 +1317,11 @@ k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ 
 //   P2(w) needs c1[slot] >= (gen+1)*n1   (its S1 complete)
 //           and c3[slot] >= gen*n3       (previous user's P3 done reading S2)
 //   P3(w) needs c2[slot] >= (gen+1)*n2   (its S2 complete)
+// S1 and S2 are stored by ordinary stores and fetched by bulk copies, which
+// read global memory through the async proxy: the counters' release and
+// acquire order ordinary accesses only, so every thread fences its stores
+// before the release and the copying threads fence after the acquire
+// (fence_async_global).  Between launches the kernel boundary does that.
 // Every dependency points to a smaller ticket, and a ticket is only ever held
 // by a running CTA (a CTA holds at most its current ticket and one
 // prefetched larger one), so the smallest unfinished ticket can always
@@ -1408,6 +1413,7 @@ k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restr
     __syncthreads();
     if (!s_t[1]) break;
     if (live) {
+      tc::fence_async_global();  // the copies come after the stores just acquired
       float2* base = scratch + (size_t)slot * slot_elems;
       const int blk = unit * NG + group_index<M>();
       if (phase == 1) {
@@ -1420,6 +1426,7 @@ k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restr
       } else if (blk < nblk) {
         phase3<M, OP, T>(base + s1_elems<M, OP>(), a, g, w, blk, gm, tw);
       }
+      tc::fence_async_global();  // this thread's scratch stores, before other blocks' copies
     }
     __syncthreads();  // every thread's scratch stores of this unit are issued
     if (threadIdx.x == 0) {
