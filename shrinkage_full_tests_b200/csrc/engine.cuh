@@ -316,23 +316,26 @@ template <> __device__ __forceinline__ pk swin2<__nv_bfloat16>(const __nv_bfloat
 }
 
 // One value and an aligned pair under a predicate (zero without it): a
-// predicated load, not a branch around one.
+// predicated load, not a branch around one.  Ordinary loads that stay behind
+// grid_wait (volatile, memory clobber): what they read may be stored by the
+// kernel before, which still runs when a dependent launch's blocks start, so
+// the read-only path (ld.global.nc) does not serve.
 __device__ __forceinline__ unsigned short ldp16(const void* p, bool on) {
   unsigned short v;
-  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b16 %0, 0;\n\t@q ld.global.nc.b16 %0, [%1];\n\t}"
-      : "=h"(v) : "l"(p), "r"((unsigned)on));
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b16 %0, 0;\n\t@q ld.global.b16 %0, [%1];\n\t}"
+               : "=h"(v) : "l"(p), "r"((unsigned)on) : "memory");
   return v;
 }
 __device__ __forceinline__ unsigned ldp32(const void* p, bool on) {
   unsigned v;
-  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.nc.b32 %0, [%1];\n\t}"
-      : "=r"(v) : "l"(p), "r"((unsigned)on));
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b32 %0, 0;\n\t@q ld.global.b32 %0, [%1];\n\t}"
+               : "=r"(v) : "l"(p), "r"((unsigned)on) : "memory");
   return v;
 }
 __device__ __forceinline__ pk ldp64(const void* p, bool on) {
   pk v;
-  asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b64 %0, 0;\n\t@q ld.global.nc.b64 %0, [%1];\n\t}"
-      : "=l"(v) : "l"(p), "r"((unsigned)on));
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.b64 %0, 0;\n\t@q ld.global.b64 %0, [%1];\n\t}"
+               : "=l"(v) : "l"(p), "r"((unsigned)on) : "memory");
   return v;
 }
 template <typename T> __device__ __forceinline__ float ldp(const T* p, bool on);
@@ -1255,7 +1258,8 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
 // kernel before is complete and visible).  Every kernel waits before it lets
 // the next one start (grid_next), so at most two kernels overlap and what a
 // kernel does before its wait may use anything older than its predecessor.
-// A no-op where the launch is an ordinary one.
+// A no-op where the launch is an ordinary one.  Only tables that are older
+// than the call (twiddles) are read through the read-only path.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -37,7 +37,7 @@ def test_short_ring_many_calls(torch_cuda, tile, N, KW, B):
     gen = torch.Generator(device="cuda").manual_seed(N)
     plans = []
     for sch in (srk.SRK_SCHEDULE_PERSISTENT, srk.SRK_SCHEDULE_THREE_PASS):
-        p = srk.SrkPlan(N, W, e, 1.0, B, tile_M=tile)
+        p = srk.SrkPlan(N, W, e, 1.0, B, spectra_M=1024, tile_M=tile)
         p.set_kernel(Kx, Ky)
         p.set_schedule(sch)
         plans.append(p)
