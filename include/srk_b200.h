@@ -147,14 +147,24 @@ srk_status srk_plan_set_schedule(srk_plan plan, srk_schedule schedule);
  * tile; 0 = derived from the grid), grid (CTAs; 0 = all that fit), prefetch
  * (1 = fetch the next ticket while running the current one). */
 srk_status srk_plan_set_persistent(srk_plan plan, int lag, int grid, int prefetch);
-/* Synchronise `stream` and report a device-side failure of the plan's last
- * persistent launch (SRK_ERR_TIMEOUT if a bounded wait gave up).  Operators
- * also report such a failure of the previous call once it has completed. */
+/* Synchronise `stream` and report a device-side failure of the plan's calls
+ * (SRK_ERR_TIMEOUT if a bounded wait gave up: an FFT pass waiting for a copy,
+ * a persistent launch waiting for another block, a tensor-core schedule's
+ * pipeline).  The outputs of that call are incomplete, and the block that
+ * gave up has stored nothing.  Operators also report such a failure of an
+ * earlier call once that has completed, except one of the tensor-core
+ * schedules, which only this call finds. */
 srk_status srk_plan_sync(srk_plan plan, srk_stream_t stream);
 /* Failure-path self test: one CTA waits, bounded by spin_limit polls, for a
  * counter that nothing increments.  Returns SRK_ERR_TIMEOUT when the wait
  * gave up as designed (the context stays usable), SRK_OK never. */
 srk_status srk_debug_wait_selftest(srk_plan plan, unsigned long long spin_limit, srk_stream_t stream);
+/* The same for an FFT pass's wait: a group of threads waits, bounded by
+ * spin_limit polls, for a copy that is never issued.  Returns SRK_OK when no
+ * thread went on after the wait; the failure itself is reported as that of an
+ * operator would be: by the plan's next operator or srk_plan_sync, or with
+ * plan == NULL by srk_noalloc_sync. */
+srk_status srk_debug_copy_wait_selftest(srk_plan plan, unsigned long long spin_limit, srk_stream_t stream);
 
 /* Import caller spectra (reference layout, size spectra_M).  Done implicitly
  * by the operators whenever they see spectrum pointers different from the
@@ -345,6 +355,10 @@ srk_status srk_cd_strip(const float* d_E, const float* d_I, const float* d_Kx, c
 srk_status srk_training_forward_noalloc(const float* d_E, const float* d_I, const void* d_Gx_freq,
                                         const void* d_Gy_freq, int N, int W, int erosion, float dx, int B,
                                         srk_stream_t stream, float* d_R);
+/* Synchronise `stream` and report (once) a bounded device-side wait that gave
+ * up in a call above on the current device: SRK_ERR_TIMEOUT, outputs
+ * incomplete.  A call itself is asynchronous and cannot. */
+srk_status srk_noalloc_sync(srk_stream_t stream);
 
 /* ---- storage-typed forms ----------------------------------------------------
  * Same operators with every image / cotangent / output buffer in the plan's

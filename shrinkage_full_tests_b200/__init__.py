@@ -73,6 +73,8 @@ _SIGS = {
     "srk_plan_set_persistent": [_P, _I, _I, _I],
     "srk_plan_sync": [_P, _P],
     "srk_debug_wait_selftest": [_P, ctypes.c_ulonglong, _P],
+    "srk_debug_copy_wait_selftest": [_P, ctypes.c_ulonglong, _P],
+    "srk_noalloc_sync": [_P],
     "srk_plan_import_spectra": [_P, _P, _P, _P],
     "srk_plan_set_kernel": [_P, _P, _P, _I, _P],
     "srk_green_tensor": [_P, _P, _I, _D, _D, _D, _P],
@@ -184,6 +186,11 @@ class SrkPlan:
     def wait_selftest(self, spin_limit=1 << 12, stream=None):
         """Return the status of the bounded-wait self test (SRK_ERR_TIMEOUT expected)."""
         return lib().srk_debug_wait_selftest(self.handle, spin_limit, _stream(stream))
+
+    def copy_wait_selftest(self, spin_limit=1 << 12, stream=None):
+        """Status of srk_debug_copy_wait_selftest; the failure it provokes is
+        reported by the next operator or sync()."""
+        return lib().srk_debug_copy_wait_selftest(self.handle, spin_limit, _stream(stream))
 
     def import_spectra(self, Gx_freq, Gy_freq, stream=None):
         _check(lib().srk_plan_import_spectra(self.handle, _ptr(Gx_freq), _ptr(Gy_freq), _stream(stream)))

@@ -242,13 +242,28 @@ __host__ __device__ inline size_t spec_index(int M, int ky, int kx) {
 //   buffer    one block of four lines (4 M complex values): the second input,
 //             the spectra, or a gradient window
 //   barriers  two mbarriers
+// A wait whose copy never comes ends the thread (wait): nothing is made from
+// the missing data and, without the leader, no further copy is issued.  The
+// call's outputs are incomplete, which the error word tells the host.
 template <int M>
 __host__ __device__ constexpr size_t exch_bytes() { return sizeof(float4) * (size_t)Quad<M>::XQ; }
 template <int M>
 __host__ __device__ constexpr size_t block_bytes() { return sizeof(float2) * (size_t)kLines * M; }
 template <int M, bool BUF>
 __host__ __device__ constexpr size_t group_bytes() { return exch_bytes<M>() + (BUF ? block_bytes<M>() : 0) + 16; }
-constexpr unsigned long long kBulkWaitLimit = 1ull << 22;
+// Polls before a wait gives up: the second half of them is the wait for a copy
+// that may still land in the block's memory.
+constexpr unsigned long long kBulkWaitLimit = 1ull << 23;
+constexpr unsigned kStopSite = 20;  // what a thread that gave up a wait writes to the error word
+// The last two quads of the exchange are used by no line (Quad<M>::LP) and
+// what lands in the exchange ends before them: a thread that gives up a wait
+// sets this word, for the code whose other threads go on.
+template <int M>
+__host__ __device__ constexpr size_t landing_bytes() { return exch_bytes<M>() - 2 * sizeof(float4); }
+template <int M>
+__device__ __forceinline__ unsigned* stop_word(void* group_memory) {
+  return reinterpret_cast<unsigned*>(static_cast<float4*>(group_memory) + Quad<M>::XQ - 1);
+}
 
 template <int M>
 struct GroupMem {
@@ -257,7 +272,7 @@ struct GroupMem {
   unsigned char* buf;
   uint64_t* bar;       // two barriers
   unsigned parity;     // bit i: the phase barrier i waits for next
-  unsigned int* err;
+  unsigned int* err;   // error word (device or mapped host memory, may be nullptr)
   __device__ __forceinline__ bool leader() const { return threadIdx.x % Quad<M>::GT == 0; }
   // Copies may be issued into memory that the group has used before.
   __device__ __forceinline__ void open() const {
@@ -271,8 +286,8 @@ struct GroupMem {
       tc::bulk_g2s(dst, src, bytes, bar + i);
     }
   }
-  __device__ __forceinline__ void wait(int i) {
-    if (!tc::mbar_wait(bar + i, parity >> i & 1u, kBulkWaitLimit) && err) atomicCAS(err, 0u, 16u);
+  __device__ __forceinline__ void wait(int i, unsigned long long limit = kBulkWaitLimit) {
+    tc::leave_unless<kStopSite>(tc::mbar_wait(bar + i, parity >> i & 1u, limit), err, stop_word<M>(ex));
     parity ^= 1u << i;
   }
 };
@@ -291,6 +306,7 @@ __device__ __forceinline__ GroupMem<M> group_mem(unsigned char* sm, unsigned int
   if (g.leader()) {
     tc::mbar_init(g.bar, 1);
     tc::mbar_init(g.bar + 1, 1);
+    *stop_word<M>(g.ex) = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   return g;
@@ -430,7 +446,7 @@ __device__ __forceinline__ bool load_columns_bulk(const T* const (&img)[2], cons
   constexpr int R = Quad<M>::R, J = Quad<M>::J;
   constexpr int CP = bulk_pitch<M, T>();
   constexpr int EPC = 16 / (int)sizeof(T);
-  static_assert(8 * CP * sizeof(T) <= exch_bytes<M>(), "the columns land in the exchange");
+  static_assert(8 * CP * sizeof(T) <= landing_bytes<M>() && block_bytes<M>() <= landing_bytes<M>(), "the columns land in the exchange");
   T* st = reinterpret_cast<T*>(gm.ex);
   int rows[2], cols[2];
   bool ok = true;
@@ -785,7 +801,7 @@ template <int M, typename T, bool TAN, int FORM>
 __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, int blk, GroupMem<M>& gm,
                                          cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
   constexpr int HP = win_pitch<T>(M);
-  static_assert(win_bytes<M, T>() <= exch_bytes<M>() && win_bytes<M, T>() <= block_bytes<M>(), "window size");
+  static_assert(win_bytes<M, T>() <= landing_bytes<M>() && win_bytes<M, T>() <= block_bytes<M>(), "window size");
   const TileRef tr[2] = {tile_of(g, 2 * w), tile_of(g, 2 * w + 1)};
   const int x = blk * kLines + gm.t.line, q2 = 2 * gm.t.q;
   T* const w0 = reinterpret_cast<T*>(gm.ex);
@@ -1118,7 +1134,7 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
   static_assert(GRAD || cot_op<OP>() || L == 1, "two-field ops have windows");
   constexpr unsigned BB = (unsigned)block_bytes<M>();
   // rows below the last output reach less than e elements past a window
-  static_assert(!WIN || (win_bytes<M, T>() + 2 * win_lead<M>() <= exch_bytes<M>() &&
+  static_assert(!WIN || (win_bytes<M, T>() + 2 * win_lead<M>() <= landing_bytes<M>() &&
                           win_bytes<M, T>() + win_lead<M>() <= block_bytes<M>()),
                 "the windows reuse the buffer (behind the exchange) and the exchange");
   const QuadThread t = gm.t;
@@ -1318,6 +1334,18 @@ k_p3(float2* __restrict__ scratch, OpArgs a, Geom g, const float4* __restrict__ 
     phase3<M, OP, T, S2L, FORM>(scratch + wl * wt_elems<M, OP>(g.S) + s1_elems<M, OP>(), a, g, w0 + wl, blk, gm, tw);
 }
 
+// Failure-path self test of the passes' waits: a group waits, with a short
+// limit, for a copy that is never issued; `out` counts the threads that go on.
+static __global__ void __launch_bounds__(kThreads)
+k_copy_wait_selftest(unsigned int* err, unsigned long long limit, unsigned int* out) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  GroupMem<512> gm = group_mem<512, false>(sm, err);
+  gm.open();
+  gm.wait(0, limit);
+  gm.open();
+  atomicAdd(out, 1u);
+}
+
 // ---- persistent schedule ---------------------------------------------------------
 // One launch processes every WT.  Work is a ticket queue of rounds; round r
 // holds the P1 units of WT r, the P2 units of WT r-lag and the P3 units of
@@ -1422,7 +1450,17 @@ k_persist(OpArgs a, Geom g, const float4* __restrict__ Gx, const float4* __restr
       s_t[1] = ok ? 1 : 0;
     }
     __syncthreads();
-    if (!s_t[1]) break;
+    // a thread of this block that gave up a wait for a copy has left (perhaps
+    // the one that draws the tickets): end the launch
+    bool stopped = false;
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+      stopped |= *const_cast<volatile unsigned*>(stop_word<M>(sm + i * group_bytes<M, true>())) != 0u;
+    if (stopped) {
+      atomicExch(&ctl->where, kStopSite);
+      atomicExch(&ctl->abort, 1u);
+    }
+    if (!s_t[1] || stopped) break;
     if (live) {
       tc::fence_async_global();  // the copies come after the stores just acquired
       float2* base = scratch + (size_t)slot * slot_elems;

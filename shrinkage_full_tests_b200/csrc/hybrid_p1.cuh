@@ -83,7 +83,12 @@ __device__ __forceinline__ void p1h_cols(const CUtensorMap* pmap, const OpArgs& 
   tc::fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
-    if ((tc::smem_u32(st) & 127u) == 0) {
+    bool stopped = false;  // a group whose columns never came has left: the planes keep what they held
+    for (int i = 0; i < NU; ++i)
+      stopped |= *const_cast<volatile unsigned*>(stop_word<M>(sm + i * group_bytes<M, false>())) != 0u;
+    if (stopped) {
+      // nothing to store
+    } else if ((tc::smem_u32(st) & 127u) == 0) {
       for (int p0 = 0; p0 < 2 * M; p0 += kP1hBox) tc::tma_store_3d(pmap, xb * kP1hCols, wl, p0, st + p0 * kP1hCols);
       tc::bulk_commit();
     } else {
@@ -103,7 +108,7 @@ k_p1h(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const float4* 
       unsigned int* __restrict__ zmax, unsigned int* err) {
   static_assert(OpTraits<OP>::K == 1, "single-field ops only");
   extern __shared__ __align__(128) unsigned char smh[];
-  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, err);
+  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, g.err);
   p1h_cols<OP, T>(&pmap, a, g, smh, gm, tw, w0, blockIdx.y, blockIdx.x, 1.f, zmax, err);
 }
 
@@ -118,7 +123,7 @@ k_p1h_refit(const __grid_constant__ CUtensorMap pmap, OpArgs a, Geom g, const fl
             const unsigned int* __restrict__ zmax, unsigned int* err) {
   constexpr int NX = kHybM / kP1hCols;  // column blocks per work tile
   extern __shared__ __align__(128) unsigned char smh[];
-  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, err);
+  GroupMem<kHybM> gm = group_mem<kHybM, false>(smh, g.err);
   P1hAux* aux = reinterpret_cast<P1hAux*>(smh + p1h_aux_offset());
   int* cnt = aux->cnt;
   int* list = aux->list;

@@ -124,7 +124,8 @@ struct srk_plan_s {
   size_t wbuf_bytes = 0;
   int schedule = SRK_SCHEDULE_THREE_PASS;
   srk::Ctl* ctl = nullptr;             // persistent-kernel control block
-  unsigned int* mailbox = nullptr;     // pinned host copy of (abort, where)
+  unsigned int* mailbox = nullptr;     // pinned host memory: copies of (abort, where), and the word `stop` points at
+  unsigned int* stop = nullptr;        // device address of mailbox[2]: the site of an FFT pass's wait that gave up
   cudaEvent_t mailbox_ev = nullptr;
   bool mailbox_pending = false;
   bool graph_mailbox = false;          // a captured persistent launch writes the mailbox on replay
@@ -190,6 +191,10 @@ srk_status tensor_rows_p1g_maps(const srk_plan_s* p, const void* img, int N, int
 // Tensor map of a chunk's FP16 planes [2M][c][M] with the given box.
 srk_status tensor_rows_plane_map(const __half* planes, int c, unsigned box_x, unsigned box_w, unsigned box_p,
                                  CUtensorMap* out, bool swizzle128 = false);
+
+// Words beside the no-allocation forward's scratch array (noalloc.cu): the
+// error word of its waits, and one for the self test.
+srk_status noalloc_words(unsigned int** stop, unsigned int** spare);
 
 // Spectrum kernels defined in spectra.cuh (compiled once, in srk_abi.cu) and
 // launched from the other translation units too.

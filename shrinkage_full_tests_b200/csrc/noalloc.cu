@@ -38,19 +38,28 @@ constexpr int kNoAllocMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
-std::mutex g_noalloc_mutex;
-void* g_noalloc_ptr[kNoAllocMaxDevices] = {};
+// [0] the error word of the passes' bounded waits (srk_noalloc_sync reads and
+// clears it), [1] spare
+static __device__ unsigned int g_noalloc_words[2];
 
-// Device address of the scratch array on the current device (resolved once
-// per device).
-srk_status noalloc_scratch(void** out) {
+struct NoAllocPtrs {
+  void* scratch;
+  unsigned int* words;
+};
+std::mutex g_noalloc_mutex;
+NoAllocPtrs g_noalloc_ptr[kNoAllocMaxDevices] = {};
+
+// Device addresses of the scratch array and the words on the current device
+// (resolved once per device).
+srk_status noalloc_ptrs(NoAllocPtrs* out) {
   int dev = 0;
   SRK_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kNoAllocMaxDevices) return fail(SRK_ERR_UNSUPPORTED, "device %d out of range", dev);
   std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-  if (!g_noalloc_ptr[dev]) {
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+  if (!g_noalloc_ptr[dev].words) {
+    NoAllocPtrs p;
+    cudaError_t e = cudaGetSymbolAddress(&p.scratch, g_noalloc_scratch);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void**>(&p.words), g_noalloc_words);
     if (e != cudaSuccess) return cuda_status(e, "cudaGetSymbolAddress(no-alloc scratch)");
     g_noalloc_ptr[dev] = p;
   }
@@ -59,6 +68,28 @@ srk_status noalloc_scratch(void** out) {
 }
 
 }  // namespace
+
+namespace srk {
+srk_status noalloc_words(unsigned int** stop, unsigned int** spare) {
+  NoAllocPtrs p;
+  SRK_TRY(noalloc_ptrs(&p));
+  *stop = p.words;
+  *spare = p.words + 1;
+  return SRK_OK;
+}
+}  // namespace srk
+
+extern "C" srk_status srk_noalloc_sync(srk_stream_t stream) {
+  g_last_error.clear();
+  NoAllocPtrs p;
+  SRK_TRY(noalloc_ptrs(&p));
+  unsigned int where = 0;
+  SRK_CUDA(cudaMemcpyAsync(&where, p.words, sizeof(where), cudaMemcpyDeviceToHost, stream));
+  SRK_CUDA(cudaStreamSynchronize(stream));
+  if (!where) return SRK_OK;
+  SRK_CUDA(cudaMemsetAsync(p.words, 0, sizeof(where), stream));
+  return fail(SRK_ERR_TIMEOUT, "a bounded device-side wait for a copy gave up (site %u); outputs are incomplete", where);
+}
 
 extern "C" srk_status srk_training_forward_noalloc(const float* d_E, const float* d_I, const void* d_Gx_freq,
                                                    const void* d_Gy_freq, int N, int W, int erosion, float dx, int B,
@@ -82,9 +113,9 @@ extern "C" srk_status srk_training_forward_noalloc(const float* d_E, const float
   if (fixed + per_wt > cap)
     return fail(SRK_ERR_UNSUPPORTED, "N=%d needs %zu bytes of scratch for one work tile, the array holds %zu", N,
                 (fixed + per_wt) * sizeof(float2), kNoAllocScratchBytes);
-  void* base = nullptr;
-  SRK_TRY(noalloc_scratch(&base));
-  float2* sc = static_cast<float2*>(base);
+  NoAllocPtrs ptrs;
+  SRK_TRY(noalloc_ptrs(&ptrs));
+  float2* sc = static_cast<float2*>(ptrs.scratch);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
   // A plan view over the static array (host struct on the stack; nothing is allocated).
@@ -118,5 +149,6 @@ extern "C" srk_status srk_training_forward_noalloc(const float* d_E, const float
   std::memset(&g, 0, sizeof(g));
   g.M = M; g.e = erosion; g.S = S; g.T = 1; g.Nin = N; g.Wout = W; g.TT = 1; g.U = B;
   g.N = N; g.W = W;
+  g.err = ptrs.words;
   return launch_conv<OP_FWD, float>(&view, a, g, false, s);
 }

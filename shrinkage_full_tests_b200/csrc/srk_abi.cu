@@ -70,7 +70,7 @@ Geom fwd_geom(const srk_plan_s* p, int B) {
   g.M = p->M; g.e = p->e; g.S = p->S; g.T = p->T;
   g.Nin = p->N; g.Wout = p->W; g.TT = p->T * p->T; g.U = B * g.TT;
   g.N = p->N; g.W = p->W; g.wout_n = 0;
-  g.err = p->direct_err;
+  g.err = p->stop;
   return g;
 }
 // Tiles per axis of the adjoint geometry.  Its input is zero outside the
@@ -87,7 +87,7 @@ Geom adj_tiles_geom(const srk_plan_s* p, int B) {
   g.M = p->M; g.e = p->e; g.S = p->S; g.T = (p->N + p->S - 1) / p->S;
   g.Nin = p->N + 2 * p->e; g.Wout = p->N; g.TT = g.T * g.T; g.U = B * g.TT;
   g.N = p->N; g.W = p->W; g.wout_n = 1;
-  g.err = p->direct_err;
+  g.err = p->stop;
   return g;
 }
 Geom adj_geom(const srk_plan_s* p, int B) {
@@ -255,9 +255,16 @@ OpArgs base_args(const srk_plan_s* p) {
 
 srk_status set_device(const srk_plan_s* p) { return cuda_status(cudaSetDevice(p->device), "cudaSetDevice"); }
 
-// Report (once) a bounded wait that gave up in an already completed
-// persistent launch of this plan.
+// Report (once) a bounded wait that gave up in an already completed launch of
+// this plan: an FFT pass writes its site into mapped host memory itself, a
+// persistent launch's abort flag is copied behind it.
 srk_status check_mailbox(srk_plan_s* p) {
+  volatile unsigned int* stop = p->mailbox + 2;
+  if (const unsigned int where = *stop) {
+    *stop = 0;
+    return fail(SRK_ERR_TIMEOUT,
+                "a bounded device-side wait for a copy gave up (site %u); that call's outputs are incomplete", where);
+  }
   if (!p->mailbox_pending) return SRK_OK;
   const cudaError_t q = cudaEventQuery(p->mailbox_ev);
   if (q == cudaErrorNotReady) return SRK_OK;
@@ -440,10 +447,12 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
   }
   if ((err = cudaMalloc(reinterpret_cast<void**>(&p->ctl), sizeof(Ctl))) != cudaSuccess)
     return cleanup(cuda_status(err, "control block allocation"));
-  if ((err = cudaHostAlloc(reinterpret_cast<void**>(&p->mailbox), 2 * sizeof(unsigned int), cudaHostAllocDefault)) !=
-      cudaSuccess)
+  if ((err = cudaHostAlloc(reinterpret_cast<void**>(&p->mailbox), 3 * sizeof(unsigned int), cudaHostAllocMapped)) !=
+          cudaSuccess ||
+      (err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&p->stop), p->mailbox, 0)) != cudaSuccess)
     return cleanup(cuda_status(err, "mailbox allocation"));
-  p->mailbox[0] = p->mailbox[1] = 0;
+  p->stop += 2;
+  p->mailbox[0] = p->mailbox[1] = p->mailbox[2] = 0;
   if ((err = cudaHostAlloc(reinterpret_cast<void**>(&p->mailbox_spins), sizeof(unsigned long long),
                            cudaHostAllocDefault)) != cudaSuccess)
     return cleanup(cuda_status(err, "mailbox allocation"));
@@ -604,8 +613,8 @@ srk_status srk_plan_sync(srk_plan p, srk_stream_t s) {
     if (derr) {
       SRK_CUDA(cudaMemset(p->direct_err, 0, sizeof(derr)));
       return fail(SRK_ERR_TIMEOUT,
-                  "a kernel stopped early (site %u: 1-13 and 16 a bounded wait gave up, 14-15 a shared memory "
-                  "block off its alignment); outputs incomplete",
+                  "a tensor-core schedule stopped early (site %u: 14, 15 and 19 a shared memory block off its "
+                  "alignment, the others a bounded wait that gave up); outputs incomplete",
                   derr);
     }
   }
@@ -631,6 +640,26 @@ srk_status srk_debug_wait_selftest(srk_plan p, unsigned long long spin_limit, sr
   SRK_CUDA(cudaEventRecord(p->mailbox_ev, s));
   p->mailbox_pending = true;
   return srk_plan_sync(p, s);
+}
+
+srk_status srk_debug_copy_wait_selftest(srk_plan p, unsigned long long spin_limit, srk_stream_t s) {
+  if (spin_limit == 0 || spin_limit > (1ull << 22)) return fail(SRK_ERR_INVALID_ARG, "spin_limit out of range");
+  unsigned int* err = nullptr;
+  unsigned int* out = nullptr;  // threads that would have stored all the same
+  if (p) {
+    SRK_TRY(enter(p, s));
+    err = p->stop;
+    out = &p->ctl->pad;
+  } else {
+    SRK_TRY(noalloc_words(&err, &out));
+  }
+  SRK_CUDA(cudaMemsetAsync(out, 0, sizeof(unsigned int), s));
+  k_copy_wait_selftest<<<1, kThreads, group_bytes<512, false>(), s>>>(err, spin_limit, out);
+  SRK_CUDA(cudaGetLastError());
+  unsigned int stored = 0;
+  SRK_CUDA(cudaMemcpyAsync(&stored, out, sizeof(stored), cudaMemcpyDeviceToHost, s));
+  SRK_CUDA(cudaStreamSynchronize(s));
+  return stored ? fail(SRK_ERR_CUDA, "%u threads went on after a wait that gave up", stored) : SRK_OK;
 }
 
 srk_status srk_plan_set_adj_convention(srk_plan p, srk_adj_convention c) {

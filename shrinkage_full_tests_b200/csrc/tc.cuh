@@ -34,6 +34,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned par, unsigned lo
   }
   return false;
 }
+// The end of a wait that gave up (`done` false; nothing else happens when it
+// is true): `site` to the error word (if there is one), 1 to the word `stop`
+// in shared memory, and this thread leaves the kernel.  Predicated
+// instructions in one piece: a branch that the compiler sees cost the last pass
+// at M = 256 6 % (spills; 153 -> 163 us per 600 work tiles), and a flag tested at
+// the stores up to 650 bytes of spills.
+template <unsigned SITE>
+__device__ __forceinline__ void leave_unless(bool done, unsigned int* err, unsigned* stop) {
+  asm volatile(
+      "{\n\t.reg .pred q, r;\n\t"
+      "setp.eq.u32 q, %0, 0;\n\t"
+      "setp.ne.and.u64 r, %1, 0, q;\n\t"
+      "@r st.volatile.global.u32 [%1], %3;\n\t"
+      "@q st.volatile.shared.u32 [%2], 1;\n\t"
+      "@q exit;\n\t}" ::"r"((unsigned)done),
+      "l"(err), "r"(smem_u32(stop)), "n"(SITE)
+      : "memory");
+}
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_u32(dst)),

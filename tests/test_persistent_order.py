@@ -21,7 +21,7 @@ def test_scratch_is_fenced_for_the_async_proxy():
     text = open(os.path.join(CSRC, "engine.cuh")).read()
     body = re.sub(r"//.*", "", text[text.index("\nk_persist("):text.index("k_wait_selftest")])
     fence = "tc::fence_async_global();"
-    order = [body.index("wait_geq"), body.index("if (!s_t[1]) break;"), body.index(fence), body.index("phase1<"),
+    order = [body.index("wait_geq"), body.index("if (!s_t[1]"), body.index(fence), body.index("phase1<"),
              body.index("phase2<"), body.index("phase3<"), body.rindex(fence), body.index("__threadfence();")]
     assert order == sorted(order) and body.count(fence) == 2
     assert "fence.proxy.async.global" in open(os.path.join(CSRC, "tc.cuh")).read()
