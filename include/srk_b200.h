@@ -137,8 +137,8 @@ srk_status srk_plan_destroy(srk_plan plan);
 #define SRK_TILE_AUTOTUNE (-1)
 /* Time every (tile size, schedule) candidate of the forward operator for this
  * configuration on synthetic device data (up to 512 images) and return the
- * fastest.  Results are cached per device name and configuration in the file
- * named by $SRK_TUNE_CACHE (default ~/.cache/srk_b200_tune.txt). */
+ * fastest.  Results are cached per device name, version of the kernels and
+ * configuration in the file named by $SRK_TUNE_CACHE (default ~/.cache/srk_b200_tune.txt). */
 srk_status srk_autotune(int N, int W, int erosion, float dx, int B, srk_dtype dtype, int* tile_M, int* schedule);
 srk_status srk_plan_get_info(srk_plan plan, srk_plan_info* info);
 srk_status srk_plan_set_adj_convention(srk_plan plan, srk_adj_convention conv);

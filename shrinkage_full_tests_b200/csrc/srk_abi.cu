@@ -312,6 +312,11 @@ std::string tune_cache_path() {
   return std::string(home ? home : "/tmp") + "/.cache/srk_b200_tune.txt";
 }
 
+// Version of the kernels that the cache's timings were taken with: raise it
+// when their speed changes.  Entries of another version are not found: a file
+// from before the present transform names tiles that are no longer the fastest.
+constexpr int kTuneVersion = 2;
+
 std::string tune_key(int N, int W, int e, int B, srk_dtype dt) {
   int dev = 0;
   cudaGetDevice(&dev);
@@ -322,7 +327,7 @@ std::string tune_key(int N, int W, int e, int B, srk_dtype dt) {
   int bb = 1;
   while (bb < B) bb <<= 1;  // batch bucket
   char buf[256];
-  snprintf(buf, sizeof(buf), "%s:N%d:W%d:e%d:B%d:t%d", name.c_str(), N, W, e, bb, (int)dt);
+  snprintf(buf, sizeof(buf), "%s:v%d:N%d:W%d:e%d:B%d:t%d", name.c_str(), kTuneVersion, N, W, e, bb, (int)dt);
   return buf;
 }
 
