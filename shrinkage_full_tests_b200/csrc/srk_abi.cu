@@ -414,9 +414,11 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
   p->schedule = sched;
   p->T = (W + p->S - 1) / p->S;
   p->Ta = adj_single(p) ? 1 : (N + p->S - 1) / p->S;
-  const size_t nwt_max = std::max<size_t>({(size_t)(B_max * (size_t)p->T * p->T + 1) / 2,
-                                           (size_t)B_max * p->T * p->T,
-                                           (size_t)(B_max * (size_t)p->Ta * p->Ta + 1) / 2});
+  // work tiles in flight at most: one per tile (JVP-type operators), or one per
+  // two tiles of the adjoint geometry, which ragged batches and slabs always
+  // cover by overlapping tiles (adj_tiles_geom)
+  const size_t Tg = (N + p->S - 1) / p->S;
+  const size_t nwt_max = std::max<size_t>((size_t)B_max * p->T * p->T, ((size_t)B_max * Tg * Tg + 1) / 2);
   const size_t per = wt_bytes(M, p->S, adj_single(p));
   // default scratch: 8 GiB, at most 1/16 of the device memory, at least
   // 256 MiB.  At B=5000 on the B200 it holds the whole N=256 batch (one
