@@ -79,6 +79,9 @@ typedef enum srk_schedule {
  * FP32 accumulation).  Used by the pair operators (training forward,
  * forward, the VJP's forward part); the tangent, the tangent-adjoint and
  * the adjoint-type pass run the three-pass FFT schedule on such a plan.
+ * A plan made with tile_M = 0 whose model chose a smaller tile (small
+ * batches) moves to tile 512 when this schedule is set, if that tile needs
+ * the least FFT work for the image (so for N = 512); its tile_stride changes.
  * The plan allocates the FP16 spectra planes (1 MB per work tile of its
  * scratch) and the DFT tables (256 KB) when the schedule is set. */
 /* SRK_SCHEDULE_DIRECT: the training forward and srk_forward run as a direct

@@ -369,10 +369,10 @@ __global__ void k_hyb_tabs(const double2* __restrict__ gbuf, const int* __restri
 }  // namespace hyb
 
 // ---- host side ------------------------------------------------------------------------------
-bool tensor_rows_supported(const srk_plan_s* p, std::string* why) {
+bool tensor_rows_supported(const srk_plan_s* p, int M, std::string* why) {
   char buf[160];
   if (p->dtype == SRK_F32) snprintf(buf, sizeof buf, "needs FP16 or BF16 storage (FP16 operands)");
-  else if (p->M != hyb::M) snprintf(buf, sizeof buf, "needs tile M = 512 (plan has %d)", p->M);
+  else if (M != hyb::M) snprintf(buf, sizeof buf, "needs tile M = 512 (plan has %d)", M);
   else if (p->e < 1 || p->e > hyb::kMaxE) snprintf(buf, sizeof buf, "needs 1 <= erosion <= %d", hyb::kMaxE);
   else return true;
   if (why) *why = buf;

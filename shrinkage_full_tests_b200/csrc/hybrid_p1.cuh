@@ -14,11 +14,10 @@
 
 #include "engine.cuh"
 #include "hybrid_scale.cuh"
+#include "internal.h"
 #include "tc.cuh"
 
 namespace srk {
-
-constexpr int kHybM = 512;
 
 // Shared memory of k_p1h / k_p1h_refit, all dynamic (static __shared__
 // variables would move the dynamic block off the 128-byte boundary the TMA

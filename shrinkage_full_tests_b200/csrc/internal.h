@@ -85,6 +85,8 @@ struct srk_plan_s {
   srk_dtype dtype = SRK_F32;
   srk_adj_convention conv = SRK_ADJ_REFERENCE;
   int M = 0, S = 0, T = 0, Ta = 0;
+  bool tile_auto = false;  // tile_M = 0: the tile was chosen by choose_tile
+  size_t budget = 0;       // scratch budget asked for (0: default)
   int chunk = 0;
   float4* G[2] = {nullptr, nullptr};   // engine-layout spectra (spec_index), scaled by dx^2/M^2
   bool have_G = false;
@@ -177,7 +179,8 @@ srk_status direct_build_tables(srk_plan_s* p, int kern, cudaStream_t s);
 srk_status direct_forward(srk_plan_s* p, const void* E, const void* I, void* R, int B, cudaStream_t s);
 
 // Tensor-core row pass of the FP16/BF16 forms at tile 512 (hybrid.cu).
-bool tensor_rows_supported(const srk_plan_s* p, std::string* why);
+constexpr int kHybM = 512;  // its tile size
+bool tensor_rows_supported(const srk_plan_s* p, int M, std::string* why);
 size_t tensor_rows_tab_bytes(const srk_plan_s* p);
 size_t tensor_rows_g_bytes(const srk_plan_s* p);
 srk_status tensor_rows_build_tables(srk_plan_s* p, cudaStream_t s);

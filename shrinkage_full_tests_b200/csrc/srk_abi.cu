@@ -64,6 +64,22 @@ int choose_tile(int N, int W, int e, int B) {
   return best;
 }
 
+// The tile with the least FFT work, T^2 M^2 log2 M per image (a smaller one
+// within 2 % of it): the tile of a plan that is to run the tensor-row schedule,
+// which exists at M = 512 only.
+int least_work_tile(int W, int e) {
+  int best = 0;
+  double best_cost = 0;
+  for (int M : {128, 256, 512}) {
+    const int S = M - 2 * e;
+    if (S < 16) continue;
+    const int T = (W + S - 1) / S;
+    const double cost = (double)T * T * M * M * std::log2((double)M);
+    if (best == 0 || cost < best_cost * 0.98) { best = M; best_cost = cost; }
+  }
+  return best;
+}
+
 Geom fwd_geom(const srk_plan_s* p, int B) {
   Geom g;
   std::memset(&g, 0, sizeof(g));
@@ -151,6 +167,62 @@ srk_status adj_wrt_f(srk_plan_s* p, const float* wx, const float* wy, const void
   return fail(SRK_ERR_UNSUPPORTED, "dtype %d", (int)p->dtype);
 }
 
+// ---- what a plan holds for its tile size ---------------------------------------------
+// Scratch, spectra, twiddles (k_fft_twiddles, shared with the no-allocation
+// forward) and the import workspace at tile size M.  On a failure the plan
+// keeps what it had.
+srk_status alloc_tile(srk_plan_s* p, int M) {
+  const int S = M - 2 * p->e, T = (p->W + S - 1) / S;
+  const bool single = p->N <= M;
+  // work tiles in flight at most: one per tile (JVP-type operators), or one per
+  // two tiles of the adjoint geometry, which ragged batches and slabs always
+  // cover by overlapping tiles (adj_tiles_geom)
+  const size_t Tg = (p->N + S - 1) / S;
+  const size_t nwt_max = std::max<size_t>((size_t)p->B_max * T * T, ((size_t)p->B_max * Tg * Tg + 1) / 2);
+  const size_t per = wt_bytes(M, S, single);
+  // default scratch: 8 GiB, at most 1/16 of the device memory, at least
+  // 256 MiB.  At B=5000 on the B200 it holds the whole N=256 batch (one
+  // chunk: -4% against 1 GiB) and N=512 runs in 15 launches (-1.3%); the
+  // ring of chunks keeps smaller budgets within a few percent of it.
+  size_t cap = p->budget;
+  if (!cap) {
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    cap = std::max<size_t>((size_t)256 << 20, std::min<size_t>((size_t)8 << 30, total_b / 16));
+  }
+  size_t chunk = cap / per;
+  if (chunk < 1) chunk = 1;
+  if (chunk > nwt_max) chunk = nwt_max;
+  if (chunk > 65535) chunk = 65535;
+  const size_t KW = 2 * (size_t)p->e + 1;
+  void* fresh[6] = {};
+  struct { void** ptr; size_t bytes; const char* what; } bufs[6] = {
+      {reinterpret_cast<void**>(&p->scratch), per * chunk, "scratch allocation"},
+      {reinterpret_cast<void**>(&p->G[0]), sizeof(float2) * (size_t)M * M, "spectrum allocation"},
+      {reinterpret_cast<void**>(&p->G[1]), sizeof(float2) * (size_t)M * M, "spectrum allocation"},
+      {reinterpret_cast<void**>(&p->tw), sizeof(float2) * M, "twiddle allocation"},
+      {reinterpret_cast<void**>(&p->imp_tab), sizeof(double2) * (size_t)M, "import workspace"},
+      {reinterpret_cast<void**>(&p->imp_P), sizeof(double2) * KW * (size_t)M, "import workspace"}};
+  for (int i = 0; i < 6; ++i) {
+    const cudaError_t err = cudaMalloc(&fresh[i], bufs[i].bytes);
+    if (err != cudaSuccess) {
+      for (int k = 0; k < i; ++k) cudaFree(fresh[k]);
+      return cuda_status(err, bufs[i].what);
+    }
+  }
+  for (int i = 0; i < 6; ++i) {
+    if (*bufs[i].ptr) cudaFree(*bufs[i].ptr);
+    *bufs[i].ptr = fresh[i];
+  }
+  p->M = M; p->S = S; p->T = T;
+  p->Ta = single ? 1 : (int)Tg;
+  p->chunk = (int)chunk;
+  p->scratch_bytes = per * chunk;
+  k_fft_twiddles<<<(M + 127) / 128, 128>>>(p->tw, M);
+  k_twiddles64<<<(M + 127) / 128, 128>>>(p->imp_tab, M);
+  return cuda_status(cudaGetLastError(), "twiddle tables");
+}
+
 // ---- spectra -----------------------------------------------------------------------
 // FP64 twiddle table (cos, sin)(2 pi m / M) built on the device.
 srk_status build_tab64(double2* tab, int M, cudaStream_t s) {
@@ -205,6 +277,18 @@ srk_status refresh_direct(srk_plan_s* p, cudaStream_t s) {
     SRK_TRY(tensor_rows_build_tables(p, s));
     p->hyb_ready = true;
   }
+  return SRK_OK;
+}
+
+// The plan at tile size M instead of its present one (its device work has
+// ended), with the bound kernel's spectra anew from the kernel in space.  For
+// FP16/BF16 plans: the ragged and slab entry points, whose tile tables depend
+// on the tile, take float.
+srk_status change_tile(srk_plan_s* p, int M) {
+  SRK_TRY(alloc_tile(p, M));
+  const double scale = (double)p->dx * (double)p->dx / ((double)M * (double)M);
+  for (int i = 0; p->have_G && i < 2; ++i)
+    SRK_TRY(spectrum_from_spatial(p->kd[i], 2 * p->e + 1, M, p->imp_tab, p->imp_P, scale, p->G[i], nullptr, nullptr));
   return SRK_OK;
 }
 
@@ -410,42 +494,15 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device);
   p->N = N; p->W = W; p->e = erosion; p->dx = dx; p->B_max = B_max; p->spectra_M = spectra_M; p->dtype = dtype;
-  p->M = M; p->S = M - 2 * erosion;
+  p->tile_auto = tile_M == 0;
+  p->budget = budget;
   p->schedule = sched;
-  p->T = (W + p->S - 1) / p->S;
-  p->Ta = adj_single(p) ? 1 : (N + p->S - 1) / p->S;
-  // work tiles in flight at most: one per tile (JVP-type operators), or one per
-  // two tiles of the adjoint geometry, which ragged batches and slabs always
-  // cover by overlapping tiles (adj_tiles_geom)
-  const size_t Tg = (N + p->S - 1) / p->S;
-  const size_t nwt_max = std::max<size_t>((size_t)B_max * p->T * p->T, ((size_t)B_max * Tg * Tg + 1) / 2);
-  const size_t per = wt_bytes(M, p->S, adj_single(p));
-  // default scratch: 8 GiB, at most 1/16 of the device memory, at least
-  // 256 MiB.  At B=5000 on the B200 it holds the whole N=256 batch (one
-  // chunk: -4% against 1 GiB) and N=512 runs in 15 launches (-1.3%); the
-  // ring of chunks keeps smaller budgets within a few percent of it.
-  size_t cap = budget;
-  if (!cap) {
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    cap = std::max<size_t>((size_t)256 << 20, std::min<size_t>((size_t)8 << 30, total_b / 16));
-  }
-  size_t chunk = cap / per;
-  if (chunk < 1) chunk = 1;
-  if (chunk > nwt_max) chunk = nwt_max;
-  if (chunk > 65535) chunk = 65535;
-  p->chunk = (int)chunk;
-  p->scratch_bytes = per * chunk;
-
   auto cleanup = [&](srk_status st) { srk_plan_destroy(p); return st; };
   cudaError_t err;
-  if ((err = cudaMalloc(reinterpret_cast<void**>(&p->scratch), p->scratch_bytes)) != cudaSuccess)
-    return cleanup(cuda_status(err, "scratch allocation"));
-  for (int i = 0; i < 2; ++i)
-    if ((err = cudaMalloc(reinterpret_cast<void**>(&p->G[i]), sizeof(float2) * (size_t)M * M)) != cudaSuccess)
-      return cleanup(cuda_status(err, "spectrum allocation"));
-  if ((err = cudaMalloc(reinterpret_cast<void**>(&p->tw), sizeof(float2) * M)) != cudaSuccess)
-    return cleanup(cuda_status(err, "twiddle allocation"));
+  {
+    const srk_status st = alloc_tile(p, M);
+    if (st != SRK_OK) return cleanup(st);
+  }
   // the derivative operators' intermediate (ensure_wbuf), allocated here once
   p->wbuf_bytes = 2 * (size_t)W * W * (size_t)B_max * sizeof(float);
   if ((err = cudaMalloc(reinterpret_cast<void**>(&p->wbuf), p->wbuf_bytes)) != cudaSuccess) {
@@ -480,9 +537,7 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
     const size_t KW = 2 * (size_t)erosion + 1;
     const size_t Mr = (size_t)spectra_M;
     struct { void** ptr; size_t bytes; } bufs[] = {
-        {reinterpret_cast<void**>(&p->imp_tab), sizeof(double2) * (size_t)M},
         {reinterpret_cast<void**>(&p->imp_tabr), sizeof(double2) * Mr},
-        {reinterpret_cast<void**>(&p->imp_P), sizeof(double2) * KW * (size_t)M},
         {reinterpret_cast<void**>(&p->imp_Tm), sizeof(double2) * (Mr / 2 + 1) * KW},
         {reinterpret_cast<void**>(&p->imp_Kd), sizeof(double) * KW * KW},
         {reinterpret_cast<void**>(&p->kd[0]), sizeof(double) * KW * KW},
@@ -491,11 +546,6 @@ srk_status srk_plan_create(srk_plan* out, int N, int W, int erosion, float dx, i
     for (auto& b : bufs)
       if ((err = cudaMalloc(b.ptr, b.bytes)) != cudaSuccess) return cleanup(cuda_status(err, "import workspace"));
   }
-  // twiddle tables built on the device: the engine's per-pass float blocks
-  // (k_fft_twiddles, shared with the no-allocation forward) and the FP64
-  // tables of the spectrum import
-  k_fft_twiddles<<<(M + 127) / 128, 128>>>(p->tw, M);
-  k_twiddles64<<<(M + 127) / 128, 128>>>(p->imp_tab, M);
   k_twiddles64<<<(spectra_M + 127) / 128, 128>>>(p->imp_tabr, spectra_M);
   if ((err = cudaMemset(p->direct_err, 0, 4 * sizeof(unsigned int))) != cudaSuccess)
     return cleanup(cuda_status(err, "error word"));
@@ -561,9 +611,13 @@ srk_status srk_plan_set_schedule(srk_plan p, srk_schedule sch) {
     return fail(SRK_ERR_INVALID_ARG, "bad schedule %d", (int)sch);
   if (sch == SRK_SCHEDULE_TENSOR_ROWS) {
     std::string why;
-    if (!tensor_rows_supported(p, &why)) return fail(SRK_ERR_UNSUPPORTED, "tensor-row schedule: %s", why.c_str());
+    // a tile that the plan chose by itself need not be the schedule's
+    const bool move = p->tile_auto && p->M != kHybM && least_work_tile(p->W, p->e) == kHybM;
+    if (!tensor_rows_supported(p, move ? kHybM : p->M, &why))
+      return fail(SRK_ERR_UNSUPPORTED, "tensor-row schedule: %s", why.c_str());
     SRK_TRY(set_device(p));
     SRK_CUDA(cudaDeviceSynchronize());  // the bound spectra may still be in flight on the caller's stream
+    if (move) SRK_TRY(change_tile(p, kHybM));
     if (!p->hyb_tabs) SRK_CUDA(cudaMalloc(reinterpret_cast<void**>(&p->hyb_tabs), tensor_rows_tab_bytes(p)));
     if (!p->hyb_g) SRK_CUDA(cudaMalloc(reinterpret_cast<void**>(&p->hyb_g), tensor_rows_g_bytes(p)));
     if (!p->hyb_s1) {
@@ -1514,7 +1568,7 @@ srk_status srk_autotune(int N, int W, int erosion, float dx, int B, srk_dtype dt
     srk_plan p = nullptr;
     if (srk_plan_create(&p, N, W, erosion, dx, Bt, N + (N & 1), dtype, 512, 0) == SRK_OK) {
       std::string why;
-      if (tensor_rows_supported(p, &why) && srk_plan_set_schedule(p, SRK_SCHEDULE_TENSOR_ROWS) == SRK_OK &&
+      if (tensor_rows_supported(p, p->M, &why) && srk_plan_set_schedule(p, SRK_SCHEDULE_TENSOR_ROWS) == SRK_OK &&
           (st = srk_plan_set_kernel(p, Kx, Ky, KW, s)) == SRK_OK) {
         for (int it = 0; it < 2; ++it) op_forward(E, E, Bt, s, R, p);
         cudaEventRecord(e0, s);
