@@ -561,21 +561,36 @@ __device__ __forceinline__ bool window_zero(int nc, int n, int c0, int c1, int r
 // Columns [c0, c1) and elements [r0, r1) (whole pieces) of a window in
 // asynchronous pieces of BYTES; 2: through registers, a batch of loads in
 // flight, in aligned words (forward of 100 FP16 images of 511, KW 31: 262 us
-// with single values, 195 so).
-template <int M, typename T, int BYTES>
+// with single values, 195 so).  FULL: a column's asynchronous copies without
+// loop or address arithmetic between them, for the group's few warps wait on
+// their issue and not on the memory (adjoint of one odd-N image, FP32, N = 257 to
+// 1501: 3 % less device time).  Not in the last pass at M = 512, whose registers
+// it takes (forward of one image of 777, KW 121: 20 -> 24 us).
+template <int M, typename T, int BYTES, bool FULL>
 __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, int c0, int c1, int r0, int r1, int HP,
                                               T* __restrict__ win) {
   constexpr int E = BYTES / (int)sizeof(T) ? BYTES / (int)sizeof(T) : 1;
   constexpr int GT = Quad<M>::GT;
   const int t = threadIdx.x % GT;
   if constexpr (BYTES > 2) {
+    const int k0 = r0 + E * t;
 #pragma unroll 1
     for (int c = c0; c < c1; ++c) {
-      const T* p = src + (long long)c * N + r0 + E * t;
-      unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(win + c * HP + r0 + E * t));
+      const T* p = src + (long long)c * N + k0;
+      unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(win + c * HP + k0));
+      auto copy = [&](int i) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d + i * BYTES * GT), "l"(p + i * E * GT),
+                     "n"(BYTES)
+                     : "memory");
+      };
+      if constexpr (FULL) {
+#pragma unroll
+        for (int i = 0; i < (win_pitch<T>(M) + E * GT - 1) / (E * GT); ++i)
+          if (k0 + i * E * GT < r1) copy(i);
+      } else {
 #pragma unroll 4
-      for (int k = r0 + E * t; k < r1; k += E * GT, p += E * GT, d += BYTES * GT)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(p), "n"(BYTES) : "memory");
+        for (int k = k0; k < r1; k += E * GT, p += E * GT, d += BYTES * GT) copy(0);
+      }
     }
   } else {
     // Four elements per thread and column from the aligned words around them,
@@ -636,7 +651,7 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 // threads cost P3 and the adjoint's P1 several hundred instructions.  Else
 // the threads copy the largest pieces that N and the image allow.  The group
 // is past gm.open().  FORM: what the launch knows of the images (Form).
-template <int M, int FORM, typename T>
+template <int M, int FORM, bool FULL, typename T>
 __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, ColSpan need,
                                                int gy0, int nr, int HP, T* __restrict__ win, bool edge,
                                                const GroupMem<M>& gm, int i) {
@@ -659,7 +674,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   const int c0 = cs.lo, c1 = cs.hi;
   const T* src = img + (long long)gx0 * N + w.at;  // (dereferenced inside the image only)
   if constexpr (FORM == kOddN) {
-    window_pieces<M, T, (int)sizeof(T)>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, (int)sizeof(T), FULL>(src, N, c0, c1, r0, r1, HP, win);
     return w;
   }
   if (w.bulk) {
@@ -669,11 +684,11 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
     if (t >= c0 && t < c1 && len) tc::bulk_g2s(win + t * HP + r0, src + (long long)t * N + r0, len, gm.bar + i);
     if constexpr (FORM != kAny) return w;
   } else if (bytes == 8) {
-    window_pieces<M, T, 8>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 8, FULL>(src, N, c0, c1, r0, r1, HP, win);
   } else if (bytes == 4) {
-    window_pieces<M, T, 4>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 4, FULL>(src, N, c0, c1, r0, r1, HP, win);
   } else {
-    window_pieces<M, T, 2>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 2, FULL>(src, N, c0, c1, r0, r1, HP, win);
   }
   if (edge) w.sync |= window_zero<M, T>(nc, n, c0, c1, r0, r1, HP, win);
   return w;
@@ -816,7 +831,7 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
     return o;
   };
   auto stage = [&](const TileRef& t, const void* img, int i) {
-    return issue_window<M, FORM>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
+    return issue_window<M, FORM, true>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
                               ColSpan{0, kWinCols}, t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
   };
   auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
@@ -1159,11 +1174,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     const TileRef tr = tile_h(h);
     if constexpr (GRAD) {
       const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
-      wn[h] = issue_window<M, FORM>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, need(1),
+      wn[h] = issue_window<M, FORM, (M < 512)>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, need(1),
                                  tr.y0 + g.e - 1, g.S + 2, HP, win[h], a.e < 1, gm, 1 - h);
     } else {
       const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
-      wn[h] = issue_window<M, FORM>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, need(0), tr.y0, g.S, HP, win[h], false,
+      wn[h] = issue_window<M, FORM, (M < 512)>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, need(0), tr.y0, g.S, HP, win[h], false,
                                  gm, 1 - h);
     }
   };
@@ -1509,18 +1524,19 @@ static __global__ void k_wait_selftest(Ctl* ctl, unsigned long long spin_limit) 
 // With one row per lane the march is bound by instruction issue (N = 4096:
 // 58 us FP32, the same at FP16 storage), so a lane owns a pair of rows, one
 // aligned access each, where the window's rows allow (W even, aligned
-// arrays; the pairs start at even window rows), and single rows in two
-// strips elsewhere.  N = 4096 from u and v: 62 us with blocks that loaded
+// arrays; the pairs start at even window rows), and single rows in strips of
+// 32 elsewhere (`rows` per warp).  N = 4096 from u and v: 62 us with blocks that loaded
 // every neighbour, 47 us (5.6 TB/s) so, FP16 38; B = 256, N = 512 from wx,
 // wy: 141 -> 108 us (6.3 TB/s).  16 columns a block: 32 and 64 measured 3 to
 // 10 % slower (fewer blocks in flight), 8 for small images.
 constexpr int kStencilThreads = 128;
 constexpr int kStencilWarpRows = 64;
-constexpr int kStencilRows = kStencilThreads / 32 * kStencilWarpRows;  // rows of a block
 constexpr int kStencilCols = 16;  // columns of a block
 // Row blocks of an image: pairs start at even window rows, one row above the
 // image for odd erosion.
-__host__ __device__ inline int stencil_row_blocks(int N, int e) { return (N + (e & 1) + kStencilRows - 1) / kStencilRows; }
+__host__ __device__ inline int stencil_row_blocks(int N, int e, int rows = kStencilWarpRows) {
+  return (N + (e & 1) + kStencilThreads / 32 * rows - 1) / (kStencilThreads / 32 * rows);
+}
 
 template <bool PAIR>
 struct StencilVal;  // a lane's value(s): one float or a packed pair
@@ -1636,9 +1652,9 @@ template <typename T, bool FROM_U>
 __device__ __forceinline__ void adj_wrt_f_block(const float* __restrict__ wx, const float* __restrict__ wy,
                                                 const T* __restrict__ v, const T* __restrict__ ux,
                                                 const T* __restrict__ uy, long long wo, long long oo, int N, int W,
-                                                int e, int gx0, int gx1, int rb, T* __restrict__ out) {
+                                                int e, int gx0, int gx1, int rb, int rows, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int r0 = rb * kStencilRows + (threadIdx.x >> 5) * kStencilWarpRows - (e & 1);  // the warp's first row
+  const int r0 = (rb * (kStencilThreads / 32) + (threadIdx.x >> 5)) * rows - (e & 1);  // the warp's first row
   if (r0 >= N) return;
   bool pair = !(W & 1);
   if constexpr (FROM_U)
@@ -1649,7 +1665,7 @@ __device__ __forceinline__ void adj_wrt_f_block(const float* __restrict__ wx, co
     adj_wrt_f_strip<T, FROM_U, true>(wx, wy, v, ux, uy, wo, oo, N, W, e, gx0, gx1, r0 + 2 * lane, out);
   } else {
 #pragma unroll 1
-    for (int s = 0; s < kStencilWarpRows; s += 32)
+    for (int s = 0; s < rows; s += 32)
       adj_wrt_f_strip<T, FROM_U, false>(wx, wy, v, ux, uy, wo, oo, N, W, e, gx0, gx1, r0 + s + lane, out);
   }
 }
@@ -1658,13 +1674,14 @@ __device__ __forceinline__ void adj_wrt_f_block(const float* __restrict__ wx, co
 template <typename T, bool FROM_U>
 __global__ void __launch_bounds__(kStencilThreads)
 k_adj_wrt_f(const float* __restrict__ wx, const float* __restrict__ wy, const T* __restrict__ v,
-            const T* __restrict__ ux, const T* __restrict__ uy, int N, int W, int e, int cols, T* __restrict__ out) {
+            const T* __restrict__ ux, const T* __restrict__ uy, int N, int W, int e, int cols, int rows,
+            T* __restrict__ out) {
   const int gx0 = blockIdx.y * cols;
   const int b = blockIdx.z;
   grid_wait();
   grid_next();
   adj_wrt_f_block<T, FROM_U>(wx, wy, v, ux, uy, (long long)b * W * W, (long long)b * N * N, N, W, e, gx0,
-                             min(gx0 + cols, N), blockIdx.x, out);
+                             min(gx0 + cols, N), blockIdx.x, rows, out);
 }
 
 // The same for a ragged batch or a column slab over the pixel columns
@@ -1687,7 +1704,7 @@ k_adj_wrt_f_rag(const float* __restrict__ wx, const float* __restrict__ wy, cons
   const int k = blk - im.blk0;
   const int gx0 = im.cx0 + (k / nby) * kStencilCols;
   adj_wrt_f_block<T, FROM_U>(wx, wy, v, ux, uy, im.ow, im.on, im.N, im.W, e, gx0, min(gx0 + kStencilCols, im.cx1),
-                             k % nby, out);
+                             k % nby, kStencilWarpRows, out);
 }
 
 }  // namespace srk
