@@ -279,6 +279,9 @@ srk_status srk_tangent_adjoint_ragged(const float* d_f, const float* d_g, const 
  *            rE = min(r0 + T*S, W) with T = ceil((r1 - r0) / S) whole tiles
  *            of the plan's tile_stride S (the W-sized intermediate of the
  *            dL/df part is computed by whole tiles from r0).
+ * With erosion 0 the central differences reach one column further on either
+ * side: I, f, df of the forward and the tangent [c0 - 1, c1 + 1), v, ux, uy
+ * of the adjoint [c0 - 1, c1 + 1).
  * c1 - c0 must be a multiple of the plan's tile_stride (srk_plan_get_info)
  * unless c1 is the last output column (W, or N for the adjoint-type
  * outputs).  The plan is one made for the whole image (N <= its N).  The

@@ -36,6 +36,8 @@ def max_over_ranks(value, dist=None, device=None):
 # gloo), so no output is reduced across ranks.  Halos (in columns):
 #   forward, tangent: N-sized inputs [lo, hi + 2e)
 #   adjoint: W-sized v, ux, uy [lo - 2e, hi); I [lo - e - 1, hi + e + 1)
+# and with erosion 0 one more column on either side of those of the forward,
+# the tangent and v, ux, uy: the central differences reach it.
 # The interior boundaries are multiples of the plan's tile stride, so every
 # slab spans whole tiles (srk_forward_oas_slab and friends).
 
@@ -55,6 +57,18 @@ def slab_bounds(N, erosion, stride, world):
 def _clip(lo, hi, n):
     lo, hi = max(lo, 0), min(hi, n)
     return (lo, hi) if lo < hi else (lo, lo)
+
+
+def forward_need(lo, hi, N, erosion):
+    """Columns of the N-sized inputs that the forward and the tangent read for
+    the output columns [lo, hi) (srk_forward_oas_slab, srk_tangent_slab)."""
+    return _clip(lo - (erosion == 0), hi + max(2 * erosion, 1), N) if lo < hi else (lo, lo)
+
+
+def adjoint_need(lo, hi, W, erosion):
+    """Columns of v, ux, uy that the adjoint reads for [lo, hi)
+    (srk_adjoint_slab)."""
+    return _clip(lo - max(2 * erosion, 1), min(hi + (erosion == 0), W), W) if lo < hi else (0, 0)
 
 
 def exchange_columns(x, own, need, owns, needs, rank, dist):
@@ -99,13 +113,14 @@ def forward_slabs(E, I, N, erosion, stride, rank, world, dist, op):
     is column c0 (srk_forward_oas_slab on the device)."""
     W = N - 2 * erosion
     owns = slab_bounds(N, erosion, stride, world)
-    needs = [_clip(lo, hi + 2 * erosion, N) if lo < hi else (lo, lo) for lo, hi in owns]
+    needs = [forward_need(lo, hi, N, erosion) for lo, hi in owns]
     E_h = exchange_columns(E, owns[rank], needs[rank], owns, needs, rank, dist)
     I_h = E_h if I is E else exchange_columns(I, owns[rank], needs[rank], owns, needs, rank, dist)
     c0, c1 = _w_owns(owns, W)[rank]
     R = E.new_zeros((c1 - c0, W))
     if c0 < c1:
-        op(E_h, I_h, c0, c1, R)
+        k = c0 - needs[rank][0]
+        op(E_h[k:], I_h[k:], c0, c1, R)
     return R
 
 
@@ -114,12 +129,12 @@ def tangent_slabs(f, g, df, dg, N, erosion, stride, rank, world, dist, op):
     op(f_h, g_h, df_h, dg_h, c0, c1, dh) as in forward_slabs."""
     W = N - 2 * erosion
     owns = slab_bounds(N, erosion, stride, world)
-    needs = [_clip(lo, hi + 2 * erosion, N) if lo < hi else (lo, lo) for lo, hi in owns]
+    needs = [forward_need(lo, hi, N, erosion) for lo, hi in owns]
     hal = [exchange_columns(x, owns[rank], needs[rank], owns, needs, rank, dist) for x in (f, g, df, dg)]
     c0, c1 = _w_owns(owns, W)[rank]
     dh = f.new_zeros((c1 - c0, W))
     if c0 < c1:
-        op(*hal, c0, c1, dh)
+        op(*[h[c0 - needs[rank][0]:] for h in hal], c0, c1, dh)
     return dh
 
 
@@ -133,7 +148,7 @@ def adjoint_slabs(v, ux, uy, I, N, erosion, stride, rank, world, dist, op):
     W = N - 2 * e
     owns = slab_bounds(N, e, stride, world)
     wowns = _w_owns(owns, W)
-    vneeds = [_clip(lo - 2 * e, min(hi, W), W) if lo < hi else (0, 0) for lo, hi in owns]
+    vneeds = [adjoint_need(lo, hi, W, e) for lo, hi in owns]
     ineeds = [_clip(lo - e - 1, hi + e + 1, N) if lo < hi else (lo, lo) for lo, hi in owns]
     vh = [exchange_columns(x, wowns[rank], vneeds[rank], wowns, vneeds, rank, dist) for x in (v, ux, uy)]
     Ih = exchange_columns(I, owns[rank], ineeds[rank], owns, ineeds, rank, dist)

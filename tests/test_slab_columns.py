@@ -8,6 +8,8 @@ import subprocess
 
 import pytest
 
+from shrinkage_full_tests_b200.shard import adjoint_need, forward_need
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "shrinkage_full_tests_b200", "csrc")
 SRC = """
@@ -56,7 +58,7 @@ def test_windows_of_the_last_pass(columns, M, rotated):
     """Central differences of forward and tangent slabs, cotangents of the
     tangent-adjoint slab: inside the declared columns, and every column that a
     valid output reads is there."""
-    for e in range(1, min(60, (M - 8) // 2) + 1):
+    for e in range(0, min(60, (M - 8) // 2) + 1):
         S = M - 2 * e
         N = 3 * S + 2 * e + max(1, S // 3)
         W = N - 2 * e
@@ -66,10 +68,12 @@ def test_windows_of_the_last_pass(columns, M, rotated):
             for x0 in range(c0, c1, S):
                 for xg in xgs:
                     lo, hi = columns(xg, e, S, 1, x0 + xg - 1, N)
-                    assert lo == hi or (c0 <= lo and hi <= min(c1 + 2 * e, N)), (e, c0, c1, xg)
+                    first, last = (max(c0 - 1, 0), min(c1 + 1, N)) if e == 0 else (c0, min(c1 + 2 * e, N))
+                    assert forward_need(c0, c1, N, e) == (first, last)
+                    assert lo == hi or (first <= lo and hi <= last), (e, c0, c1, xg)
                     for x in range(max(xg, e), min(xg + 4, e + S)):
                         if x0 + x - e < W:
-                            assert lo <= x0 + x - 1 and x0 + x + 1 < hi
+                            assert lo <= max(x0 + x - 1, 0) and min(x0 + x + 1, N - 1) < hi
         for c0, c1 in slabs(N, S):
             r0, r1 = max(c0 - e - 1, 0), min(c1 - e + 1, W)
             T = -(-(r1 - r0) // S) if r1 > r0 else 0
@@ -96,3 +100,15 @@ def test_windows_of_the_adjoint(columns, M):
                 for xg in range(0, M, 4):
                     lo, hi = columns(0, 0, 0, 0, x0 + xg - e - 1, N, whole=6)
                     assert lo == hi or (max(c0 - e - 1, 0) <= lo and hi <= min(c1 + e + 1, N)), (e, c0, c1, xg)
+
+
+def test_columns_of_the_stencil():
+    """dL/dI of the adjoint slab [c0, c1) reads u v at the window columns
+    [c0 - e - 1, c1 - e + 1); the first pass reads v at [c0 - 2 e, c1)."""
+    for e in (0, 1, 2, 15, 60):
+        N, S = 700, 100
+        W = N - 2 * e
+        for c0, c1 in slabs(N, S):
+            first, last = adjoint_need(c0, c1, W, e)
+            assert first <= max(c0 - e - 1, 0) and min(c1 - e + 1, W) <= last
+            assert first <= max(c0 - 2 * e, 0) and min(c1, W) <= last
