@@ -1193,11 +1193,14 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
         X[i * Q::J + m] = src[4 * (S2L == kS2Rotated ? (ky + blk) & (M - 1) : ky)];
       }
   };
-  // One copy of the transform for both fields where that does not spill: at
-  // M = 512 159 -> 148 us per 150 work tiles with pairs of stores, 208 -> 198
-  // with single ones; at M = 256 and 128 two copies are as fast or faster (153
-  // against 156, 161 against 162), and beside the copies in smaller pieces of
-  // kAny and kOddN one copy spills (177 against 181, 241 against 269).
+  // One copy of the transform for both fields at M = 512, images in 16-byte
+  // columns.  Forward of 150 work tiles 159 -> 148 us with pairs of stores, 208 ->
+  // 198 with single ones (24 bytes of spills); the cotangent operators spill 24
+  // bytes with one copy and 32 - 40 with two and take the same time (VJP of 64
+  // images of 512, KW 61: 278.6 against 277.7 us, KW 121: 259.3 against 260.1).  At
+  // M = 256 and 128 two copies are as fast or faster (153 against 156, 161 against
+  // 162), and beside the copies in smaller pieces of kAny and kOddN one copy costs
+  // more spills than it saves (177 against 181, 241 against 269).
   constexpr bool LOOP = M == 512 && rows16_form(FORM);
   float2 X[Q::VPT];
   cpk u0[Q::R], u1[Q::R];
