@@ -561,12 +561,15 @@ __device__ __forceinline__ bool window_zero(int nc, int n, int c0, int c1, int r
 // Columns [c0, c1) and elements [r0, r1) (whole pieces) of a window in
 // asynchronous pieces of BYTES; 2: through registers, a batch of loads in
 // flight, in aligned words (forward of 100 FP16 images of 511, KW 31: 262 us
-// with single values, 195 so).  FULL: a column's asynchronous copies without
-// loop or address arithmetic between them, for the group's few warps wait on
-// their issue and not on the memory (adjoint of one odd-N image, FP32, N = 257 to
-// 1501: 3 % less device time).  Not in the last pass at M = 512, whose registers
-// it takes (forward of one image of 777, KW 121: 20 -> 24 us).
-template <int M, typename T, int BYTES, bool FULL>
+// with single values, 195 so).  A column's asynchronous copies have no loop or
+// address arithmetic between them, for the group's few warps wait on their
+// issue and not on the memory (adjoint of one odd-N image, FP32, N = 257 to 1501:
+// 3 % less device time); not in the last pass at M = 512, whose registers that
+// takes (forward of one image of 777, KW 121: 20 -> 24 us).  The words come by
+// predicated loads in the tangent-adjoint's first pass (one odd-N FP16 image, N =
+// 257 to 1501: 3 % less); in the adjoint's they cost 1 %, in the last pass 4 %.
+enum WindowUser : int { kLastPass = 0, kFirstPass = 1, kFirstPassTan = 2 };
+template <int M, typename T, int BYTES, int USER>
 __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, int c0, int c1, int r0, int r1, int HP,
                                               T* __restrict__ win) {
   constexpr int E = BYTES / (int)sizeof(T) ? BYTES / (int)sizeof(T) : 1;
@@ -583,7 +586,7 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
                      "n"(BYTES)
                      : "memory");
       };
-      if constexpr (FULL) {
+      if constexpr (USER != kLastPass || M < 512) {
 #pragma unroll
         for (int i = 0; i < (win_pitch<T>(M) + E * GT - 1) / (E * GT); ++i)
           if (k0 + i * E * GT < r1) copy(i);
@@ -620,7 +623,12 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
       for (int c = 0; c < kWinCols; ++c) {
         const int s = shift(c);
         const unsigned* q = reinterpret_cast<const unsigned*>(src + (long long)c * N + k - s);
-        if (c >= c0 && c < c1 && k - s >= r0 && k + 4 + s <= r1) {
+        const bool on = c >= c0 && c < c1 && k - s >= r0 && k + 4 + s <= r1;
+        if constexpr (USER == kFirstPassTan) {
+          w[c][0] = ldp32(q, on);
+          w[c][1] = ldp32(q + 1, on);
+          w[c][2] = ldp32(q + 2, on && s);
+        } else if (on) {
           w[c][0] = q[0];
           w[c][1] = q[1];
           if (s) w[c][2] = q[2];
@@ -651,7 +659,7 @@ __device__ __forceinline__ void window_pieces(const T* __restrict__ src, int N, 
 // threads cost P3 and the adjoint's P1 several hundred instructions.  Else
 // the threads copy the largest pieces that N and the image allow.  The group
 // is past gm.open().  FORM: what the launch knows of the images (Form).
-template <int M, int FORM, bool FULL, typename T>
+template <int M, int FORM, int USER, typename T>
 __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N, bool live, int gx0, int nc, ColSpan need,
                                                int gy0, int nr, int HP, T* __restrict__ win, bool edge,
                                                const GroupMem<M>& gm, int i) {
@@ -674,7 +682,7 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
   const int c0 = cs.lo, c1 = cs.hi;
   const T* src = img + (long long)gx0 * N + w.at;  // (dereferenced inside the image only)
   if constexpr (FORM == kOddN) {
-    window_pieces<M, T, (int)sizeof(T), FULL>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, (int)sizeof(T), USER>(src, N, c0, c1, r0, r1, HP, win);
     return w;
   }
   if (w.bulk) {
@@ -684,11 +692,11 @@ __device__ __forceinline__ Window issue_window(const T* __restrict__ img, int N,
     if (t >= c0 && t < c1 && len) tc::bulk_g2s(win + t * HP + r0, src + (long long)t * N + r0, len, gm.bar + i);
     if constexpr (FORM != kAny) return w;
   } else if (bytes == 8) {
-    window_pieces<M, T, 8, FULL>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 8, USER>(src, N, c0, c1, r0, r1, HP, win);
   } else if (bytes == 4) {
-    window_pieces<M, T, 4, FULL>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 4, USER>(src, N, c0, c1, r0, r1, HP, win);
   } else {
-    window_pieces<M, T, 2, FULL>(src, N, c0, c1, r0, r1, HP, win);
+    window_pieces<M, T, 2, USER>(src, N, c0, c1, r0, r1, HP, win);
   }
   if (edge) w.sync |= window_zero<M, T>(nc, n, c0, c1, r0, r1, HP, win);
   return w;
@@ -817,7 +825,6 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
                                          cpk (&hx)[Quad<M>::R], cpk (&hy)[Quad<M>::R]) {
   constexpr int HP = win_pitch<T>(M);
   static_assert(win_bytes<M, T>() <= landing_bytes<M>() && win_bytes<M, T>() <= block_bytes<M>(), "window size");
-  const TileRef tr[2] = {tile_of(g, 2 * w), tile_of(g, 2 * w + 1)};
   const int x = blk * kLines + gm.t.line, q2 = 2 * gm.t.q;
   T* const w0 = reinterpret_cast<T*>(gm.ex);
   T* const w1 = reinterpret_cast<T*>(gm.buf);
@@ -831,8 +838,9 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
     return o;
   };
   auto stage = [&](const TileRef& t, const void* img, int i) {
-    return issue_window<M, FORM, true>(static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols,
-                              ColSpan{0, kWinCols}, t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
+    return issue_window<M, FORM, TAN ? kFirstPassTan : kFirstPass>(
+        static_cast<const T*>(img) + t.on, t.N, t.live, t.x0 + blk * kLines - a.e - 1, kWinCols, ColSpan{0, kWinCols},
+        t.y0 - a.e - 1, M + 2, HP, i ? w1 : w0, a.e < 1, gm, i);
   };
   auto inside = [&](const TileRef& t) {  // every column of the group lies in the valid window
     const int ox = t.x0 + blk * kLines - 2 * a.e;
@@ -842,24 +850,34 @@ __device__ __forceinline__ void load_adj(const OpArgs& a, const Geom& g, int w, 
   gm.open();
   const T* const f0 = w0 + gm.t.line * HP;
   const T* const f1 = w1 + gm.t.line * HP;
-  const OutCol o0 = column(tr[0]), o1 = column(tr[1]);
   if constexpr (TAN) {
-    pk vv[Quad<M>::R], dv[Quad<M>::R];
-    Window f = stage(tr[0], a.I, 0), d = stage(tr[0], a.dI, 1);
-    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, vv);
-    load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[0], o0, dv);
-    window_wait<FORM>(f, gm, 0);
-    window_wait<FORM>(d, gm, 1);
-    adj_lane<M, T, true, 0, FORM>(gm, inside(tr[0]), vv, dv, o0, f0, f1, row(tr[0], f), hx, hy);
-    gm.open();  // the windows are read
-    f = stage(tr[1], a.I, 0);
-    d = stage(tr[1], a.dI, 1);
-    load_cotangent<M, T>(static_cast<const T*>(a.v), tr[1], o1, vv);
-    load_cotangent<M, T>(static_cast<const T*>(a.dv), tr[1], o1, dv);
-    window_wait<FORM>(f, gm, 0);
-    window_wait<FORM>(d, gm, 1);
-    adj_lane<M, T, true, 1, FORM>(gm, inside(tr[1]), vv, dv, o1, f0, f1, row(tr[1], f), hx, hy);
+    // One copy of the code for both tiles: the first tile's fields arrive in the
+    // im parts and move to the re parts when the second's take their place.
+    // The pass is short of instruction cache, most of all in the calls of a few
+    // blocks: tangent-adjoint of N >= 2047 1 - 3 % faster, FP16 of N <= 1022 up to 8 %.
+#pragma unroll
+    for (int r = 0; r < Quad<M>::R; ++r) hx[r] = hy[r] = cpk{0ull, 0ull};
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const TileRef th = tile_of(g, 2 * w + h);
+      const OutCol o = column(th);
+      pk vv[Quad<M>::R], dv[Quad<M>::R];
+      if (h) gm.open();  // the windows are read
+      const Window f = stage(th, a.I, 0), d = stage(th, a.dI, 1);
+      load_cotangent<M, T>(static_cast<const T*>(a.v), th, o, vv);
+      load_cotangent<M, T>(static_cast<const T*>(a.dv), th, o, dv);
+      window_wait<FORM>(f, gm, 0);
+      window_wait<FORM>(d, gm, 1);
+#pragma unroll
+      for (int r = 0; r < Quad<M>::R; ++r) {
+        hx[r].re = hx[r].im;
+        hy[r].re = hy[r].im;
+      }
+      adj_lane<M, T, true, 1, FORM>(gm, inside(th), vv, dv, o, f0, f1, row(th, f), hx, hy);
+    }
   } else {
+    const TileRef tr[2] = {tile_of(g, 2 * w), tile_of(g, 2 * w + 1)};
+    const OutCol o0 = column(tr[0]), o1 = column(tr[1]);
     pk v0[Quad<M>::R], v1[Quad<M>::R];
     const Window f = stage(tr[0], a.I, 0), s = stage(tr[1], a.I, 1);
     load_cotangent<M, T>(static_cast<const T*>(a.v), tr[0], o0, v0);
@@ -1174,11 +1192,11 @@ __device__ __forceinline__ void phase3(const float2* __restrict__ S2, const OpAr
     const TileRef tr = tile_h(h);
     if constexpr (GRAD) {
       const T* img = static_cast<const T*>(OP == OP_FWD || h == 0 ? a.I : a.dI) + tr.on;
-      wn[h] = issue_window<M, FORM, (M < 512)>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, need(1),
+      wn[h] = issue_window<M, FORM, kLastPass>(img, tr.N, tr.live, tr.x0 + xg - 1, kWinCols, need(1),
                                  tr.y0 + g.e - 1, g.S + 2, HP, win[h], a.e < 1, gm, 1 - h);
     } else {
       const T* img = static_cast<const T*>(OP == OP_VJP_F || h == 0 ? a.v : a.dv) + tr.ow;
-      wn[h] = issue_window<M, FORM, (M < 512)>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, need(0), tr.y0, g.S, HP, win[h], false,
+      wn[h] = issue_window<M, FORM, kLastPass>(img, tr.W, tr.live, tr.x0 + xg - a.e, kLines, need(0), tr.y0, g.S, HP, win[h], false,
                                  gm, 1 - h);
     }
   };
