@@ -39,34 +39,8 @@ struct NvtxRange {
 namespace {
 
 // ---- tile choice -------------------------------------------------------------
-// Time of a forward call in microseconds, fitted to the engine on a B200:
-//   launch(M) + B T^2 M^2 7.2e-6 (0.35 + 0.65 S / M).
-// The second term is the throughput limit (the passes cost the same per point
-// of a tile at every M; the row pass's stores and the last pass only touch the
-// S valid columns): B=300 N=256 KW=31 measures 270 / 141 / 594 us at M = 128 /
-// 256 / 512, B=64 N=333 KW=31 119 / 148 / 158, B=100 N=512 KW=31 240 / 422 /
-// 191.  The first is the latency of the three dependent kernels when the
-// tiles do not fill the device: shorter for small tiles, whose lines have
-// fewer values per thread (N=1024 KW=31 B=1: 22 / 35 / 36 us; N=256 KW=31
-// B=1: 15.1 / 15.7 / 21.7, its adjoint 18 / 23 / 24).
-// The valid stride S = M - 2e keeps at least 16 outputs.
-int choose_tile(int N, int W, int e, int B) {
-  int best = 0;
-  double best_cost = 0;
-  for (int M : {128, 256, 512}) {
-    const int S = M - 2 * e;
-    if (S < 16) continue;
-    const int T = (W + S - 1) / S;
-    const double launch = M == 128 ? 14.5 : M == 256 ? (T == 1 ? 15.5 : 20.0) : 21.0;
-    const double cost = launch + (double)B * T * T * M * M * 7.2e-6 * (0.35 + 0.65 * S / M);
-    if (best == 0 || cost < best_cost) { best = M; best_cost = cost; }
-  }
-  return best;
-}
-
 // The tile with the least FFT work, T^2 M^2 log2 M per image (a smaller one
-// within 2 % of it): the tile of a plan that is to run the tensor-row schedule,
-// which exists at M = 512 only.
+// within 2 % of it).
 int least_work_tile(int W, int e) {
   int best = 0;
   double best_cost = 0;
@@ -78,6 +52,46 @@ int least_work_tile(int W, int e) {
     if (best == 0 || cost < best_cost * 0.98) { best = M; best_cost = cost; }
   }
   return best;
+}
+
+// Time of a forward call in microseconds, fitted to the engine on a B200:
+//   launch(M) + B T^2 M^2 7.2e-6 (0.35 + 0.65 S / M).
+// The second term is the throughput limit (the passes cost the same per point
+// of a tile at every M; the row pass's stores and the last pass only touch the
+// S valid columns): B=300 N=256 KW=31 measures 270 / 141 / 594 us at M = 128 /
+// 256 / 512, B=64 N=333 KW=31 119 / 148 / 158, B=100 N=512 KW=31 240 / 422 /
+// 191.  The first is the latency of the three dependent kernels when the
+// tiles do not fill the device: shorter for small tiles, whose lines have
+// fewer values per thread (N=1024 KW=31 B=1: 22 / 35 / 36 us; N=256 KW=31
+// B=1: 15.1 / 15.7 / 21.7, its adjoint 18 / 23 / 24).
+// The valid stride S = M - 2e keeps at least 16 outputs.
+//
+// A tile that is the fastest for the forward may be far from it for the
+// derivatives: their overlapping tiles cover all N outputs at the same stride,
+// one tile where N <= M.  Where the same model of them (tiles 1.2 times as dear,
+// every column of S2 in use where one tile covers the image) is 1.4 times that
+// of a larger tile of least work, the plan takes that one (VJP of 4 images of 257, KW
+// 101: 57 -> 40 us, forward 17.4 -> 17.8; of 16 of 333, KW 75: 116 -> 73, forward
+// 33.6 -> 29.1; below the line the two cross: 4 of 333, KW 75: 43.5 and 41.7).
+int choose_tile(int N, int W, int e, int B) {
+  auto cost = [&](int M, int T, double per_tile) {
+    const double launch = M == 128 ? 14.5 : M == 256 ? (T == 1 ? 15.5 : 20.0) : 21.0;
+    return launch + (double)B * T * T * M * M * 7.2e-6 * per_tile;
+  };
+  auto derivative = [&](int M) {
+    const int S = M - 2 * e, T = N <= M ? 1 : (N + S - 1) / S;
+    return cost(M, T, 1.2 * (0.5 + 0.5 * (N <= M ? 1.0 : (double)S / M)));
+  };
+  int best = 0;
+  double best_cost = 0;
+  for (int M : {128, 256, 512}) {
+    const int S = M - 2 * e;
+    if (S < 16) continue;
+    const double c = cost(M, (W + S - 1) / S, 0.35 + 0.65 * S / M);
+    if (best == 0 || c < best_cost) { best = M; best_cost = c; }
+  }
+  const int lw = least_work_tile(W, e);
+  return best && best < lw && derivative(best) > 1.4 * derivative(lw) ? lw : best;
 }
 
 Geom fwd_geom(const srk_plan_s* p, int B) {
