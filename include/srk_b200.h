@@ -129,7 +129,7 @@ const char* srk_last_error(void);
  *         (cached on disk, see srk_autotune), else 128, 256 or 512.
  * scratch_budget_bytes: 0 = default (8 GiB, at most 1/16 of the device
  *         memory, at least 256 MiB); the scratch holds the work tiles in
- *         flight (5.3 MB each at N = 512, KW = 121), never more than B_max needs.
+ *         flight (6.3 MB each at N = 512, KW = 121), never more than B_max needs.
  * The plan also holds 2 W^2 B_max floats for the intermediate of the VJP
  * and the tangent-adjoint (u*v between the FFT passes and the transposed
  * stencil): every device buffer an operator uses is allocated here (plus the
